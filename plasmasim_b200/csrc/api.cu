@@ -48,7 +48,7 @@ struct Store {
   bool spill_pending = false;
   cudaEvent_t readback = nullptr;
   int* holes = nullptr;   // per-slot scratch: hole rows of every lane column
-  int* nholes = nullptr;  // per interior cell: holes of its lane column
+  int* nholes = nullptr;  // per lane of every group: holes of its column
   int* nonhome = nullptr; // a particle outside its home cell stayed in the layout
   // a refill's shell deletion over the layout is left to the next classify pass
   bool shell_pending = false;
@@ -86,6 +86,9 @@ struct pic_ctx {
   // tiled layout of each species, double-buffered (the sort reads the old one)
   int* goff[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
   int* gmax[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
+  int* gtop[2] = {nullptr, nullptr};  // rows in use of each group of the current layout
+  int2* gfree = nullptr;              // a full sort's free slots (NewLayout)
+  int* gcursor = nullptr;             // and its per-group cursor
   int lay[2] = {0, 0};                // current layout buffer
   bool layout[2] = {false, false};    // slots [0, tiled_end) follow goff/gmax[lay]
   long long tiled_end[2] = {0, 0};
@@ -714,7 +717,7 @@ int do_push_tiled(pic_ctx* c, int s) {
   if (!c->layout[s]) return do_push<real, PUSH_FUSED>(c, s);
   CKR((do_push<real, PUSH_FUSED>(c, s, c->tiled_end[s])));
   const int ntiles = c->tg.ntx * c->tg.nty * c->tg.ntz;
-  TileArgs ta{c->tg, c->goff[s][c->lay[s]], c->gmax[s][c->lay[s]]};
+  TileArgs ta{c->tg, c->goff[s][c->lay[s]], c->gtop[s]};
   const bool vec = sizeof(real) == 4 && c->g.gz % 4 == 0;
   const Parts<real> P = parts<real>(c, s);
   const Fields<real> F = fields<real>(c);
@@ -769,9 +772,10 @@ int refill_slabs(const pic_ctx* c, Slab* slabs);
 // sorting (:7475-7590) into the tiled layout of tiled.cuh: count the
 // particles of every interior cell (stayers of the previous layout per lane
 // column, movers and appended particles per destination cell), size every
-// group by its fullest lane, scan the group sizes, then write stayers in their
-// previous column order and movers after them. Particles outside the interior
-// are dropped, as the reference's sort drops them.
+// group by its mean lane plus slack, scan the group sizes, then write stayers
+// in their previous column order, movers after them and what exceeds the
+// group's level into the other lanes' free slots. Particles outside the
+// interior are dropped, as the reference's sort drops them.
 template <typename real>
 int do_sort_species(pic_ctx* c, int s) {
   Store& st = c->sp[s];
@@ -799,7 +803,7 @@ int do_sort_species(pic_ctx* c, int s) {
   Slab slabs[5];
   refill_slabs(c, slabs);
   group_size_kernel<<<gblocks, kThreads, 0, c->stream>>>(c->g, tg, stay, moved, source_params(c, s, slabs, 5, 0),
-                                                         c->gmax[s][nw], c->gcap);
+                                                         c->gmax[s][nw], c->gtop[s], c->gfree, c->gcap);
   CKL();
   CKR(scan_exclusive(c, c->gcap, c->goff[s][nw], tg.ngroups, c->scan_tmp, c->scan_tmp_len));
   tiled_total_kernel<<<1, 1, 0, c->stream>>>(c->goff[s][nw], c->gcap, tg.ngroups, c->total_dev);
@@ -810,16 +814,18 @@ int do_sort_species(pic_ctx* c, int s) {
   if (total > st.cap) return PIC_ERR_CAPACITY;
   Parts<real> Q = parts<real>(c, s, 1 - st.cur);
   group_pad_kernel<<<gblocks, kThreads, 0, c->stream>>>(c->g, tg, stay, moved, c->goff[s][nw], c->gmax[s][nw],
-                                                        Q.cell);
+                                                        c->gtop[s], Q.cell);
   CKL();
+  CK(cudaMemsetAsync(c->gcursor, 0, sizeof(int) * tg.ngroups, c->stream));
+  const NewLayout nl{c->goff[s][nw], c->gtop[s], c->gfree, stay, c->cursor, c->gcursor};
   if (have) {
     tiled_scatter_kernel<real><<<gblocks, kThreads, 0, c->stream>>>(
-        P, c->g, tg, c->goff[s][old], c->gmax[s][old], c->goff[s][nw], stay, c->cursor, Q);
+        P, c->g, tg, c->goff[s][old], c->gmax[s][old], nl, Q);
     CKL();
   }
   if (st.count > first) {
     append_scatter_kernel<real><<<particle_blocks(st.count - first), kThreads, 0, c->stream>>>(
-        P, (int)first, st.count_dev, c->g, tg, c->goff[s][nw], stay, c->cursor, Q);
+        P, (int)first, st.count_dev, c->g, tg, nl, Q);
     CKL();
   }
   st.cur = 1 - st.cur;
@@ -855,15 +861,14 @@ int place_launch(pic_ctx* c, int s) {
   place_count_kernel<real><<<particle_blocks(st.cap - first), kThreads, 0, c->stream>>>(
       P, (int)first, st.count_dev, c->g, c->cursor, c->rank);
   CKL();
-  int* off = c->offs;  // per cell: arrivals that fit, then their bucket offset
-  place_fit_kernel<<<particle_blocks(c->ncells), kThreads, 0, c->stream>>>(c->cursor, st.nholes, off, c->ncells);
-  CKL();
-  CKR(scan_exclusive(c, off, off, c->ncells, c->scan_tmp, c->scan_tmp_len));
+  int* off = c->offs;  // per cell: bucket offset of its arrivals
+  CKR(scan_exclusive(c, c->cursor, off, c->ncells, c->scan_tmp, c->scan_tmp_len));
   place_bucket_kernel<real><<<particle_blocks(st.cap - first), kThreads, 0, c->stream>>>(
-      P, (int)first, st.count_dev, c->g, st.nholes, off, c->rank, c->bucket, c->total_dev, Q);
+      P, (int)first, st.count_dev, c->g, off, c->rank, c->bucket);
   CKL();
-  place_fill_kernel<real><<<gblocks, kThreads, 0, c->stream>>>(P, (int)first, c->g, tg, c->goff[s][c->lay[s]],
-                                                               st.holes, c->cursor, st.nholes, off, c->bucket);
+  place_fill_kernel<real><<<gblocks, kThreads, 0, c->stream>>>(
+      P, (int)first, c->g, tg, c->goff[s][c->lay[s]], c->gmax[s][c->lay[s]], c->gtop[s], st.holes, c->cursor,
+      st.nholes, off, c->bucket, c->total_dev, Q);
   CKL();
   unspill_kernel<real><<<particle_blocks(st.cap), kThreads, 0, c->stream>>>(Q, c->total_dev, P, (int)first);
   CKL();
@@ -889,7 +894,7 @@ int relayout_launch(pic_ctx* c, int s) {
   copy_int_kernel<<<1, 1, 0, c->stream>>>(c->append_dev, st.count_dev);
   CKL();
   classify_kernel<real><<<gblocks, kThreads, 0, c->stream>>>(P, c->g, tg, c->goff[s][c->lay[s]],
-                                                             c->gmax[s][c->lay[s]], (int)st.cap, st.holes,
+                                                             c->gmax[s][c->lay[s]], c->gtop[s], (int)st.cap, st.holes,
                                                              st.nholes, c->append_dev, st.nonhome,
                                                              st.shell_pending ? 1 : 0);
   CKL();
@@ -1698,13 +1703,19 @@ int pic_create(const pic_config* cfg, pic_ctx** out) {
         if (cudaMalloc(&c->gmax[s][b], sizeof(int) * t.ngroups) != cudaSuccess) return fail(PIC_ERR_CUDA);
       }
     }
+    // gfree, gtop of both species and gcursor in one block
+    if (cudaMalloc(&c->gfree, (sizeof(int2) * kLanes + sizeof(int) * 3) * t.ngroups) != cudaSuccess)
+      return fail(PIC_ERR_CUDA);
+    c->gtop[0] = (int*)(c->gfree + (size_t)kLanes * t.ngroups);
+    c->gtop[1] = c->gtop[0] + t.ngroups;
+    c->gcursor = c->gtop[1] + t.ngroups;
     if (cudaMalloc(&c->gcap, sizeof(int) * t.ngroups) != cudaSuccess) return fail(PIC_ERR_CUDA);
     if (cudaMalloc(&c->total_dev, sizeof(int)) != cudaSuccess) return fail(PIC_ERR_CUDA);
     if (cudaMalloc(&c->append_dev, sizeof(int)) != cudaSuccess) return fail(PIC_ERR_CUDA);
     if (tiled) {  // re-layout scratch
       for (int s = 0; s < 2; ++s) {  // each species' hole lists live from its push to its next placement
         if (cudaMalloc(&c->sp[s].holes, sizeof(int) * (size_t)cap) != cudaSuccess) return fail(PIC_ERR_CUDA);
-        if (cudaMalloc(&c->sp[s].nholes, sizeof(int) * c->ncells) != cudaSuccess) return fail(PIC_ERR_CUDA);
+        if (cudaMalloc(&c->sp[s].nholes, sizeof(int) * kLanes * t.ngroups) != cudaSuccess) return fail(PIC_ERR_CUDA);
         if (cudaMalloc(&c->sp[s].nonhome, sizeof(int)) != cudaSuccess) return fail(PIC_ERR_CUDA);
         cudaMemsetAsync(c->sp[s].nonhome, 0, sizeof(int), c->stream);
       }
@@ -1753,6 +1764,7 @@ int pic_destroy(pic_ctx* c) {
       cudaFree(c->gmax[s][b]);
     }
   }
+  cudaFree(c->gfree);
   cudaFree(c->gcap);
   cudaFree(c->total_dev);
   cudaFree(c->append_dev);

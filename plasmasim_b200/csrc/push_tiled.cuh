@@ -273,7 +273,7 @@ push_tiled_kernel(Parts<real> P, TileArgs ta, Fields<real> F, Geom g, PushConst<
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int G = tile * (kTileX * kTileY) + warp;
-  const int base = ta.goff[G], jmax = ta.gmax[G];
+  const int base = ta.goff[G], jmax = ta.gtop[G];
   // home cell of this lane
   const int hi = wx0 + 2 + warp / kTileY, hj = wy0 + 2 + warp % kTileY, hk = wz0 + 2 + lane;
   const int hcell = pack_cell(hi, hj, hk);
@@ -285,7 +285,7 @@ push_tiled_kernel(Parts<real> P, TileArgs ta, Fields<real> F, Geom g, PushConst<
   if (kFixedN) {
     int slots = 0;
 #pragma unroll
-    for (int w = 0; w < kTileX * kTileY; ++w) slots += ta.gmax[tile * (kTileX * kTileY) + w];
+    for (int w = 0; w < kTileX * kTileY; ++w) slots += ta.gtop[tile * (kTileX * kTileY) + w];
     // below 2^23 as well, where scatter8_win_fixed's rounding by an added 2^23 is exact
     nscale = fminf(4294967295.f / (float)(slots * kLanes + 1), 8388607.f);
   }

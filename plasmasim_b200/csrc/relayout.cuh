@@ -2,21 +2,24 @@
 //
 // Between two sorts most particles stay in their home cell. A re-layout
 // leaves those where they are and moves only the rest:
-//  1. classify (one warp per group): a particle whose cell is no longer its
-//     lane's home cell is copied to the append region after `count` and its
-//     slot becomes a hole (cell = -1); each lane lists the rows of its holes,
-//     in row order, in a scratch array laid out like the slots themselves.
-//     A warp takes append slots 64 at a time from the shared counter and
-//     marks the slots of its last block it does not use empty, so the counter
-//     sees one atomic per 64 movers instead of one per row;
+//  1. classify (one warp per group): a particle whose cell is not its lane's
+//     home cell (it moved, or sits in another lane's free slot) is copied to
+//     the append region after `count` and its slot becomes a hole (cell = -1);
+//     each lane lists the rows of its holes, in row order, in a scratch array
+//     laid out like the slots themselves. A warp takes append slots 64 at a
+//     time from the shared counter and marks the slots of its last block it
+//     does not use empty, so the counter sees one atomic per 64 movers instead
+//     of one per row;
 //  2. place (movers and refilled particles, all appended after `count`): the
 //     particles are bucketed by their new cell -- a rank per particle from a
-//     per-cell counter, an exclusive scan of the arrivals that find a hole,
-//     the particle's index written to its bucket slot -- and then one warp
-//     per group fills each lane's holes, in row order, from its cell's
-//     bucket. A particle ranked past its cell's holes is copied, compacted,
-//     into the spare buffer instead. Every pass streams its input, so its
-//     scattered accesses are independent of one another;
+//     per-cell counter, an exclusive scan of the arrivals, the particle's
+//     index written to its bucket slot -- and then one warp per group fills
+//     the holes below the group's level (tiled.cuh), in row order: each lane
+//     its own from its cell's bucket, then the lanes with holes left from the
+//     buckets that did not fit (strangers). The particles of a group beyond
+//     its rows are copied, compacted, into the spare buffer. Every pass
+//     streams its input, so its scattered accesses are independent of one
+//     another;
 //  3. the particles without a hole are copied back right after the layout,
 //     where the slot-order push handles them until a later re-layout finds
 //     them a hole (or a full sort, when they become too many).
@@ -42,7 +45,7 @@ __device__ __forceinline__ void copy_slot(const Parts<real>& S, int s, const Par
 // (:6015-6031) would have: one pass over the layout for both.
 template <typename real>
 __global__ void classify_kernel(Parts<real> P, Geom g, TileGeom t, const int* __restrict__ goff,
-                                const int* __restrict__ gmax, int cap, int* holes, int* nholes,
+                                const int* __restrict__ gmax, int* gtop, int cap, int* holes, int* nholes,
                                 int* append_at, int* nonhome, int shell) {
   constexpr int U = 4;  // rows whose loads are in flight together (8 measured no faster)
   const int G = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -51,7 +54,7 @@ __global__ void classify_kernel(Parts<real> P, Geom g, TileGeom t, const int* __
   const unsigned below = (1u << lane) - 1u;
   const int home = home_key(g, t, G, lane);
   const int base = goff[G], m = gmax[G];
-  int nh = 0;
+  int nh = 0, top = 0;
   int blk = 0, used = kAppendBlock;  // current block of append slots (warp-uniform)
   for (int r0 = 0; r0 < m; r0 += U) {
     int c[U], d[U];
@@ -72,7 +75,7 @@ __global__ void classify_kernel(Parts<real> P, Geom g, TileGeom t, const int* __
     for (int u = 0; u < U; ++u) {
       const int r = r0 + u;
       const int key = interior_key(g, c[u]);
-      const bool leaves = c[u] >= 0 && key != home;
+      const bool leaves = c[u] >= 0 && (key < 0 || key != home);
       const bool mover = leaves && key >= 0;
       const unsigned mm = __ballot_sync(0xffffffffu, mover);
       const int nm = __popc(mm);
@@ -95,6 +98,7 @@ __global__ void classify_kernel(Parts<real> P, Geom g, TileGeom t, const int* __
         holes[base + nh * kLanes + lane] = r;
         ++nh;
       }
+      if (!hole) top = r + 1;  // a particle stays in this row
     }
     // the movers of the U rows: their record loads issued together, then the copies
     Rec<real> rec[U];
@@ -111,7 +115,10 @@ __global__ void classify_kernel(Parts<real> P, Geom g, TileGeom t, const int* __
   }
   for (int q = used + lane; q < kAppendBlock; q += kLanes)
     if (blk + q < cap && used < kAppendBlock) P.cell[blk + q] = -1;
-  if (home >= 0) nholes[home] = nh;
+  nholes[G * kLanes + lane] = nh;
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, s));
+  if (lane == 0) gtop[G] = top;
 }
 
 __global__ void clamp_count_kernel(const int* append_at, int cap, int* count_dev) {
@@ -135,73 +142,110 @@ __global__ void __launch_bounds__(256) place_count_kernel(Parts<real> P, int fir
   }
 }
 
-// Pass 2, per interior cell: the arrivals that find a hole, min(arrivals, holes)
-// (exclusive-scanned afterwards into each cell's bucket offset).
-__global__ void place_fit_kernel(const int* __restrict__ arrivals, const int* __restrict__ nholes, int* fit,
-                                 long long ncells) {
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < ncells;
-       c += (long long)gridDim.x * blockDim.x)
-    fit[c] = min(arrivals[c], nholes[c]);
-}
-
-// Pass 3: a particle ranked below its cell's holes writes its index to its
-// bucket slot; the others are copied, compacted, into the spare buffer Q.
+// Pass 2 (after an exclusive scan of the arrivals into bucket offsets): every
+// particle writes its index to its bucket slot.
 template <typename real>
 __global__ void __launch_bounds__(256) place_bucket_kernel(Parts<real> P, int first, const int* __restrict__ count,
-                                                           Geom g, const int* __restrict__ nholes,
-                                                           const int* __restrict__ off, const int* __restrict__ rank,
-                                                           int* bucket, int* nspill, Parts<real> Q) {
+                                                           Geom g, const int* __restrict__ off,
+                                                           const int* __restrict__ rank, int* bucket) {
   const int span = *count - first;
-  const int lane = threadIdx.x & 31;
-  const unsigned below = (1u << lane) - 1u;
-  const int stride = gridDim.x * blockDim.x;
-  for (int w0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; w0 < span; w0 += stride) {  // warp-uniform
-    const int q = w0 + lane;
-    const int c = q < span ? P.cell[first + q] : -1;
-    const int key = interior_key(g, c);
-    const int r = q < span ? rank[q] : -1;
-    const bool fits = key >= 0 && r < nholes[key];
-    const bool spill = key >= 0 && !fits;
-    if (fits) bucket[off[key] + r] = q;
-    const unsigned ms = __ballot_sync(0xffffffffu, spill);
-    int sb = 0;
-    if (lane == 0 && ms) sb = atomicAdd(nspill, __popc(ms));
-    sb = __shfl_sync(0xffffffffu, sb, 0);
-    if (spill) copy_record(P, first + q, Q, sb + __popc(ms & below), c);
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < span; q += gridDim.x * blockDim.x) {
+    const int r = rank[q];
+    if (r >= 0) bucket[off[interior_key(g, P.cell[first + q])] + r] = q;
   }
 }
 
-// Pass 4, one warp per group: lane l copies the k-th particle of its home
-// cell's bucket into the slot of its k-th hole. U holes per lane are in
-// flight at once; their slots lie in the lane's own column.
+// Pass 3, one warp per group: lane l copies the k-th particle of its home
+// cell's bucket into the slot of its k-th hole below the level, U holes per
+// lane in flight at once; then the particles that found no hole of their own
+// lane go to the holes below the level that are left, the lowest of each lane
+// first. The level counts the particles that stayed and those that arrive, so
+// the holes below it hold all arrivals unless the group has outgrown its rows;
+// what is left then goes to the spare buffer Q. gtop comes in as one past the
+// last row that kept a particle and goes out covering the filled rows as well.
 template <typename real>
 __global__ void place_fill_kernel(Parts<real> P, int first, Geom g, TileGeom t, const int* __restrict__ goff,
-                                  const int* __restrict__ holes, const int* __restrict__ arrivals,
-                                  const int* __restrict__ nholes, const int* __restrict__ off,
-                                  const int* __restrict__ bucket) {
+                                  const int* __restrict__ gmax, int* gtop, const int* __restrict__ holes,
+                                  const int* __restrict__ arrivals, const int* __restrict__ nholes,
+                                  const int* __restrict__ off, const int* __restrict__ bucket, int* nspill,
+                                  Parts<real> Q) {
   constexpr int U = 4;  // holes per lane in flight together
   const int G = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (G >= t.ngroups) return;  // warp-uniform
+  const unsigned below = (1u << lane) - 1u;
   const int home = home_key(g, t, G, lane);
-  const int n = home >= 0 ? min(arrivals[home], nholes[home]) : 0;
+  const int arr = home >= 0 ? arrivals[home] : 0;
+  const int narr = warp_sum(arr);
+  if (narr == 0) return;
   const int o = home >= 0 ? off[home] : 0;
-  const int base = goff[G];
-  int nmax = n;
-#pragma unroll
-  for (int s = 16; s > 0; s >>= 1) nmax = max(nmax, __shfl_xor_sync(0xffffffffu, nmax, s));
-  for (int k0 = 0; k0 < nmax; k0 += U) {
+  const int nh = nholes[G * kLanes + lane];
+  const int base = goff[G], rows = gmax[G];
+  const int level = min(rows, group_level(rows * kLanes - warp_sum(nh) + narr));
+  const int n = min(arr, nh);
+  int top = gtop[G];
+  int used = 0;  // holes this lane has filled
+  for (int k0 = 0;; k0 += U) {
     int src[U], dst[U];
+    bool more = false;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int k = k0 + u;
-      src[u] = k < n ? first + bucket[o + k] : -1;
-      dst[u] = k < n ? base + holes[base + k * kLanes + lane] * kLanes + lane : -1;
+      const int row = k < n ? holes[base + k * kLanes + lane] : level;
+      src[u] = row < level ? first + bucket[o + k] : -1;
+      dst[u] = base + row * kLanes + lane;
+      if (row < level) {
+        top = max(top, row + 1);
+        used = k + 1;
+        more = u == U - 1;
+      }
     }
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if (src[u] >= 0) copy_record(P, src[u], P, dst[u], P.cell[src[u]]);
+    if (!__any_sync(0xffffffffu, more)) break;
   }
+  // strangers: number s of the group is entry used + (s - pre) of its lane's bucket
+  const int rest = arr - used;
+  const int pre = warp_scan(rest) - rest;
+  const int nrest = warp_sum(rest);
+  int done = 0;
+  for (int k = used; done < nrest; ++k) {
+    const int row = k < nh ? holes[base + k * kLanes + lane] : level;
+    const unsigned m = __ballot_sync(0xffffffffu, row < level);
+    if (!m) break;
+    const int s = done + __popc(m & below);
+    int b = 0;  // the last lane whose strangers start at or before s
+#pragma unroll
+    for (int q = 16; q > 0; q >>= 1)
+      if (__shfl_sync(0xffffffffu, pre, b + q) <= s) b += q;
+    const int e = __shfl_sync(0xffffffffu, o + used - pre, b) + s;
+    if (row < level && s < nrest) {
+      const int src = first + bucket[e];
+      top = max(top, row + 1);
+      copy_record(P, src, P, base + row * kLanes + lane, P.cell[src]);
+    }
+    done += __popc(m);
+  }
+  // a group that has outgrown its rows
+  for (int s0 = done; s0 < nrest; s0 += kLanes) {
+    const int s = s0 + lane;
+    int b = 0;
+#pragma unroll
+    for (int q = 16; q > 0; q >>= 1)
+      if (__shfl_sync(0xffffffffu, pre, b + q) <= s) b += q;
+    const int e = __shfl_sync(0xffffffffu, o + used - pre, b) + s;
+    int sb = 0;
+    if (lane == 0) sb = atomicAdd(nspill, min(kLanes, nrest - s0));
+    sb = __shfl_sync(0xffffffffu, sb, 0);
+    if (s < nrest) {
+      const int src = first + bucket[e];
+      copy_record(P, src, Q, sb + lane, P.cell[src]);
+    }
+  }
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, s));
+  if (lane == 0) gtop[G] = top;
 }
 
 // The particles without a hole back to slots [first, first + n).

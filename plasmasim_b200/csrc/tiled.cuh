@@ -3,12 +3,23 @@
 //
 // Layout. The interior cells are cut into tiles of TX x TY x 32 cells (x, y,
 // z). Each (x, y) column of a tile -- 32 consecutive z cells -- is a "group"
-// handled by one warp, lane L owning cell z0 + L (its "home" cell). A sort
-// writes the particles of a group interleaved: particle r of the cell in lane
-// L goes to slot goff[G] + 32 r + L, every lane's column padded with empty
-// slots (cell = -1) up to the group's largest cell count gmax[G]. A warp then
-// reads 32 consecutive slots per step of its loop (one coalesced 128-byte line
-// per array) and its 32 lanes work on 32 different cells.
+// handled by one warp, lane L owning cell z0 + L (its "home" cell). A group's
+// slots are gmax[G] rows of 32: slot goff[G] + 32 r + L is row r of lane L's
+// column. A sort fills each lane's column with the particles of its cell up to
+// the group's level -- its mean particles per lane, rounded up -- and puts the
+// rest of the fuller cells ("strangers") into the free slots below the level
+// of the group's other lanes, so that a group runs through as many rows as it
+// has particles for, not as many as its fullest cell. Slots above are empty
+// (cell = -1), kept for later arrivals; gtop[G] is one past the last row that
+// holds a particle. A warp then reads 32 consecutive slots per step of its
+// loop (one coalesced 128-byte line per array) and its 32 lanes work on 32
+// cells, nearly all of them different. Rows sized for the fullest of the 32
+// cells left a fifth (64 particles per cell) to 40 % (8) of the lanes idle
+// once the particles had mixed. Measured, push of both species per step, such
+// rows against these: 7.90 -> 7.02 ms (128^3 cells x 64 per cell), 0.413 ->
+// 0.345 (64^3 x 16), 0.092 -> 0.075 (32^3 x 8), FP64 64^3 x 32 2.05 -> 1.73;
+// the re-layout, which moves the strangers as well, 1.82 -> 2.01, 0.091 ->
+// 0.103 and 0.0345 -> 0.035.
 //
 // Deposit. A lane accumulates the current of the particles that are in its
 // home cell in registers (the 2x3x3 / 3x2x3 / 3x3x2 nodes such a particle can
@@ -24,7 +35,8 @@
 // row by row, so stayers are written in order without atomics, into nearly
 // the same 128-byte lines they came from) and places the others -- movers,
 // and particles appended by a refill -- after the stayers of their new cell
-// with per-cell atomic cursors.
+// with per-cell atomic cursors. A particle ranked past the level takes its
+// group's next free slot below the level (a per-group cursor).
 #pragma once
 
 #include "common.cuh"
@@ -32,10 +44,16 @@
 
 namespace pb {
 
-// Layout slack of a full sort: rows added to a group beyond its fullest lane,
-// count / kSlackDiv + kSlackRows (a slack of count / 32 measured no faster).
-constexpr int kSlackDiv = 16;
-constexpr int kSlackRows = 2;
+// Rows that a full sort adds to a group above its level, level / kSlackDiv +
+// kSlackRows: room for a group that gains particles until the next full sort
+// (empty rows above gtop cost memory only).
+constexpr int kSlackDiv = 8;
+constexpr int kSlackRows = 3;
+// Rows of the level above the group's mean particles per lane: each spares
+// some of the fuller cells' strangers and adds a partly filled row. One and
+// two rows measured 9.32 and 9.34 ms per step against 9.30 at 128^3 x 64, and
+// 0.682 and 0.687 against 0.682 at 64^3 x 16.
+constexpr int kLevelRows = 0;
 
 constexpr int kTileX = 2;
 constexpr int kTileY = 4;
@@ -50,7 +68,7 @@ struct TileGeom {
 struct TileArgs {
   TileGeom t;
   const int* goff;  // first slot of each group
-  const int* gmax;  // slots per lane of each group
+  const int* gtop;  // rows of each group up to the last one that holds a particle
 };
 
 // Group and lane of an interior cell (absolute indices), -1 outside the interior.
@@ -142,40 +160,88 @@ __device__ __forceinline__ int refill_reserve(const SourceParams& sp, const Geom
   return need > 0 ? need + need / 8 + 4 : 0;
 }
 
-// One warp per group: gmax = largest (stayers + movers) count of its 32
-// lanes, or a lane's refill reserve when that is larger, plus a sixteenth and
-// two rows of slack: the fullest columns then take the next re-layouts'
-// arrivals in holes instead of spilling them to the slot-order tail.
-__global__ void group_size_kernel(Geom g, TileGeom t, const int* __restrict__ stay,
-                                  const int* __restrict__ moved, SourceParams refill, int* gmax,
-                                  int* gcap) {
-  const int G = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// Inclusive sum over the lanes of a warp.
+__device__ __forceinline__ int warp_scan(int v) {
   const int lane = threadIdx.x & 31;
-  if (G >= t.ngroups) return;
-  const int home = home_key(g, t, G, lane);
-  int c = home >= 0 ? stay[home] + moved[home] : 0;
-  c = max(c, refill_reserve(refill, g, t, G, lane));
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) c = max(c, __shfl_xor_sync(0xffffffffu, c, o));
-  if (c > 0) c += c / kSlackDiv + kSlackRows;
-  if (lane == 0) {
-    gmax[G] = c;
-    gcap[G] = c * kLanes;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += y;
   }
+  return v;
+}
+__device__ __forceinline__ int warp_sum(int v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
 }
 
-// Marks the padding slots of every lane column empty.
-template <typename CellArray>
-__global__ void group_pad_kernel(Geom g, TileGeom t, const int* __restrict__ stay,
-                                 const int* __restrict__ moved, const int* __restrict__ goff,
-                                 const int* __restrict__ gmax, CellArray cell) {
+// The level of a group of n particles: the rows that hold them when every lane
+// is filled equally, plus kLevelRows.
+__device__ __forceinline__ int group_level(int n) { return n > 0 ? (n + kLanes - 1) / kLanes + kLevelRows : 0; }
+
+// One warp per group, from the (stayers + movers) counts of its 32 cells: the
+// level (into gtop), gmax = the level of the group with every lane's refill
+// reserve counted, plus the slack, and where the group's strangers go: the
+// slots free below the level, numbered lane by lane (NewLayout::free).
+__global__ void group_size_kernel(Geom g, TileGeom t, const int* __restrict__ stay,
+                                  const int* __restrict__ moved, SourceParams refill, int* gmax,
+                                  int* gtop, int2* free, int* gcap) {
   const int G = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (G >= t.ngroups) return;
   const int home = home_key(g, t, G, lane);
   const int c = home >= 0 ? stay[home] + moved[home] : 0;
+  const int level = group_level(warp_sum(c));
+  const int room = group_level(warp_sum(max(c, refill_reserve(refill, g, t, G, lane))));
+  const int rows = room > 0 ? room + room / kSlackDiv + kSlackRows : 0;
+  const int free_below = max(level - c, 0);
+  free[G * kLanes + lane] = make_int2(warp_scan(free_below) - free_below, min(c, level));
+  if (lane == 0) {
+    gmax[G] = rows;
+    gtop[G] = level;
+    gcap[G] = rows * kLanes;
+  }
+}
+
+// Marks the slots of every lane column above its own particles empty (the
+// strangers among them are written afterwards).
+template <typename CellArray>
+__global__ void group_pad_kernel(Geom g, TileGeom t, const int* __restrict__ stay,
+                                 const int* __restrict__ moved, const int* __restrict__ goff,
+                                 const int* __restrict__ gmax, const int* __restrict__ gtop, CellArray cell) {
+  const int G = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (G >= t.ngroups) return;
+  const int home = home_key(g, t, G, lane);
+  const int c = min(home >= 0 ? stay[home] + moved[home] : 0, gtop[G]);
   const int m = gmax[G], base = goff[G];
   for (int r = c; r < m; ++r) cell[base + r * kLanes + lane] = -1;
+}
+
+// The new layout of a full sort, as the scatter kernels need it.
+struct NewLayout {
+  const int* goff;
+  const int* level;   // per group (group_size_kernel's gtop)
+  const int2* free;   // per lane of each group: its first stranger's number in the group, its first free row
+  const int* stay;    // per cell: stayers
+  int* cursor;        // per cell: movers placed so far
+  int* gcursor;       // per group: strangers placed so far
+};
+
+// Slot of the particle ranked `rank` of the cell of group G, lane l: its own
+// column below the level, else the group's next free slot (the slots below
+// the level hold the whole group, so every stranger finds one).
+__device__ __forceinline__ int layout_slot(const NewLayout& nl, int G, int l, int rank) {
+  const int base = nl.goff[G];
+  if (rank < nl.level[G]) return base + rank * kLanes + l;
+  const int q = atomicAdd(nl.gcursor + G, 1);
+  const int2* f = nl.free + G * kLanes;
+  int b = 0;  // the last lane whose strangers start at or before number q: it has free slots
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1)
+    if (f[b + s].x <= q) b += s;
+  return base + (f[b].y + q - f[b].x) * kLanes + b;
 }
 
 template <typename real>
@@ -188,13 +254,12 @@ __device__ __forceinline__ void copy_particle(const Parts<real>& P, int s, const
 // a mover goes after the stayers of its new cell.
 template <typename real>
 __global__ void tiled_scatter_kernel(Parts<real> P, Geom g, TileGeom t, const int* __restrict__ goff_old,
-                                     const int* __restrict__ gmax_old, const int* __restrict__ goff_new,
-                                     const int* __restrict__ stay, int* cursor, Parts<real> Q) {
+                                     const int* __restrict__ gmax_old, NewLayout nl, Parts<real> Q) {
   const int G = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (G >= t.ngroups) return;
   const int home = home_key(g, t, G, lane);
-  const int base = goff_old[G], m = gmax_old[G], nbase = goff_new[G];
+  const int base = goff_old[G], m = gmax_old[G];
   int rnew = 0;
   constexpr int U = 4;  // rows whose loads are in flight together
   for (int r0 = 0; r0 < m; r0 += U) {
@@ -217,13 +282,12 @@ __global__ void tiled_scatter_kernel(Parts<real> P, Geom g, TileGeom t, const in
       if (key < 0) continue;
       int d;
       if (key == home) {
-        d = nbase + rnew * kLanes + lane;
+        d = layout_slot(nl, G, lane, rnew);
         ++rnew;
       } else {
         int l2;
         const int G2 = group_of_key(g, t, key, l2);
-        const int rank = stay[key] + atomicAdd(cursor + key, 1);
-        d = goff_new[G2] + rank * kLanes + l2;
+        d = layout_slot(nl, G2, l2, nl.stay[key] + atomicAdd(nl.cursor + key, 1));
       }
       Q.cell[d] = cell[u];
 #pragma unroll
@@ -237,8 +301,7 @@ __global__ void tiled_scatter_kernel(Parts<real> P, Geom g, TileGeom t, const in
 
 template <typename real>
 __global__ void append_scatter_kernel(Parts<real> P, int first, const int* __restrict__ count, Geom g,
-                                      TileGeom t, const int* __restrict__ goff_new,
-                                      const int* __restrict__ stay, int* cursor, Parts<real> Q) {
+                                      TileGeom t, NewLayout nl, Parts<real> Q) {
   const int n = *count;
   for (int s = first + blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
     const int c = P.cell[s];
@@ -246,8 +309,7 @@ __global__ void append_scatter_kernel(Parts<real> P, int first, const int* __res
     if (key < 0) continue;
     int l2;
     const int G2 = group_of_key(g, t, key, l2);
-    const int rank = stay[key] + atomicAdd(cursor + key, 1);
-    copy_particle(P, s, Q, goff_new[G2] + rank * kLanes + l2, c);
+    copy_particle(P, s, Q, layout_slot(nl, G2, l2, nl.stay[key] + atomicAdd(nl.cursor + key, 1)), c);
   }
 }
 

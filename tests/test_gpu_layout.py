@@ -1,0 +1,64 @@
+"""The tiled particle layout (rows sized for a group's mean lane, the excess of
+fuller cells in other lanes' free slots) against the slot-order push, where it
+can go wrong: crowded and empty cells, ragged sides, groups that outgrow their
+rows between two full sorts."""
+import numpy as np
+import pytest
+
+from plasmasim_b200 import ELECTRON, ION, Pic3D, PicConfig
+from util import rel_norm
+
+pytestmark = pytest.mark.gpu
+
+
+def crowd(n, rng, speed):
+    """Rows over an (nx, ny, nz) grid: a few cells with up to 300 particles
+    (one of them the last lane of the last group), a thin background; all
+    drifting along x at `speed`, so that at 0.9 they leave their columns
+    within six steps."""
+    cells = [tuple(2 + int(rng.integers(m)) for m in n) for _ in range(6)]
+    cells.append(tuple(m + 1 for m in n))
+    xyz = [np.array(c) + rng.random((k, 3)) for c, k in zip(cells, (300, 100, 33, 32, 31, 1, 65))]
+    xyz.append(2 + rng.random((40, 3)) * np.array(n))
+    xyz = np.concatenate(xyz)
+    v = rng.normal(0, 0.02, xyz.shape) + [speed, 0, 0.05]
+    return np.column_stack([xyz, v, np.full(len(xyz), 0.01 / 4)])
+
+
+def context(n, precision, slot_order):
+    P = Pic3D(PicConfig.normalized(*n, 4, precision=precision, diag_every_step=0, sort_interval=1,
+                                   add_interval=1000, slot_order=slot_order, capacity=200000))
+    P.init_grid()
+    return P
+
+
+def ordered(rows):
+    return rows[np.lexsort(rows.T[::-1])]
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("n", [(8, 8, 8), (5, 7, 31), (6, 5, 33), (9, 6, 64)])
+@pytest.mark.parametrize("speed", [0.1, 0.9])
+def test_layout_keeps_particles_and_their_sums(n, speed, precision):
+    rng = np.random.default_rng(sum(n) + int(10 * speed))
+    rows = [crowd(n, rng, speed) for _ in range(2)]
+    with context(n, precision, 0) as T, context(n, precision, 1) as S:
+        for s in (ION, ELECTRON):
+            T.set_particles(s, rows[s])
+            S.set_particles(s, rows[s])
+        T.sorting()
+        for s in (ION, ELECTRON):  # a sort moves records, bit for bit
+            assert np.array_equal(ordered(T.particles(s)), ordered(S.particles(s)))
+        for _ in range(8):  # a re-layout in every second step or so
+            T.step(1)
+            S.step(1)
+            if precision == 64:  # each step rounds a value a few times: 8 steps stay within 1e-12 of it
+                g, h = T.grid(), S.grid()
+                for q in range(18):
+                    assert rel_norm(g[..., q], h[..., q]) < 1e-11 or np.abs(g[..., q] - h[..., q]).max() < 1e-15
+        for s in (ION, ELECTRON):
+            a, b = T.particles(s), S.particles(s)
+            assert len(a) == len(b)
+            if precision == 64:
+                assert rel_norm(ordered(np.round(a, 9)), ordered(np.round(b, 9))) < 1e-8
+        assert T.status()[0] == 0
