@@ -8,6 +8,7 @@
 #include <cstring>
 #include <map>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 #include <cudaTypedefs.h>
@@ -105,7 +106,7 @@ struct pic_ctx {
   size_t scan_tmp_len = 0;
   long long ncells = 0;
   // diagnostics
-  double* acc = nullptr;        // 33 thrust/energy sums, then 4 Gauss-law values
+  double* acc = nullptr;        // 33 thrust/energy sums, 4 Gauss-law values (40), thrust_kernel's sums and ticket (44)
   unsigned long long* maxbits = nullptr;
   double* fave = nullptr;       // 27
   // Poisson cleaning (renew_phi3): two interior-sized work arrays, the sine
@@ -1144,45 +1145,98 @@ int do_init_particles(pic_ctx* c) {
 }
 
 // -------------------------------------------------------- diagnostics
-template <typename real>
-int do_thrust_sums(pic_ctx* c) {
-  CK(cudaMemsetAsync(c->acc, 0, sizeof(double) * 33, c->stream));
-  const pic_config& k = c->cfg;
-  CellBox b{};
-  const int n3[3] = {c->g.gnx, c->g.gny, k.nz};  // PROCESS_N Grid_N (:4971-4973)
-  for (int a = 0; a < 3; ++a) {
-    b.lo[a] = n3[a] * 0.2;
-    b.hi[a] = n3[a] * 0.8;
+// Where `past`, false and then true along the cells i + f of an axis, changes:
+// the cell c with past(c + f) for f > f0 only (f0 = -1: for every f of it), from
+// a first guess of c. Offsets are non-negative, so their bits order them.
+template <typename real, typename Past>
+void box_face(int guess, Past past, int& c, real& f0) {
+  using bits = typename std::conditional<sizeof(real) == 4, uint32_t, uint64_t>::type;
+  const auto value = [](bits b) {
+    real f;
+    std::memcpy(&f, &b, sizeof(f));
+    return f;
+  };
+  const real one = (real)1;
+  bits top;  // the last offset below 1
+  std::memcpy(&top, &one, sizeof(top));
+  --top;
+  for (c = guess - 2; c < guess + 4 && !past((double)c + (double)value(top));) ++c;  // the guess is one off at most
+  f0 = (real)-1;
+  if (past((double)c)) return;
+  bits lo = 0, hi = top;  // past(value(hi)), not past(value(lo))
+  while (hi - lo > 1) {
+    const bits mid = lo + (hi - lo) / 2;
+    (past((double)c + (double)value(mid)) ? hi : lo) = mid;
   }
-  b.e0 = k.e0;
-  b.inv_mu0 = 1.0 / k.mu0;
-  b.ox = c->g.ox;
-  b.oy = c->g.oy;
-  const long long nint = (long long)k.nx * k.ny * k.nz;
-  field_energy_kernel<real><<<particle_blocks(nint), kThreads, 0, c->stream>>>(fields<real>(c), c->g, b, c->acc);
-  CKL();
+  f0 = value(lo);
+}
+
+// thrust_f's sums into c->acc; with `mean`, thrust_fave's running mean too.
+template <typename real>
+int do_thrust_sums(pic_ctx* c, bool mean = false) {
+  const pic_config& k = c->cfg;
+  const Geom& g = c->g;
+  ThrustArgs<real> a{};
+  const int n3[3] = {g.gnx, g.gny, k.nz};  // PROCESS_N Grid_N (:4971-4973)
+  const int o3[3] = {g.ox, g.oy, 0};
+  for (int q = 0; q < 3; ++q) {
+    a.cells.lo[q] = n3[q] * 0.2;
+    a.cells.hi[q] = n3[q] * 0.8;
+    // the reference compares off + x with 0.2 N dx and 0.8 N dx in FP64
+    const double lo = (double)n3[q] * k.dx * 0.2, hi = (double)n3[q] * k.dx * 0.8, off = (double)o3[q] * k.dx;
+    box_face<real>((int)std::floor(n3[q] * 0.2) - o3[q], [=](double x) { return off + x * k.dx > lo; }, a.box[q].cl,
+                   a.box[q].fl);
+    box_face<real>((int)std::floor(n3[q] * 0.8) - o3[q], [=](double x) { return !(off + x * k.dx < hi); },
+                   a.box[q].ch, a.box[q].fh);
+  }
+  a.cells.e0 = k.e0;
+  a.cells.inv_mu0 = 1.0 / k.mu0;
+  a.cells.ox = g.ox;
+  a.cells.oy = g.oy;
+  a.F = fields<real>(c);
+  a.g = g;
+  a.tg = c->tg;
+  a.vec = sizeof(real) == 4 && g.gz % 4 == 0;
+  // tiles whose cells [2 + T t, 2 + T (t + 1)) lie in the box's cells or next to them
+  const int tile[3] = {kTileX, kTileY, kLanes}, nt[3] = {c->tg.ntx, c->tg.nty, c->tg.ntz};
+  int per = 1;
+  for (int q = 0; q < 3; ++q) {
+    const int first = std::max(0, a.box[q].cl - 3), last = a.box[q].ch - 1;  // interior cells from 0
+    a.near.lo[q] = std::min(nt[q], first / tile[q]);
+    a.near.n[q] = last < first ? 0 : std::max(0, std::min(nt[q] - 1, last / tile[q]) - a.near.lo[q] + 1);
+    per *= a.near.n[q];
+  }
+  long long far = 1;
   for (int s = 0; s < 2; ++s) {
-    if (slot_bound(c, s) == 0) continue;
-    ThrustParams tp{};
-    tp.xlo = (double)c->g.gnx * k.dx * 0.2; tp.xhi = (double)c->g.gnx * k.dx * 0.8;
-    tp.ylo = (double)c->g.gny * k.dx * 0.2; tp.yhi = (double)c->g.gny * k.dx * 0.8;
-    tp.zlo = (double)k.nz * k.dx * 0.2; tp.zhi = (double)k.nz * k.dx * 0.8;
-    tp.ox = (double)c->g.ox * k.dx;
-    tp.oy = (double)c->g.oy * k.dx;
-    tp.dx = k.dx;
-    const double sg = s == 0 ? 1.0 : -1.0;
+    ThrustStore<real>& st = a.sp[s];
     const double w = k.q * species_weight(c) * k.dx * k.dx * k.dx;
-    const int o = s == 0 ? 3 : 9;
-    for (int q = 0; q < 3; ++q) { tp.idx[q] = q; tp.scale[q] = sg * w; }
-    for (int q = 0; q < 6; ++q) { tp.idx[3 + q] = o + q; tp.scale[3 + q] = sg * w; }
-    tp.idx[9] = 27 + (s == 0 ? 2 : 3);
-    tp.scale[9] = 0.5 * species_mass(c, s) * species_weight(c) * k.dx * k.dx * k.dx;
-    thrust_particles_kernel<real><<<particle_blocks(slot_bound(c, s)), kThreads, 0, c->stream>>>(
-        parts<real>(c, s), c->sp[s].count_dev, fields<real>(c), c->g, tp, c->acc);
+    st.P = parts<real>(c, s);
+    st.count = c->sp[s].count_dev;
+    st.goff = c->goff[s][c->lay[s]];
+    st.gtop = c->gtop[s];
+    st.layout = c->layout[s];
+    st.near = c->layout[s] ? per : 0;
+    st.tail = c->layout[s] ? (int)c->tiled_end[s] : 0;
+    st.scale = s == 0 ? w : -w;
+    st.ke = 0.5 * species_mass(c, s) * species_weight(c) * k.dx * k.dx * k.dx;
+    far = std::max(far, c->layout[s] ? (long long)nt[0] * nt[1] * nt[2] - per : (slot_bound(c, s) + kThreads - 1) / kThreads);
+  }
+  a.raw = c->acc + 44;
+  a.ticket = (unsigned*)(c->acc + 60);
+  a.acc = c->acc;
+  a.fave = mean && !c->has_xport ? c->fave : nullptr;
+  a.nfar = (int)std::min<long long>(far, 148 * 2);
+  const int nodes = (int)std::min<long long>(grid_blocks((long long)k.nx * k.ny * k.nz), 148);
+  const size_t smem = sizeof(real) == 4 ? 6 * ThrustPlan::WN * sizeof(float) : 0;
+  thrust_kernel<real><<<a.sp[0].near + a.sp[1].near + 2 * a.nfar + nodes, kThreads, smem, c->stream>>>(a);
+  CKL();
+  if (!c->has_xport) return PIC_OK;
+  // thrust_f's MPI_Allreduce of F and E over the ranks (:5103-5108)
+  if (c->xport.allreduce_sum_f64(c->xport.user, c->acc, 33, (void*)c->stream) != 0) return PIC_ERR_COMM;
+  if (mean) {
+    fave_accumulate_kernel<<<1, 32, 0, c->stream>>>(c->acc, c->fave, 1.0 / 500.0);
     CKL();
   }
-  // thrust_f's MPI_Allreduce of F and E over the ranks (:5103-5108)
-  if (c->has_xport && c->xport.allreduce_sum_f64(c->xport.user, c->acc, 33, (void*)c->stream) != 0) return PIC_ERR_COMM;
   return PIC_OK;
 }
 
@@ -1262,9 +1316,7 @@ int do_step(pic_ctx* c) {
   CKR(phase_mark(c, PH_FIELD));
   if (c->cfg.diag_every_step) {
     CKR(phase_mark(c, PH_DIAG));
-    CKR(do_thrust_sums<real>(c));
-    fave_accumulate_kernel<<<1, 32, 0, c->stream>>>(c->acc, c->fave, 1.0 / 500.0);
-    CKL();
+    CKR(do_thrust_sums<real>(c, true));
     CKR(phase_mark(c, PH_DIAG));
   }
   c->c_add++;
@@ -1872,7 +1924,7 @@ int pic_sort(pic_ctx* c) {
 
 int pic_thrust_f(pic_ctx* c, double* F27, double* E6) {
   CKR(check_ctx(c));
-  CKR(DISPATCH(c, do_thrust_sums)(c));
+  CKR(DISPATCH(c, do_thrust_sums)(c, false));
   double h[33];
   CK(cudaMemcpyAsync(h, c->acc, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));

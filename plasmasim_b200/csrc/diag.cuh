@@ -5,6 +5,8 @@
 
 #include "common.cuh"
 #include "particles.cuh"
+#include "push_tiled.cuh"
+#include "tiled.cuh"
 
 namespace pb {
 
@@ -33,49 +35,31 @@ __device__ __forceinline__ void block_reduce_add(double (&v)[N], double* out, co
   }
 }
 
-struct ThrustParams {
-  double xlo, xhi, ylo, yhi, zlo, zhi;  // open box (0.2 N dx, 0.8 N dx) per axis (:4986-4988)
-  double ox, oy;                        // myrank_x Grid_Nx dx, myrank_y Grid_Ny dx (:4984-4985)
-  double dx;
-  int idx[10];      // output slot per partial sum (F0..F2, F[o..o+5], E[oe])
-  double scale[10];
+// thrust_f's central box on one axis, (0.2 N dx, 0.8 N dx) open (:4984-4988),
+// as cells and offsets: a particle (i, f) is above its lower face when i > cl
+// or i == cl and f > fl, below its upper one when i < ch or i == ch and
+// f <= fh. The host finds the offsets at which the reference's comparison of
+// x = (i + f) dx in FP64 changes, so the result is the same for every (i, f).
+template <typename real>
+struct BoxAxis {
+  int cl, ch;
+  real fl, fh;
 };
 
-// Particle part of thrust_f (:4984-5101) for one species with flag > 0:
-// sums over particles inside the central box of (E + v x B), E, v x B and v^2.
+// One species' store as the sums walk it: the rows in use of every group of
+// the tiled layout, then the slots from `tail` to the count.
 template <typename real>
-__global__ void __launch_bounds__(256) thrust_particles_kernel(Parts<real> P, const int* __restrict__ count,
-                                                               Fields<real> F, Geom g, ThrustParams tp,
-                                                               double* acc) {
-  double s[10];
-#pragma unroll
-  for (int q = 0; q < 10; ++q) s[q] = 0.0;
-  const int n = *count;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-    const int c = P.cell[t];
-    if (c < 0) continue;
-    int i, j, k;
-    unpack_cell(c, i, j, k);
-    const real fx = P.o[0][t], fy = P.o[1][t], fz = P.o[2][t];
-    const double x = ((double)i + (double)fx) * tp.dx;
-    const double y = ((double)j + (double)fy) * tp.dx;
-    const double z = ((double)k + (double)fz) * tp.dx;
-    if (!(tp.ox + x < tp.xhi && tp.ox + x > tp.xlo && tp.oy + y < tp.yhi && tp.oy + y > tp.ylo && z < tp.zhi &&
-          z > tp.zlo))
-      continue;
-    if (!stencil_ok(g, i, j, k)) continue;
-    const Axis<real> X = axis_weights(i, fx), Y = axis_weights(j, fy), Z = axis_weights(k, fz);
-    const Gathered<real> e = gather6(F, g, X, Y, Z);
-    const double ex = e.ex, ey = e.ey, ez = e.ez, bx = e.bx, by = e.by, bz = e.bz;
-    const double vx = P.v[0][t], vy = P.v[1][t], vz = P.v[2][t];
-    const double lx = vy * bz - vz * by, ly = vz * bx - vx * bz, lz = vx * by - vy * bx;
-    s[0] += ex + lx; s[1] += ey + ly; s[2] += ez + lz;
-    s[3] += ex; s[4] += ey; s[5] += ez;
-    s[6] += lx; s[7] += ly; s[8] += lz;
-    s[9] += vx * vx + vy * vy + vz * vz;
-  }
-  block_reduce_add<10>(s, acc, tp.idx, tp.scale);
-}
+struct ThrustStore {
+  Parts<real> P;
+  const int* goff;
+  const int* gtop;
+  int layout;        // 0: every slot is in the tail
+  int near;          // near tiles, 0 without a layout
+  int tail;
+  const int* count;
+  double scale;      // s_p q n dx^3
+  double ke;         // m n dx^3 / 2
+};
 
 struct CellBox {
   double lo[3], hi[3];   // open box on k-2, l-2, m-2 (:4965-4967)
@@ -83,25 +67,247 @@ struct CellBox {
   double e0, inv_mu0;
 };
 
-// Field part of thrust_f (:4963-4973): E[0] = sum e0 |E|^2 / 2, E[1] = sum |B|^2 / (2 mu0)
-// over interior nodes of the central box (no volume factor, as in the reference).
 template <typename real>
-__global__ void __launch_bounds__(256) field_energy_kernel(Fields<real> F, Geom g, CellBox b, double* acc) {
-  double s[2] = {0.0, 0.0};
-  const int nint = g.nx * g.ny * g.nz;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nint; t += gridDim.x * blockDim.x) {
-    const int m = t % g.nz, l = (t / g.nz) % g.ny, k = t / (g.nz * g.ny);
-    const int kg = b.ox + k, lg = b.oy + l;
-    if (!(kg < b.hi[0] && kg > b.lo[0] && lg < b.hi[1] && lg > b.lo[1] && m < b.hi[2] && m > b.lo[2])) continue;
-    const int n = (k + 2) * g.sx + (l + 2) * g.gz + (m + 2);
-    const double ex = F.f[F_EX][n], ey = F.f[F_EY][n], ez = F.f[F_EZ][n];
-    const double bx = F.f[F_BX][n], by = F.f[F_BY][n], bz = F.f[F_BZ][n];
-    s[0] += ex * ex + ey * ey + ez * ez;
-    s[1] += bx * bx + by * by + bz * bz;
+struct ThrustArgs {
+  ThrustStore<real> sp[2];
+  Fields<real> F;
+  Geom g;
+  BoxAxis<real> box[3];
+  CellBox cells;
+  double* raw;       // 7 sums of each species (E, v x B, v^2), 2 of the fields; zero between launches
+  unsigned* ticket;  // blocks done; zero between launches
+  TileGeom tg;
+  struct { int lo[3], n[3]; } near;  // tiles that reach into the box
+  int nfar;          // blocks per species for the rest of its store
+  bool vec;          // FP32 planes whose rows are multiples of 16 bytes
+  double* acc;       // F[27], E[6]
+  double* fave;      // when set, the running mean gains F / 500 (thrust_fave :5265-5267)
+};
+
+constexpr int kThrustRaw = 16;
+
+template <typename real>
+__device__ __forceinline__ bool in_axis(const BoxAxis<real>& b, int i, real f) {
+  return (i > b.cl || (i == b.cl && f > b.fl)) && (i < b.ch || (i == b.ch && f <= b.fh));
+}
+
+// E and B at a particle: from the tile's window when its stencil lies in it.
+struct ThrustWin {
+  const float* fw;   // null without one
+  int x0, y0, z0;
+};
+using ThrustPlan = PushSmem<float>;
+
+__device__ __forceinline__ Gathered<double> thrust_gather(const ThrustWin&, const Fields<double>& F, const Geom& g,
+                                                          const Axis<double>& X, const Axis<double>& Y,
+                                                          const Axis<double>& Z, int, int, int) {
+  return gather6(F, g, X, Y, Z);
+}
+__device__ __forceinline__ Gathered<float> thrust_gather(const ThrustWin& w, const Fields<float>& F, const Geom& g,
+                                                         const Axis<float>& X, const Axis<float>& Y,
+                                                         const Axis<float>& Z, int i, int j, int k) {
+  using S = ThrustPlan;
+  if (w.fw && i - 1 >= w.x0 && i + 1 < w.x0 + S::WX && j - 1 >= w.y0 && j + 1 < w.y0 + S::WY && k - 1 >= w.z0 &&
+      k + 1 < w.z0 + S::WZ)
+    return gather6_win<S::WY, S::WZ, S::WN>(w.fw, w.x0, w.y0, w.z0, X, Y, Z);
+  return gather6(F, g, X, Y, Z);
+}
+
+template <typename real>
+__device__ __forceinline__ bool in_box(const ThrustArgs<real>& a, const Rec<real>& q, int& i, int& j, int& k) {
+  unpack_cell(q.cell, i, j, k);
+  return in_axis(a.box[0], i, q.o[0]) && in_axis(a.box[1], j, q.o[1]) && in_axis(a.box[2], k, q.o[2]);
+}
+
+// The terms of thrust_f (:4984-5101) of a particle in the box's cell (i, j, k).
+template <typename real>
+__device__ __forceinline__ void thrust_terms(const ThrustArgs<real>& a, const ThrustWin& win, int i, int j, int k,
+                                             const Rec<real>& q, double (&s)[7]) {
+  if (!stencil_ok(a.g, i, j, k)) return;
+  const Gathered<real> e =
+      thrust_gather(win, a.F, a.g, axis_weights(i, q.o[0]), axis_weights(j, q.o[1]), axis_weights(k, q.o[2]), i, j, k);
+  const double vx = q.v[0], vy = q.v[1], vz = q.v[2];
+  const double bx = e.bx, by = e.by, bz = e.bz;
+  s[0] += (double)e.ex;
+  s[1] += (double)e.ey;
+  s[2] += (double)e.ez;
+  s[3] += vy * bz - vz * by;
+  s[4] += vz * bx - vx * bz;
+  s[5] += vx * by - vy * bx;
+  s[6] += vx * vx + vy * vy + vz * vz;
+}
+
+template <typename real>
+__device__ __forceinline__ Rec<real> empty_rec() {
+  return Rec<real>{-1, {(real)0, (real)0, (real)0}, {(real)0, (real)0, (real)0}};
+}
+// Record A of particle t, its velocity left zero.
+__device__ __forceinline__ Rec<float> load_record_a(const Parts<float>& P, int t) {
+  const float4 a = reinterpret_cast<const float4*>(P.ra)[t];
+  return Rec<float>{__float_as_int(a.x), {a.y, a.z, a.w}, {0.f, 0.f, 0.f}};
+}
+__device__ __forceinline__ Rec<double> load_record_a(const Parts<double>& P, int t) {
+  const double2* a = reinterpret_cast<const double2*>(P.ra + 4 * (long long)t);
+  const double2 a0 = a[0], a1 = a[1];
+  return Rec<double>{__double2loint(a0.x), {a0.y, a1.x, a1.y}, {0., 0., 0.}};
+}
+
+// thrust_f (:4963-5101): E, v x B and v^2 summed over the particles of each
+// species inside the central box, the field energies over its nodes (no volume
+// factor, as in the reference); the last block to finish forms F and E, adds
+// F / 500 to the running mean and clears the sums.
+//
+// A grid of three kinds of blocks, the dearest first: one per species and tile
+// that reaches into the box (`near`, a box of tiles), `nfar` per species that
+// walk the other tiles and the tail, the rest over the nodes. A near block
+// stages E and B of its tile in shared memory as the push does (FP32); one
+// warp walks a group's rows in use, U records in flight. In a far tile only
+// record A is read, and B of the rare particle that has come into the box.
+//
+// Bound by instruction issue over the near tiles' particles (the gathers and
+// FP64 sums; reading every record A, 16 bytes a particle, takes a third of the
+// time). The box test is one of cells and FP32 offsets; E + v x B, which the
+// reference sums beside E and v x B, is formed from the two sums; both
+// species, the fields and the mean share one launch. Per step, a kernel each
+// for the fields and the species with a test in FP64 per particle -> this:
+// 0.162 -> 0.094 ms at 64^3 x 16, 0.063 -> 0.023 at 32^3 x 8, 0.469 ->
+// 0.319 at 96 x 96 x 128 x 16. (Blocks that took tiles from an atomic
+// counter: 0.099, 0.034, 0.316.)
+template <typename real>
+__global__ void __launch_bounds__(256, 3) thrust_kernel(const __grid_constant__ ThrustArgs<real> a) {
+  using S = ThrustPlan;
+  constexpr int U = sizeof(real) == 4 ? 4 : 2;
+  constexpr bool kWin = sizeof(real) == 4;
+  extern __shared__ __align__(16) float thrust_win[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const Geom& g = a.g;
+  const int nnear = a.sp[0].near + a.sp[1].near;
+  double s[7] = {0., 0., 0., 0., 0., 0., 0.};
+  int ph;
+  if ((int)blockIdx.x < nnear) {
+    ph = (int)blockIdx.x >= a.sp[0].near;
+    const ThrustStore<real>& st = a.sp[ph];
+    const Parts<real>& P = st.P;
+    int b = ph ? (int)blockIdx.x - a.sp[0].near : (int)blockIdx.x;
+    const int tz = a.near.lo[2] + b % a.near.n[2];
+    b /= a.near.n[2];
+    const int ty = a.near.lo[1] + b % a.near.n[1], tx = a.near.lo[0] + b / a.near.n[1];
+    ThrustWin win{nullptr, tx * kTileX, ty * kTileY, tz * kLanes};
+    const int G = ((tx * a.tg.nty + ty) * a.tg.ntz + tz) * (kTileX * kTileY) + warp;
+    const int base = st.goff[G] + lane, m = st.gtop[G];
+    Rec<real> q[U];
+    const auto fetch = [&](int r0) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        q[u] = r0 + u < m ? load_records(P, base + (r0 + u) * kLanes) : empty_rec<real>();
+    };
+    fetch(0);
+    if constexpr (kWin) {
+      if (a.vec) fill_win<S::WX, S::WY, S::WZ, true>(thrust_win, a.F, g, win.x0, win.y0, win.z0);
+      else fill_win<S::WX, S::WY, S::WZ, false>(thrust_win, a.F, g, win.x0, win.y0, win.z0);
+      win.fw = thrust_win;
+      __syncthreads();
+    }
+    for (int r0 = 0; r0 < m; r0 += U) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        int i, j, k;
+        if (q[u].cell >= 0 && in_box(a, q[u], i, j, k)) thrust_terms(a, win, i, j, k, q[u], s);
+      }
+      fetch(r0 + U);
+    }
+  } else if ((int)blockIdx.x < nnear + 2 * a.nfar) {
+    ph = (int)blockIdx.x - nnear >= a.nfar;
+    const ThrustStore<real>& st = a.sp[ph];
+    const Parts<real>& P = st.P;
+    const ThrustWin none{nullptr, 0, 0, 0};
+    const int f = (int)blockIdx.x - nnear - ph * a.nfar;
+    if (st.layout) {  // its other tiles
+      const int ntiles = a.tg.ntx * a.tg.nty * a.tg.ntz;
+      for (int tile = f; tile < ntiles; tile += a.nfar) {
+        const int tz = tile % a.tg.ntz, ty = (tile / a.tg.ntz) % a.tg.nty, tx = tile / (a.tg.ntz * a.tg.nty);
+        if ((unsigned)(tx - a.near.lo[0]) < (unsigned)a.near.n[0] && (unsigned)(ty - a.near.lo[1]) < (unsigned)a.near.n[1] &&
+            (unsigned)(tz - a.near.lo[2]) < (unsigned)a.near.n[2])
+          continue;
+        const int G = tile * (kTileX * kTileY) + warp;
+        const int base = st.goff[G] + lane, m = st.gtop[G];
+        constexpr int UF = 2 * U;
+        for (int r0 = 0; r0 < m; r0 += UF) {
+          Rec<real> q[UF];
+#pragma unroll
+          for (int u = 0; u < UF; ++u)
+            q[u] = r0 + u < m ? load_record_a(P, base + (r0 + u) * kLanes) : empty_rec<real>();
+#pragma unroll
+          for (int u = 0; u < UF; ++u) {
+            int i, j, k;
+            if (q[u].cell >= 0 && in_box(a, q[u], i, j, k))  // it has come in from outside
+              thrust_terms(a, none, i, j, k, load_records(P, base + (r0 + u) * kLanes), s);
+          }
+        }
+      }
+    }
+    const int n = *st.count;
+    for (int t = st.tail + f * blockDim.x + threadIdx.x; t < n; t += a.nfar * blockDim.x) {
+      const Rec<real> q = load_records(P, t);
+      int i, j, k;
+      if (q.cell >= 0 && in_box(a, q, i, j, k)) thrust_terms(a, none, i, j, k, q, s);
+    }
+  } else {
+    ph = 2;
+    const CellBox& b = a.cells;
+    const int nint = g.nx * g.ny * g.nz, first = nnear + 2 * a.nfar;
+    for (int t = ((int)blockIdx.x - first) * blockDim.x + threadIdx.x; t < nint; t += (gridDim.x - first) * blockDim.x) {
+      const int m = t % g.nz, l = (t / g.nz) % g.ny, k = t / (g.nz * g.ny);
+      const int kg = b.ox + k, lg = b.oy + l;
+      if (!(kg < b.hi[0] && kg > b.lo[0] && lg < b.hi[1] && lg > b.lo[1] && m < b.hi[2] && m > b.lo[2])) continue;
+      const int n = (k + 2) * g.sx + (l + 2) * g.gz + (m + 2);
+      const double ex = a.F.f[F_EX][n], ey = a.F.f[F_EY][n], ez = a.F.f[F_EZ][n];
+      const double bx = a.F.f[F_BX][n], by = a.F.f[F_BY][n], bz = a.F.f[F_BZ][n];
+      s[0] += ex * ex + ey * ey + ez * ez;
+      s[1] += bx * bx + by * by + bz * bz;
+    }
   }
-  const int idx[2] = {27, 28};
-  const double scale[2] = {0.5 * b.e0, 0.5 * b.inv_mu0};
-  block_reduce_add<2>(s, acc, idx, scale);
+  {
+    const bool part = ph < 2;
+    const int idx[7] = {0, 1, part ? 2 : -1, part ? 3 : -1, part ? 4 : -1, part ? 5 : -1, part ? 6 : -1};
+    const double one[7] = {1., 1., 1., 1., 1., 1., 1.};
+    block_reduce_add<7>(s, a.raw + 7 * ph, idx, one);
+  }
+  // the last block's first warp forms the results
+  if (threadIdx.x >= 32) return;
+  unsigned last = 0;
+  if (lane == 0) {
+    __threadfence();
+    last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
+    __threadfence();
+  }
+  if (!__shfl_sync(0xffffffffu, last, 0)) return;
+  const double mine = lane < kThrustRaw ? __ldcg(a.raw + lane) : 0.0;
+  double raw[kThrustRaw];
+#pragma unroll
+  for (int q = 0; q < kThrustRaw; ++q) raw[q] = __shfl_sync(0xffffffffu, mine, q);
+  double f = 0.0;  // F[lane]
+#pragma unroll
+  for (int q = 0; q < 3; ++q)
+    if (lane == q)
+      f = a.sp[0].scale * (raw[q] + raw[3 + q]) + a.sp[1].scale * (raw[7 + q] + raw[10 + q]);
+#pragma unroll
+  for (int q = 0; q < 6; ++q) {
+    if (lane == 3 + q) f = a.sp[0].scale * raw[q];
+    if (lane == 9 + q) f = a.sp[1].scale * raw[7 + q];
+  }
+  if (lane < 27) a.acc[lane] = f;
+  if (a.fave && lane < 27) a.fave[lane] += f * (1.0 / 500.0);
+  if (lane < 6) {
+    double e = 0.0;
+    if (lane == 0) e = 0.5 * a.cells.e0 * raw[14];
+    if (lane == 1) e = 0.5 * a.cells.inv_mu0 * raw[15];
+    if (lane == 2) e = a.sp[0].ke * raw[6];
+    if (lane == 3) e = a.sp[1].ke * raw[13];
+    a.acc[27 + lane] = e;
+  }
+  if (lane < kThrustRaw) a.raw[lane] = 0.0;
+  if (lane == 0) *a.ticket = 0;
 }
 
 // Gauss-law residual r = div4(E) - q (ni - ne)/e0 at cell centres; acc gets
