@@ -310,8 +310,7 @@ int adj_forward_step(pic_ctx* c, AdjRun& R, AdjSnap* rec, bool objective, bool d
     CKL();
   }
   CKR(adj_resolve(c, R, rec));  // waits for the refill's counts while the GPU pushes
-  CKR(do_renew_b<real>(c));
-  CKR(do_fold<real>(c));
+  CKR(do_renew_b_fold<real>(c));
   CKR(do_renew_e<real>(c));
   c->c_add++;
   c->c_thrust++;

@@ -531,24 +531,50 @@ int wrap_planes(pic_ctx* c, const int* ids, int n) {
   for (int q = 0; q < n; ++q) s.p[q] = F.f[ids[q]];
   s.count = n;
   if (c->has_xport) return halo_ghosts<real>(c, s, s, HALO_COPY);
-  wrap_kernel<real><<<grid_blocks(4LL * n * c->g.gy * c->g.gz), kThreads, 0, c->stream>>>(s, c->g, 0);
-  CKL();
-  wrap_kernel<real><<<grid_blocks(4LL * n * c->g.gx * c->g.gz), kThreads, 0, c->stream>>>(s, c->g, 1);
+  wrap_kernel<real><<<grid_blocks(n * layer_items(c->g)), kThreads, 0, c->stream>>>(s, c->g);
   CKL();
   return PIC_OK;
 }
 
+// What rides in renew_b4_2's launch (fields.cuh): nothing, renew_grid's clear
+// of J and n (F_JIX .. F_NE, contiguous), or sr_current2's fold at size 1.
+enum { RIDE_NONE = 0, RIDE_CLEAR = 1, RIDE_FOLD = 2 };
+
 template <typename real>
-int do_renew_b(pic_ctx* c) {
+Rider<real> make_rider(pic_ctx* c, int mode) {
+  Rider<real> r{};
+  r.mode = mode;
+  const Fields<real> F = fields<real>(c);
+  r.clear = (float4*)F.f[F_JIX];  // planes are multiples of 256 bytes
+  r.nclear = (long long)((F_NE - F_JIX + 1) * c->plane_bytes / sizeof(float4));
+  for (int q = 0; q < 8; ++q) r.fold.p[q] = F.f[F_JIX + q];
+  r.fold.count = 8;
+  return r;
+}
+
+int rider_blocks(const pic_ctx* c, int mode) {
+  if (mode == RIDE_NONE) return 0;
+  const long long units = mode == RIDE_CLEAR ? (long long)(F_NE - F_JIX + 1) * (long long)c->plane_bytes / 64 : 8 * layer_items(c->g);
+  return (int)std::min<long long>(grid_blocks(units), 148 * 8);
+}
+
+// renew_b4_2 + sr_b; the update writes the ghost images itself (at size 1).
+template <typename real>
+int do_renew_b(pic_ctx* c, int ride = RIDE_NONE) {
   BParams p{1. / c->cfg.e0 * c->cfg.dt * 0.5 * 0.5, 0.5 * c->cfg.dt, 1.0 / (24.0 * c->cfg.dx)};
+  const bool ghosts = !c->has_xport;
+  Rider<real> rider = make_rider<real>(c, ride);
+  const int extra = rider_blocks(c, ride);
   if (c->staged) {
     constexpr int TX = StShape<real>::TX, TY = StShape<real>::TY;
     const int ty = (c->g.ny + TY - 1) / TY, tz = (c->g.nz + kStZ - 1) / kStZ, tx = (c->g.nx + TX - 1) / TX;
-    renew_b_tma_kernel<real, TX, TY><<<tx * ty * tz, kStThreads, StTile<real>::bytes, c->stream>>>(
-        c->tm_e[0], c->tm_e[1], c->tm_e[2], fields<real>(c), c->g, ramps(c), p, ty, tz, c->err);
+    rider.first = tx * ty * tz;
+    renew_b_tma_kernel<real, TX, TY><<<tx * ty * tz + extra, kStThreads, StTile<real>::bytes, c->stream>>>(
+        c->tm_e[0], c->tm_e[1], c->tm_e[2], fields<real>(c), c->g, ramps(c), p, ty, tz, ghosts, rider, c->err);
   } else {
-    const long long nint = (long long)c->g.nx * c->g.ny * c->g.nz;
-    renew_b_kernel<real><<<grid_blocks(nint), kThreads, 0, c->stream>>>(fields<real>(c), c->g, ramps(c), p);
+    rider.first = grid_blocks((long long)c->g.nx * c->g.ny * c->g.nz);
+    renew_b_kernel<real><<<rider.first + extra, kThreads, 0, c->stream>>>(fields<real>(c), c->g, ramps(c), p, ghosts,
+                                                                         rider);
   }
   CKL();
   if (c->has_xport) {
@@ -563,42 +589,41 @@ int do_renew_b(pic_ctx* c) {
     aux.count = 6;
     return halo_ghosts<real>(c, s, aux, HALO_BTOTAL);
   }
-  wrap_b_kernel<real><<<grid_blocks(12LL * c->g.gy * c->g.gz), kThreads, 0, c->stream>>>(fields<real>(c), c->g, 0);
-  CKL();
-  wrap_b_kernel<real><<<grid_blocks(12LL * c->g.gx * c->g.gz), kThreads, 0, c->stream>>>(fields<real>(c), c->g, 1);
-  CKL();
   return PIC_OK;
 }
 
 template <typename real>
 int do_renew_e(pic_ctx* c) {
   EParams p{c->cfg.c * c->cfg.c * c->cfg.dt, c->cfg.mu0, 1.0 / (24.0 * c->cfg.dx)};
+  const bool ghosts = !c->has_xport;
   if (c->staged) {
     constexpr int TX = StShape<real>::TX, TY = StShape<real>::TY;
     const int ty = (c->g.ny + TY - 1) / TY, tz = (c->g.nz + kStZ - 1) / kStZ, tx = (c->g.nx + TX - 1) / TX;
     renew_e_tma_kernel<real, TX, TY><<<tx * ty * tz, kStThreads, StTile<real>::bytes, c->stream>>>(
-        c->tm_db[0], c->tm_db[1], c->tm_db[2], fields<real>(c), c->g, ramps(c), p, ty, tz, c->err);
+        c->tm_db[0], c->tm_db[1], c->tm_db[2], fields<real>(c), c->g, ramps(c), p, ty, tz, ghosts, c->err);
   } else {
     const long long nint = (long long)c->g.nx * c->g.ny * c->g.nz;
-    renew_e_kernel<real><<<grid_blocks(nint), kThreads, 0, c->stream>>>(fields<real>(c), c->g, ramps(c), p);
+    renew_e_kernel<real><<<grid_blocks(nint), kThreads, 0, c->stream>>>(fields<real>(c), c->g, ramps(c), p, ghosts);
   }
   CKL();
   static const int ids[3] = {F_EX, F_EY, F_EZ};
-  return wrap_planes<real>(c, ids, 3);
+  return ghosts ? PIC_OK : wrap_planes<real>(c, ids, 3);
 }
 
 template <typename real>
 int do_fold(pic_ctx* c) {
-  PlaneSet<real> s{};
-  Fields<real> F = fields<real>(c);
-  for (int q = 0; q < 8; ++q) s.p[q] = F.f[F_JIX + q];
-  s.count = 8;
-  if (c->has_xport) return halo_fold<real>(c, s);
-  fold_kernel<real><<<grid_blocks(32LL * c->g.gy * c->g.gz), kThreads, 0, c->stream>>>(s, c->g, 0);
-  CKL();
-  fold_kernel<real><<<grid_blocks(32LL * c->g.gx * c->g.gz), kThreads, 0, c->stream>>>(s, c->g, 1);
+  Rider<real> r = make_rider<real>(c, RIDE_FOLD);
+  if (c->has_xport) return halo_fold<real>(c, r.fold);
+  fold_kernel<real><<<rider_blocks(c, RIDE_FOLD), kThreads, 0, c->stream>>>(r, c->g);
   CKL();
   return PIC_OK;
+}
+
+// renew_b4_2 and sr_current2, neither of which reads what the other writes.
+template <typename real>
+int do_renew_b_fold(pic_ctx* c) {
+  CKR(do_renew_b<real>(c, c->has_xport ? RIDE_NONE : RIDE_FOLD));
+  return c->has_xport ? do_fold<real>(c) : PIC_OK;
 }
 
 // renew_phi3 + sr_phi + sr_e (:8315-8665, :1389-1574): the Gauss residual,
@@ -1267,9 +1292,6 @@ template <typename real>
 int do_step(pic_ctx* c) {
   // a placement's spill count that has landed is acted on without waiting
   for (int s = 0; s < 2; ++s) CKR(check_spill<real>(c, s, false));
-  CKR(phase_mark(c, PH_FIELD));
-  CKR(do_renew_grid(c));
-  CKR(phase_mark(c, PH_FIELD));
   if (c->c_thrust > c->cfg.sort_interval - 1) {
     c->c_thrust = 0;
     // sorting (:696-697) only reorders particles, for locality. The tiled
@@ -1289,7 +1311,7 @@ int do_step(pic_ctx* c) {
     c->c_add = 0;
   }
   CKR(phase_mark(c, PH_FIELD));
-  CKR(do_renew_b<real>(c));
+  CKR(do_renew_b<real>(c, RIDE_CLEAR));  // and renew_grid
   CKR(phase_mark(c, PH_FIELD));
   // a re-layout after a refill or an import
   const bool which[2] = {!c->cfg.slot_order && !c->tiled[0], !c->cfg.slot_order && !c->tiled[1]};
@@ -1309,8 +1331,7 @@ int do_step(pic_ctx* c) {
   if (c->has_xport) CKR(do_migrate<real>(c));  // sr_particle's exchange between ranks
   CKR(phase_mark(c, PH_PUSH));
   CKR(phase_mark(c, PH_FIELD));
-  CKR(do_renew_b<real>(c));
-  CKR(do_fold<real>(c));
+  CKR(do_renew_b_fold<real>(c));
   CKR(do_renew_e<real>(c));
   if (c->cfg.poisson_clean) CKR(do_poisson<real>(c));
   CKR(phase_mark(c, PH_FIELD));
@@ -1873,7 +1894,7 @@ int pic_renew_grid(pic_ctx* c) {
 
 int pic_renew_b4_2(pic_ctx* c) {
   CKR(check_ctx(c));
-  return DISPATCH(c, do_renew_b)(c);
+  return DISPATCH(c, do_renew_b)(c, RIDE_NONE);
 }
 
 int pic_renew_e4_2(pic_ctx* c) {

@@ -71,6 +71,17 @@ __device__ __forceinline__ void st2(real* p, long long i, real a, real b) {
   *reinterpret_cast<typename Two<real>::T*>(p + i) = v;
 }
 
+// put_images_b of two z-adjacent nodes.
+template <typename real>
+__device__ __forceinline__ void put_images_b2(const Fields<real>& F, int c, long long n, const Images& im, real v0,
+                                              real v1) {
+  for (int q = 0; q < im.n; ++q) {
+    const auto b0 = ld2(F.f[F_B0X + c], n + im.d[q]);
+    st2(F.f[F_BX + c], n + im.d[q], v0, v1);
+    st2(F.f[F_DBX + c], n + im.d[q], v0 - b0.x, v1 - b0.y);
+  }
+}
+
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count) {
@@ -148,8 +159,10 @@ template <typename real, int TX, int TY>
 __global__ void __launch_bounds__(kStThreads, sizeof(real) == 4 ? 3 : 2)
     renew_b_tma_kernel(const __grid_constant__ CUtensorMap tex, const __grid_constant__ CUtensorMap tey,
                        const __grid_constant__ CUtensorMap tez, Fields<real> F, Geom g, Ramps rp, BParams p,
-                       int tiles_y, int tiles_z, unsigned long long* err) {
+                       int tiles_y, int tiles_z, bool ghosts, const __grid_constant__ Rider<real> rider,
+                       unsigned long long* err) {
   using T = StencilTile<real, TX, TY>;
+  if (rider.mode && (int)blockIdx.x >= rider.first) return ride(rider, g);
   extern __shared__ __align__(128) unsigned char fsm[];
   int k0, l0, m0;
   tile_origin<TX, TY>(tiles_y, tiles_z, k0, l0, m0);
@@ -181,6 +194,8 @@ __global__ void __launch_bounds__(kStThreads, sizeof(real) == 4 ? 3 : 2)
       waited = true;
     }
     if (!in) continue;
+    Images im{0, {0, 0, 0}};
+    if (ghosts) im = images_of(g, k, l);
     const int s0 = (a * T::EY0 + b + 2) * kStBoxZ + z + 2;        // ex
     const int s1 = ((a + 2) * T::EY1 + b) * kStBoxZ + z + 2;      // ey
     const int s2 = ((a + 2) * T::EY2 + b + 2) * kStBoxZ + z + 2;  // ez
@@ -211,7 +226,9 @@ __global__ void __launch_bounds__(kStThreads, sizeof(real) == 4 ? 3 : 2)
         db[j] = (real)ca * dbo[j] - (real)cb * curl;
       }
       st2(F.f[F_DBX], n, db[0], db[1]);
-      st2(F.f[F_BX], n, b0[0] + db[0], b0[1] + db[1]);
+      const real b[2] = {b0[0] + db[0], b0[1] + db[1]};
+      st2(F.f[F_BX], n, b[0], b[1]);
+      put_images_b2(F, 0, n, im, b[0], b[1]);
     }
     // y component at (k, l+1/2, m): ex along z, ez along x
     {
@@ -228,7 +245,9 @@ __global__ void __launch_bounds__(kStThreads, sizeof(real) == 4 ? 3 : 2)
         db[j] = (real)ca * dbo[j] - (real)cb * curl;
       }
       st2(F.f[F_DBY], n, db[0], db[1]);
-      st2(F.f[F_BY], n, b0[0] + db[0], b0[1] + db[1]);
+      const real b[2] = {b0[0] + db[0], b0[1] + db[1]};
+      st2(F.f[F_BY], n, b[0], b[1]);
+      put_images_b2(F, 1, n, im, b[0], b[1]);
     }
     // z component at (k, l, m+1/2): ey along x, ex along y
     {
@@ -247,7 +266,13 @@ __global__ void __launch_bounds__(kStThreads, sizeof(real) == 4 ? 3 : 2)
         db[j] = (real)ca * dbo[j] - (real)cb * curl;
       }
       st2(F.f[F_DBZ], n, db[0], db[1]);
-      st2(F.f[F_BZ], n, b0[0] + db[0], b0[1] + db[1]);
+      const real b[2] = {b0[0] + db[0], b0[1] + db[1]};
+      st2(F.f[F_BZ], n, b[0], b[1]);
+      put_images_b2(F, 2, n, im, b[0], b[1]);
+    }
+    if (im.n) {
+      if (m == 2) z_end_images(F, g, F_BX, true, n - m, im, true);
+      if (m == g.nz) z_end_images(F, g, F_BX, true, n - m, im, false);
     }
   }
 }
@@ -256,7 +281,7 @@ template <typename real, int TX, int TY>
 __global__ void __launch_bounds__(kStThreads, sizeof(real) == 4 ? 3 : 2)
     renew_e_tma_kernel(const __grid_constant__ CUtensorMap tbx, const __grid_constant__ CUtensorMap tby,
                        const __grid_constant__ CUtensorMap tbz, Fields<real> F, Geom g, Ramps rp, EParams p,
-                       int tiles_y, int tiles_z, unsigned long long* err) {
+                       int tiles_y, int tiles_z, bool ghosts, unsigned long long* err) {
   using T = StencilTile<real, TX, TY>;
   extern __shared__ __align__(128) unsigned char fsm[];
   int k0, l0, m0;
@@ -291,6 +316,8 @@ __global__ void __launch_bounds__(kStThreads, sizeof(real) == 4 ? 3 : 2)
       waited = true;
     }
     if (!in) continue;
+    Images im{0, {0, 0, 0}};
+    if (ghosts) im = images_of(g, k, l);
     const int s0 = (a * T::EY0 + b + 1) * kStBoxZ + z + 2;        // bx
     const int s1 = ((a + 1) * T::EY1 + b) * kStBoxZ + z + 2;      // by
     const int s2 = ((a + 1) * T::EY2 + b + 1) * kStBoxZ + z + 2;  // bz
@@ -321,6 +348,7 @@ __global__ void __launch_bounds__(kStThreads, sizeof(real) == 4 ? 3 : 2)
         en[j] = (real)ca * eo[j] + (real)cb * (curl - mu0 * (ji[j] - je[j]));
       }
       st2(F.f[F_EX], n, en[0], en[1]);
+      for (int q = 0; q < im.n; ++q) st2(F.f[F_EX], n + im.d[q], en[0], en[1]);
     }
     // y component at (k+1/2, l, m+1/2): bx along z, bz along x
     {
@@ -337,6 +365,7 @@ __global__ void __launch_bounds__(kStThreads, sizeof(real) == 4 ? 3 : 2)
         en[j] = (real)ca * eo[j] + (real)cb * (curl - mu0 * (ji[j] - je[j]));
       }
       st2(F.f[F_EY], n, en[0], en[1]);
+      for (int q = 0; q < im.n; ++q) st2(F.f[F_EY], n + im.d[q], en[0], en[1]);
     }
     // z component at (k+1/2, l+1/2, m): by along x, bx along y
     {
@@ -355,6 +384,11 @@ __global__ void __launch_bounds__(kStThreads, sizeof(real) == 4 ? 3 : 2)
         en[j] = (real)ca * eo[j] + (real)cb * (curl - mu0 * (ji[j] - je[j]));
       }
       st2(F.f[F_EZ], n, en[0], en[1]);
+      for (int q = 0; q < im.n; ++q) st2(F.f[F_EZ], n + im.d[q], en[0], en[1]);
+    }
+    if (im.n) {
+      if (m == 2) z_end_images(F, g, F_EX, false, n - m, im, true);
+      if (m == g.nz) z_end_images(F, g, F_EX, false, n - m, im, false);
     }
   }
 }
