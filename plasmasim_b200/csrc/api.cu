@@ -249,6 +249,8 @@ PushConst<real> push_const(const pic_ctx* c, int s) {
   // when it lies below bal_l* or at or above bal_h* (fdtd :733-735)
   pc.bal_interior = pc.bal_lx > 2 || pc.bal_ly > 2 || pc.bal_lz > 2 || pc.bal_hx < k.nx + 2 ||
                     pc.bal_hy < k.ny + 2 || pc.bal_hz < k.nz + 2;
+  // |v| < c after a push, whatever the fields; c dt / dx is below 1/2 in any stable run
+  pc.long_moves = !(0.5 * k.c * k.dt / k.dx < 0.99);
   pc.out = Outbox<real>{nullptr, 0, nullptr};
   if (c->has_xport && c->mig) {  // list s of the packet lists is species s's outbox
     pc.out.count = c->mig_cnt + s;
@@ -736,22 +738,32 @@ int do_push(pic_ctx* c, int s, long long first = 0) {
 
 __global__ void copy_int_kernel(int* dst, const int* src) { *dst = *src; }
 
-// The push of species s: the slots after the layout (particles a placement
-// could not place) with the slot-order kernel, then the tiled kernel.
+// The push of species s. `overlap`: the launch just before on the stream is the
+// other species' tiled push, which this one may run beside (push_tiled.cuh).
 template <typename real>
-int do_push_tiled(pic_ctx* c, int s) {
+int do_push_tiled(pic_ctx* c, int s, bool overlap = false) {
   if (!c->layout[s]) return do_push<real, PUSH_FUSED>(c, s);
-  CKR((do_push<real, PUSH_FUSED>(c, s, c->tiled_end[s])));
   const int ntiles = c->tg.ntx * c->tg.nty * c->tg.ntz;
-  TileArgs ta{c->tg, c->goff[s][c->lay[s]], c->gtop[s]};
-  const bool vec = sizeof(real) == 4 && c->g.gz % 4 == 0;
+  // a CTA per SM for the tail, whose length only the device may know
+  const long long tail = slot_bound(c, s) - c->tiled_end[s];
+  const int ntail = (int)std::min<long long>((std::max<long long>(tail, 0) + kThreads - 1) / kThreads, 148);
+  const TileArgs ta{c->tg, c->goff[s][c->lay[s]], c->gtop[s], ntail, (int)c->tiled_end[s], c->sp[s].count_dev};
+  const bool vec = c->g.gz * sizeof(real) % 16 == 0;
+  cudaLaunchConfig_t k{};
+  k.gridDim = dim3(ntail + ntiles);
+  k.blockDim = dim3(kTileX * kTileY * 32);
+  k.dynamicSmemBytes = PushSmem<real>::bytes;
+  k.stream = c->stream;
+  cudaLaunchAttribute early{};
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  k.attrs = &early;
+  k.numAttrs = overlap ? 1 : 0;
   const Parts<real> P = parts<real>(c, s);
   const Fields<real> F = fields<real>(c);
   const PushConst<real> pc = push_const<real>(c, s);
-  const dim3 grid(ntiles), block(kTileX * kTileY * 32);
-  const size_t smem = PushSmem<real>::bytes;
-  if (vec) push_tiled_kernel<real, true><<<grid, block, smem, c->stream>>>(P, ta, F, c->g, pc, c->err);
-  else push_tiled_kernel<real, false><<<grid, block, smem, c->stream>>>(P, ta, F, c->g, pc, c->err);
+  CK(vec ? cudaLaunchKernelEx(&k, push_tiled_kernel<real, true>, P, ta, F, c->g, pc, c->err)
+         : cudaLaunchKernelEx(&k, push_tiled_kernel<real, false>, P, ta, F, c->g, pc, c->err));
   CKL();
   return PIC_OK;
 }
@@ -1327,7 +1339,7 @@ int do_step(pic_ctx* c) {
   // the counts stay on the device: the push and the diagnostics cover the
   // slots up to the capacity and stop at the device count, and the host reads
   // a count back only when an entry point needs it
-  for (int s = 0; s < 2; ++s) CKR(do_push_tiled<real>(c, s));
+  for (int s = 0; s < 2; ++s) CKR(do_push_tiled<real>(c, s, s == 1 && c->layout[0]));
   if (c->has_xport) CKR(do_migrate<real>(c));  // sr_particle's exchange between ranks
   CKR(phase_mark(c, PH_PUSH));
   CKR(phase_mark(c, PH_FIELD));
@@ -1797,6 +1809,8 @@ int pic_create(const pic_config* cfg, pic_ctx** out) {
     }
     const int pb_f = (int)PushSmem<float>::bytes, pb_d = (int)PushSmem<double>::bytes;
     if (cudaFuncSetAttribute(push_tiled_kernel<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, pb_d) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(push_tiled_kernel<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, pb_d) !=
             cudaSuccess ||
         cudaFuncSetAttribute(push_tiled_kernel<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, pb_f) !=
             cudaSuccess ||

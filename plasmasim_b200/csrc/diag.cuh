@@ -99,18 +99,18 @@ struct ThrustWin {
 using ThrustPlan = PushSmem<float>;
 
 __device__ __forceinline__ Gathered<double> thrust_gather(const ThrustWin&, const Fields<double>& F, const Geom& g,
-                                                          const Axis<double>& X, const Axis<double>& Y,
-                                                          const Axis<double>& Z, int, int, int) {
-  return gather6(F, g, X, Y, Z);
+                                                          const Rec<double>& q, int i, int j, int k) {
+  return gather6(F, g, axis_weights(i, q.o[0]), axis_weights(j, q.o[1]), axis_weights(k, q.o[2]));
 }
 __device__ __forceinline__ Gathered<float> thrust_gather(const ThrustWin& w, const Fields<float>& F, const Geom& g,
-                                                         const Axis<float>& X, const Axis<float>& Y,
-                                                         const Axis<float>& Z, int i, int j, int k) {
+                                                         const Rec<float>& q, int i, int j, int k) {
   using S = ThrustPlan;
-  if (w.fw && i - 1 >= w.x0 && i + 1 < w.x0 + S::WX && j - 1 >= w.y0 && j + 1 < w.y0 + S::WY && k - 1 >= w.z0 &&
-      k + 1 < w.z0 + S::WZ)
-    return gather6_win<S::WY, S::WZ, S::WN>(w.fw, w.x0, w.y0, w.z0, X, Y, Z);
-  return gather6(F, g, X, Y, Z);
+  if (w.fw && i > 0 && j > 0 && k > 0 && i - 1 >= w.x0 && i + 1 < w.x0 + S::WX && j - 1 >= w.y0 &&
+      j + 1 < w.y0 + S::WY && k - 1 >= w.z0 && k + 1 < w.z0 + S::WZ)
+    return gather6_win<S::WY, S::WZ, S::WN>(w.fw + (((i - w.x0) * S::WY + j - w.y0) * S::WZ + k - w.z0),
+                                            win_axis(q.o[0], S::WY * S::WZ), win_axis(q.o[1], S::WZ),
+                                            win_axis(q.o[2], 1));
+  return gather6(F, g, axis_weights(i, q.o[0]), axis_weights(j, q.o[1]), axis_weights(k, q.o[2]));
 }
 
 template <typename real>
@@ -125,7 +125,7 @@ __device__ __forceinline__ void thrust_terms(const ThrustArgs<real>& a, const Th
                                              const Rec<real>& q, double (&s)[7]) {
   if (!stencil_ok(a.g, i, j, k)) return;
   const Gathered<real> e =
-      thrust_gather(win, a.F, a.g, axis_weights(i, q.o[0]), axis_weights(j, q.o[1]), axis_weights(k, q.o[2]), i, j, k);
+      thrust_gather(win, a.F, a.g, q, i, j, k);
   const double vx = q.v[0], vy = q.v[1], vz = q.v[2];
   const double bx = e.bx, by = e.by, bz = e.bz;
   s[0] += (double)e.ex;
@@ -203,8 +203,8 @@ __global__ void __launch_bounds__(256, 3) thrust_kernel(const __grid_constant__ 
     };
     fetch(0);
     if constexpr (kWin) {
-      if (a.vec) fill_win<S::WX, S::WY, S::WZ, true>(thrust_win, a.F, g, win.x0, win.y0, win.z0);
-      else fill_win<S::WX, S::WY, S::WZ, false>(thrust_win, a.F, g, win.x0, win.y0, win.z0);
+      if (a.vec) fill_win<float, S::WX, S::WY, S::WZ, true>(thrust_win, a.F, g, win.x0, win.y0, win.z0);
+      else fill_win<float, S::WX, S::WY, S::WZ, false>(thrust_win, a.F, g, win.x0, win.y0, win.z0);
       win.fw = thrust_win;
       __syncthreads();
     }

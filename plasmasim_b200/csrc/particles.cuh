@@ -108,20 +108,27 @@ __device__ __forceinline__ Rec<double> load_records(const Parts<double>& P, long
   return Rec<double>{__double2loint(a0.x), {a0.y, a1.x, a1.y}, {b0.x, b0.y, b1.x}};
 }
 
-// Particle t's records, written with vector stores.
+// An int32 in a real's first 4 bytes, as record A holds the cell.
+__device__ __forceinline__ int word_int(float x) { return __float_as_int(x); }
+__device__ __forceinline__ int word_int(double x) { return __double2loint(x); }
+template <typename real> __device__ __forceinline__ real int_word(int c);
+template <> __device__ __forceinline__ float int_word<float>(int c) { return __int_as_float(c); }
+template <> __device__ __forceinline__ double int_word<double>(int c) { return __hiloint2double(0, c); }
+
+// Particle t's records, written with vector stores (w: record B's fourth word).
 __device__ __forceinline__ void store_records(const Parts<float>& P, long long t, int c, float fx, float fy,
-                                              float fz, float vx, float vy, float vz) {
+                                              float fz, float vx, float vy, float vz, float w = 0.f) {
   reinterpret_cast<float4*>(P.ra)[t] = make_float4(__int_as_float(c), fx, fy, fz);
-  reinterpret_cast<float4*>(P.rb)[t] = make_float4(vx, vy, vz, 0.f);
+  reinterpret_cast<float4*>(P.rb)[t] = make_float4(vx, vy, vz, w);
 }
 __device__ __forceinline__ void store_records(const Parts<double>& P, long long t, int c, double fx, double fy,
-                                              double fz, double vx, double vy, double vz) {
+                                              double fz, double vx, double vy, double vz, double w = 0.0) {
   double2* a = reinterpret_cast<double2*>(P.ra + 4 * t);
   double2* b = reinterpret_cast<double2*>(P.rb + 4 * t);
   a[0] = make_double2(__hiloint2double(0, c), fx);
   a[1] = make_double2(fy, fz);
   b[0] = make_double2(vx, vy);
-  b[1] = make_double2(vz, 0.0);
+  b[1] = make_double2(vz, w);
 }
 // Particle s of S to slot d of D with cell index c: two vector copies.
 __device__ __forceinline__ void copy_record(const Parts<float>& S, long long s, const Parts<float>& D, long long d,
@@ -178,6 +185,7 @@ struct PushConst {
   int bal_lx, bal_ly, bal_lz;
   int bal_hx, bal_hy, bal_hz;
   int bal_interior;            // the ballistic region reaches an interior cell of this rank
+  int long_moves;              // a half step may take a particle a whole cell
   int pjx, pjy, pjz, pn;       // deposit planes of this species
   Outbox<real> out;            // decomposed runs: particles leaving the rank's x-y interior
 };
@@ -314,63 +322,78 @@ enum PushMode { PUSH_J = 0, PUSH_FUSED = 1 };
 //              drift, the density deposit nor the removal reads a field, so the
 //              second B half-step that the reference runs between them changes
 //              nothing they compute.
+// Particle t of P through the push (MODE as below), its records read and
+// written; any cell of the padded array.
 template <typename real, int MODE>
-__global__ void __launch_bounds__(256) push_kernel(Parts<real> P, int first, const int* __restrict__ count,
-                                                   Fields<real> F, Geom g, PushConst<real> pc,
-                                                   unsigned long long* err) {
-  const int n = *count;
-  unsigned pushed = 0;
-  for (int t = first + blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-    const Rec<real> r = load_records(P, t);
-    if (r.cell < 0) continue;
-    ++pushed;
-    int i, j, k;
-    unpack_cell(r.cell, i, j, k);
-    real fx = r.o[0], fy = r.o[1], fz = r.o[2];
-    real vx = r.v[0], vy = r.v[1], vz = r.v[2];
-    bool bal = ballistic(pc, i, j, k, fx, fy, fz);
-    if (!bal && !stencil_ok(g, i, j, k)) {
-      count_err(err, ERR_DEPOSIT_OOB);
-      bal = true;
-    }
-    if (!bal) {
+__device__ __forceinline__ void push_one(const Parts<real>& P, int t, const Rec<real>& r, const Fields<real>& F,
+                                         const Geom& g, const PushConst<real>& pc, unsigned long long* err) {
+  int i, j, k;
+  unpack_cell(r.cell, i, j, k);
+  real fx = r.o[0], fy = r.o[1], fz = r.o[2];
+  real vx = r.v[0], vy = r.v[1], vz = r.v[2];
+  bool bal = ballistic(pc, i, j, k, fx, fy, fz);
+  if (!bal && !stencil_ok(g, i, j, k)) {
+    count_err(err, ERR_DEPOSIT_OOB);
+    bal = true;
+  }
+  if (!bal) {
+    const Axis<real> X = axis_weights(i, fx), Y = axis_weights(j, fy), Z = axis_weights(k, fz);
+    boris4(pc, gather6(F, g, X, Y, Z), vx, vy, vz);
+    if (!(isfinite(vx) && isfinite(vy) && isfinite(vz))) count_err(err, ERR_NONFINITE);
+  }
+  advance(i, fx, vx * pc.hdt);
+  advance(j, fy, vy * pc.hdt);
+  advance(k, fz, vz * pc.hdt);
+  if (in_array(g, i, j, k)) {
+    if (stencil_ok(g, i, j, k)) {
       const Axis<real> X = axis_weights(i, fx), Y = axis_weights(j, fy), Z = axis_weights(k, fz);
-      boris4(pc, gather6(F, g, X, Y, Z), vx, vy, vz);
-      if (!(isfinite(vx) && isfinite(vy) && isfinite(vz))) count_err(err, ERR_NONFINITE);
+      deposit_j(F, g, pc, X, Y, Z, vx, vy, vz);
+    } else {
+      count_err(err, ERR_DEPOSIT_OOB);
     }
+  }
+  int cell;
+  if (MODE == PUSH_FUSED) {
     advance(i, fx, vx * pc.hdt);
     advance(j, fy, vy * pc.hdt);
     advance(k, fz, vz * pc.hdt);
     if (in_array(g, i, j, k)) {
       if (stencil_ok(g, i, j, k)) {
         const Axis<real> X = axis_weights(i, fx), Y = axis_weights(j, fy), Z = axis_weights(k, fz);
-        deposit_j(F, g, pc, X, Y, Z, vx, vy, vz);
+        deposit_n(F, g, pc, X, Y, Z);
       } else {
         count_err(err, ERR_DEPOSIT_OOB);
       }
     }
-    int cell;
-    if (MODE == PUSH_FUSED) {
-      advance(i, fx, vx * pc.hdt);
-      advance(j, fy, vy * pc.hdt);
-      advance(k, fz, vz * pc.hdt);
-      if (in_array(g, i, j, k)) {
-        if (stencil_ok(g, i, j, k)) {
-          const Axis<real> X = axis_weights(i, fx), Y = axis_weights(j, fy), Z = axis_weights(k, fz);
-          deposit_n(F, g, pc, X, Y, Z);
-        } else {
-          count_err(err, ERR_DEPOSIT_OOB);
-        }
-      }
-      cell = settle(g, pc.out, i, j, k, fx, fy, fz, vx, vy, vz, err);
-    } else {
-      cell = repack(i, j, k, err);
-    }
-    store_records(P, t, cell, fx, fy, fz, vx, vy, vz);
+    cell = settle(g, pc.out, i, j, k, fx, fy, fz, vx, vy, vz, err);
+  } else {
+    cell = repack(i, j, k, err);
+  }
+  store_records(P, t, cell, fx, fy, fz, vx, vy, vz);
+}
+
+// Slots first, first + stride, ... below n.
+template <typename real, int MODE>
+__device__ __forceinline__ void push_slots(const Parts<real>& P, int first, int stride, int n, const Fields<real>& F,
+                                           const Geom& g, const PushConst<real>& pc, unsigned long long* err) {
+  unsigned pushed = 0;
+  for (int t = first; t < n; t += stride) {
+    const Rec<real> r = load_records(P, t);
+    if (r.cell < 0) continue;
+    ++pushed;
+    push_one<real, MODE>(P, t, r, F, g, pc, err);
   }
   // particle pushes of this warp, one atomic per warp
   for (int o = 16; o > 0; o >>= 1) pushed += __shfl_down_sync(0xffffffffu, pushed, o);
   if ((threadIdx.x & 31) == 0 && pushed) atomicAdd(err + CNT_PUSHED, (unsigned long long)pushed);
+}
+
+template <typename real, int MODE>
+__global__ void __launch_bounds__(256) push_kernel(Parts<real> P, int first, const int* __restrict__ count,
+                                                   Fields<real> F, Geom g, PushConst<real> pc,
+                                                   unsigned long long* err) {
+  push_slots<real, MODE>(P, first + blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, *count, F, g, pc,
+                         err);
 }
 
 // Drift to x^{n+1} and density deposit (fdtd :818-867).

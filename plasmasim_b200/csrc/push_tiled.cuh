@@ -7,100 +7,148 @@
 
 namespace pb {
 
-constexpr int kStages = 3;   // particle rows in flight per warp
+// Particle rows in flight per warp (with 3 to 6 rows the FP32 push of 128^3 x 64
+// took 7.04, 7.02, 7.09 and 7.08 ms per step, FP64 64^3 x 32 1.690, 1.692, 1.710, 1.728).
+template <typename real>
+constexpr int kStages = sizeof(real) == 4 ? 4 : 3;
 
-
-// A box of cells: first cell (ci0, cj0, ck0) and extents; the push uses the
-// domain's interior cells [2, n + 2) of each axis.
-struct InteriorBox {
-  int ci0, cj0, ck0;
+// Cells [lo, lo + ext) of each axis.
+struct CellRange {
+  int lx, ly, lz;
   unsigned ex, ey, ez;
   __device__ __forceinline__ bool has(int i, int j, int k) const {
-    return (unsigned)(i - ci0) < ex && (unsigned)(j - cj0) < ey && (unsigned)(k - ck0) < ez;
+    return (unsigned)(i - lx) < ex && (unsigned)(j - ly) < ey && (unsigned)(k - lz) < ez;
   }
 };
 
-// Shared-memory plan of one CTA (8 warps): the J/n window, per warp a ring of
-// kStages particle rows fetched ahead with cp.async (records A and B of each
-// slot) and, in FP32, the tile's E and B over the same window (the gather
-// reads them there; FP64 gathers from global memory, its window would not
-// leave room for two CTAs per SM).
+// Shared-memory plan of one CTA (8 warps): the density window; per warp a ring
+// of kStages particle rows fetched ahead with cp.async (records A and B of each
+// slot: 8 reals), whose memory takes the J window after the last row; the
+// tile's E and B over the window, where the gather reads them; per warp a queue
+// of kQ off-home J deposits, 7 words each (cell, offsets, velocities), made 32
+// at a time by the whole warp (1.7 % off the FP32 step against each particle
+// depositing where it is found), and the slots left to the general path.
 template <typename real>
 struct PushSmem {
   static constexpr int WX = kTileX + 4, WY = kTileY + 4, WZ = kWinZ, WN = WX * WY * WZ;
   static constexpr int kWarps = kTileX * kTileY;
-  static constexpr bool kFieldWin = sizeof(real) == 4;
-  static constexpr size_t win_bytes = 4 * WN * sizeof(real);
-  static constexpr size_t prec_off = (win_bytes + 15) & ~(size_t)15;  // records A, B of each slot: 8 reals
-  static constexpr size_t fwin_off = prec_off + (size_t)kWarps * kStages * kLanes * 8 * sizeof(real);
-  // FP32: per warp a queue of kQ off-home J deposits, 7 words each (cell,
-  // offsets, velocities), made 32 at a time by the whole warp (1.7 % off the
-  // step against each particle depositing where it is found); FP64 has no
-  // room for it beside two CTAs per SM
-  static constexpr bool kJQueue = sizeof(real) == 4;
   static constexpr int kQ = 2 * kLanes;
-  static constexpr size_t jq_off = fwin_off + (kFieldWin ? (size_t)6 * WN * sizeof(float) : 0);
-  static constexpr size_t bytes = jq_off + (kJQueue ? (size_t)kWarps * kQ * 7 * sizeof(float) : 0);
+  static constexpr int kRest = 8 * kLanes;
+  static constexpr size_t ring_off = (WN * sizeof(real) + 15) & ~(size_t)15;
+  static constexpr size_t ring_bytes = (size_t)kWarps * kStages<real> * kLanes * 8 * sizeof(real);
+  static_assert(ring_bytes >= 3 * WN * sizeof(real), "the ring holds the J window");
+  static constexpr size_t fwin_off = ring_off + ring_bytes;
+  static constexpr size_t jq_off = fwin_off + (size_t)6 * WN * sizeof(real);
+  static constexpr size_t slow_off = jq_off + (size_t)kWarps * kQ * 7 * sizeof(real);
+  static constexpr size_t bytes = slow_off + (size_t)kWarps * kRest * sizeof(int);
 };
 
 // Trilinear interpolation from a window plane with compile-time strides (the
-// 2x2x2 nodes at window index n), the two x planes as one packed pair.
+// 2x2x2 nodes from w on), the two x planes as one packed pair.
 template <int WY, int WZ>
-__device__ __forceinline__ float trilerp_win(const float* __restrict__ w, int n, float x0, float x1, float2 Y0,
-                                             float2 Y1, float2 Z0, float2 Z1) {
+__device__ __forceinline__ float trilerp_win(const float* __restrict__ w, float x0, float x1, float2 Y0, float2 Y1,
+                                             float2 Z0, float2 Z1) {
   constexpr int P = WY * WZ;  // next x plane
-  const float2 n00 = make_float2(w[n], w[n + P]), n01 = make_float2(w[n + 1], w[n + P + 1]);
-  const float2 n10 = make_float2(w[n + WZ], w[n + P + WZ]), n11 = make_float2(w[n + WZ + 1], w[n + P + WZ + 1]);
+  const float2 n00 = make_float2(w[0], w[P]), n01 = make_float2(w[1], w[P + 1]);
+  const float2 n10 = make_float2(w[WZ], w[P + WZ]), n11 = make_float2(w[WZ + 1], w[P + WZ + 1]);
   const float2 cy0 = __ffma2_rn(n01, Z1, __fmul2_rn(n00, Z0));
   const float2 cy1 = __ffma2_rn(n11, Z1, __fmul2_rn(n10, Z0));
   const float2 cx = __ffma2_rn(cy1, Y1, __fmul2_rn(cy0, Y0));
   return cx.x * x0 + cx.y * x1;
 }
 
+template <int WY, int WZ>
+__device__ __forceinline__ double trilerp_win(const double* __restrict__ w, double x0, double x1, double y0, double y1,
+                                              double z0, double z1) {
+  constexpr int P = WY * WZ;
+  const double c00 = w[0] * z0 + w[1] * z1, c01 = w[WZ] * z0 + w[WZ + 1] * z1;
+  const double c10 = w[P] * z0 + w[P + 1] * z1, c11 = w[P + WZ] * z0 + w[P + WZ + 1] * z1;
+  return (c00 * y0 + c01 * y1) * x0 + (c10 * y0 + c11 * y1) * x1;
+}
+
+// Weights along one axis of a particle at offset f of an interior cell (so
+// never cell 0, where axis_weights' half-shifted base is the cell itself), and
+// the step from the cell's node to the half-shifted base (0 or -stride).
+template <typename real>
+struct WinAxis {
+  real a0, a1, b0, b1;
+  int s;
+};
+template <typename real>
+__device__ __forceinline__ WinAxis<real> win_axis(real f, int stride) {
+  WinAxis<real> w;
+  const bool up = f >= (real)0.5;
+  w.a1 = f;
+  w.a0 = (real)1 - f;
+  w.b1 = f + (up ? (real)-0.5 : (real)0.5);
+  w.b0 = (real)1 - w.b1;
+  w.s = up ? 0 : -stride;
+  return w;
+}
+
 // gather6 from a window of one plane per component (ex ey ez bx by bz, WN
-// nodes each, origin (wx0, wy0, wz0)); the caller checks that the stencil lies inside.
+// nodes each) at node n, the particle's cell; its stencil lies inside.
 template <int WY, int WZ, int WN>
-__device__ __forceinline__ Gathered<float> gather6_win(const float* __restrict__ fw, int wx0, int wy0, int wz0,
-                                                       const Axis<float>& X, const Axis<float>& Y,
-                                                       const Axis<float>& Z) {
-  const int ax = X.a - wx0, bx = X.b - wx0, ay = Y.a - wy0, by = Y.b - wy0, az = Z.a - wz0, bz = Z.b - wz0;
+__device__ __forceinline__ Gathered<float> gather6_win(const float* __restrict__ n, const WinAxis<float>& X,
+                                                       const WinAxis<float>& Y, const WinAxis<float>& Z) {
   const float2 ya0 = make_float2(Y.a0, Y.a0), ya1 = make_float2(Y.a1, Y.a1);
   const float2 yb0 = make_float2(Y.b0, Y.b0), yb1 = make_float2(Y.b1, Y.b1);
   const float2 za0 = make_float2(Z.a0, Z.a0), za1 = make_float2(Z.a1, Z.a1);
   const float2 zb0 = make_float2(Z.b0, Z.b0), zb1 = make_float2(Z.b1, Z.b1);
   Gathered<float> r;
-  r.ex = trilerp_win<WY, WZ>(fw, (ax * WY + by) * WZ + bz, X.a0, X.a1, yb0, yb1, zb0, zb1);
-  r.ey = trilerp_win<WY, WZ>(fw + WN, (bx * WY + ay) * WZ + bz, X.b0, X.b1, ya0, ya1, zb0, zb1);
-  r.ez = trilerp_win<WY, WZ>(fw + 2 * WN, (bx * WY + by) * WZ + az, X.b0, X.b1, yb0, yb1, za0, za1);
-  r.bx = trilerp_win<WY, WZ>(fw + 3 * WN, (bx * WY + ay) * WZ + az, X.b0, X.b1, ya0, ya1, za0, za1);
-  r.by = trilerp_win<WY, WZ>(fw + 4 * WN, (ax * WY + by) * WZ + az, X.a0, X.a1, yb0, yb1, za0, za1);
-  r.bz = trilerp_win<WY, WZ>(fw + 5 * WN, (ax * WY + ay) * WZ + bz, X.a0, X.a1, ya0, ya1, zb0, zb1);
+  r.ex = trilerp_win<WY, WZ>(n + Y.s + Z.s, X.a0, X.a1, yb0, yb1, zb0, zb1);
+  r.ey = trilerp_win<WY, WZ>(n + WN + X.s + Z.s, X.b0, X.b1, ya0, ya1, zb0, zb1);
+  r.ez = trilerp_win<WY, WZ>(n + 2 * WN + X.s + Y.s, X.b0, X.b1, yb0, yb1, za0, za1);
+  r.bx = trilerp_win<WY, WZ>(n + 3 * WN + X.s, X.b0, X.b1, ya0, ya1, za0, za1);
+  r.by = trilerp_win<WY, WZ>(n + 4 * WN + Y.s, X.a0, X.a1, yb0, yb1, za0, za1);
+  r.bz = trilerp_win<WY, WZ>(n + 5 * WN + Z.s, X.a0, X.a1, ya0, ya1, zb0, zb1);
+  return r;
+}
+template <int WY, int WZ, int WN>
+__device__ __forceinline__ Gathered<double> gather6_win(const double* __restrict__ n, const WinAxis<double>& X,
+                                                        const WinAxis<double>& Y, const WinAxis<double>& Z) {
+  Gathered<double> r;
+  r.ex = trilerp_win<WY, WZ>(n + Y.s + Z.s, X.a0, X.a1, Y.b0, Y.b1, Z.b0, Z.b1);
+  r.ey = trilerp_win<WY, WZ>(n + WN + X.s + Z.s, X.b0, X.b1, Y.a0, Y.a1, Z.b0, Z.b1);
+  r.ez = trilerp_win<WY, WZ>(n + 2 * WN + X.s + Y.s, X.b0, X.b1, Y.b0, Y.b1, Z.a0, Z.a1);
+  r.bx = trilerp_win<WY, WZ>(n + 3 * WN + X.s, X.b0, X.b1, Y.a0, Y.a1, Z.a0, Z.a1);
+  r.by = trilerp_win<WY, WZ>(n + 4 * WN + Y.s, X.a0, X.a1, Y.b0, Y.b1, Z.a0, Z.a1);
+  r.bz = trilerp_win<WY, WZ>(n + 5 * WN + Z.s, X.a0, X.a1, Y.a0, Y.a1, Z.b0, Z.b1);
   return r;
 }
 
 // The window's planes from F_EX .. F_BZ (16-byte loads where the row pitch
 // allows), zero outside the array.
-template <int WX, int WY, int WZ, bool VEC>
-__device__ __forceinline__ void fill_win(float* __restrict__ fw, const Fields<float>& F, const Geom& g, int wx0,
-                                         int wy0, int wz0) {
-  constexpr int NZ4 = WZ / 4, WN = WX * WY * WZ;
-  for (int q4 = threadIdx.x; q4 < 6 * WX * WY * NZ4; q4 += blockDim.x) {
-    const int p = q4 / (WX * WY * NZ4), r = q4 % (WX * WY * NZ4);
-    const int a = r / (WY * NZ4), b = (r / NZ4) % WY, c4 = r % NZ4;
-    const int ga = wx0 + a, gb = wy0 + b, gc = wz0 + 4 * c4;
-    float v[4] = {0.f, 0.f, 0.f, 0.f};
+template <typename real, int WX, int WY, int WZ, bool VEC>
+__device__ __forceinline__ void fill_win(real* __restrict__ fw, const Fields<real>& F, const Geom& g, int wx0, int wy0,
+                                         int wz0) {
+  constexpr int V = sizeof(real) == 4 ? 4 : 2, NZV = WZ / V, WN = WX * WY * WZ;
+  for (int q = threadIdx.x; q < 6 * WX * WY * NZV; q += blockDim.x) {
+    const int p = q / (WX * WY * NZV), r = q % (WX * WY * NZV);
+    const int a = r / (WY * NZV), b = (r / NZV) % WY, c = r % NZV;
+    const int ga = wx0 + a, gb = wy0 + b, gc = wz0 + V * c;
+    real v[V];
+#pragma unroll
+    for (int e = 0; e < V; ++e) v[e] = (real)0;
     if (ga < g.gx && gb < g.gy) {
-      const float* src = F.f[p] + (long long)ga * g.sx + gb * g.gz + gc;
-      if (VEC && gc + 3 < g.gz) {
-        const float4 f4 = __ldg(reinterpret_cast<const float4*>(src));
-        v[0] = f4.x; v[1] = f4.y; v[2] = f4.z; v[3] = f4.w;
+      const real* src = F.f[p] + (long long)ga * g.sx + gb * g.gz + gc;
+      if (VEC && gc + V - 1 < g.gz) {
+        if constexpr (V == 4) {
+          const float4 f4 = __ldg(reinterpret_cast<const float4*>(src));
+          v[0] = f4.x; v[1] = f4.y; v[2] = f4.z; v[3] = f4.w;
+        } else {
+          const double2 f2 = __ldg(reinterpret_cast<const double2*>(src));
+          v[0] = f2.x; v[1] = f2.y;
+        }
       } else {
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
+        for (int e = 0; e < V; ++e)
           if (gc + e < g.gz) v[e] = __ldg(src + e);
       }
     }
-    *reinterpret_cast<float4*>(fw + p * WN + (a * WY + b) * WZ + 4 * c4) = make_float4(v[0], v[1], v[2], v[3]);
+    real* dst = fw + p * WN + (a * WY + b) * WZ + V * c;
+    if constexpr (V == 4) *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+    else *reinterpret_cast<double2*>(dst) = make_double2(v[0], v[1]);
   }
 }
 
@@ -123,10 +171,10 @@ struct HomeJ {
           if (c < 2) jz[a][b][c] = (real)0;
         }
   }
-  __device__ __forceinline__ void add(real qx, real qy, real qz, const Axis<real>& X, const Axis<real>& Y,
-                                      const Axis<real>& Z, const W3<real>& bx, const W3<real>& by,
-                                      const W3<real>& bz) {
-    const real ax[2] = {X.a0, X.a1}, ay[2] = {Y.a0, Y.a1}, az[2] = {Z.a0, Z.a1};
+  // the current (qx, qy, qz) of a particle at the offsets (fx, fy, fz)
+  __device__ __forceinline__ void add(real qx, real qy, real qz, real fx, real fy, real fz, const W3<real>& bx,
+                                      const W3<real>& by, const W3<real>& bz) {
+    const real ax[2] = {(real)1 - fx, fx}, ay[2] = {(real)1 - fy, fy}, az[2] = {(real)1 - fz, fz};
 #pragma unroll
     for (int b = 0; b < 3; ++b)
 #pragma unroll
@@ -152,10 +200,32 @@ struct HomeJ {
         jz[a][b][1] += (qz * az[1]) * xy;
       }
   }
+  template <typename F>
+  __device__ __forceinline__ void each(F f) {
+#pragma unroll
+    for (int q = 0; q < 18; ++q) {
+      f(jx[q / 9][q / 3 % 3][q % 3]);
+      f(jy[q / 6][q / 3 % 2][q % 3]);
+      f(jz[q / 6][q / 2 % 3][q % 2]);
+    }
+  }
   __device__ __forceinline__ real x(int a, int b, int c) const { return jx[a][b][c]; }
   __device__ __forceinline__ real y(int a, int b, int c) const { return jy[a][b][c]; }
   __device__ __forceinline__ real z(int a, int b, int c) const { return jz[a][b][c]; }
 };
+
+// The sums of the lanes that share a cell (lane z of the first nv and z + nv,
+// z + 2 nv, ...) into the first of them: `each` calls its argument on every sum.
+template <typename J>
+__device__ __forceinline__ void merge_lanes(J& acc, int nv, int lane) {
+  for (int from = lane + nv, end = kLanes; nv < end; end -= nv, from += nv) {
+    const bool take = lane < nv && from < kLanes;
+    acc.each([&](auto& v) {
+      const auto o = __shfl_sync(0xffffffffu, v, from & (kLanes - 1));
+      if (take) v += o;
+    });
+  }
+}
 
 // FP32: the two nodes of each component's unshifted axis as one packed pair,
 // updated with the two-wide multiplies and FMAs of sm_100.
@@ -168,12 +238,11 @@ struct HomeJ<float> {
 #pragma unroll
       for (int b = 0; b < 3; ++b) jx[a][b] = jy[a][b] = jz[a][b] = make_float2(0.f, 0.f);
   }
-  __device__ __forceinline__ void add(float qx, float qy, float qz, const Axis<float>& X, const Axis<float>& Y,
-                                      const Axis<float>& Z, const W3<float>& bx, const W3<float>& by,
-                                      const W3<float>& bz) {
-    const float2 qxa = make_float2(qx * X.a0, qx * X.a1);
-    const float2 qya = make_float2(qy * Y.a0, qy * Y.a1);
-    const float2 qza = make_float2(qz * Z.a0, qz * Z.a1);
+  __device__ __forceinline__ void add(float qx, float qy, float qz, float fx, float fy, float fz, const W3<float>& bx,
+                                      const W3<float>& by, const W3<float>& bz) {
+    const float2 qxa = __fmul2_rn(make_float2(qx, qx), make_float2(1.f - fx, fx));
+    const float2 qya = __fmul2_rn(make_float2(qy, qy), make_float2(1.f - fy, fy));
+    const float2 qza = __fmul2_rn(make_float2(qz, qz), make_float2(1.f - fz, fz));
     float2 dx[3], dy[3], dz[3];
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
@@ -193,6 +262,20 @@ struct HomeJ<float> {
         jz[q][r] = __ffma2_rn(tz, dy[r], jz[q][r]);  // b = r
       }
     }
+  }
+  template <typename F>
+  __device__ __forceinline__ void each(F f) {
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        f(jx[q][r].x);
+        f(jx[q][r].y);
+        f(jy[q][r].x);
+        f(jy[q][r].y);
+        f(jz[q][r].x);
+        f(jz[q][r].y);
+      }
   }
   __device__ __forceinline__ float x(int a, int b, int c) const { return a ? jx[b][c].y : jx[b][c].x; }
   __device__ __forceinline__ float y(int a, int b, int c) const { return b ? jy[a][c].y : jy[a][c].x; }
@@ -231,63 +314,173 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" :: "n"(N) : "memory"); }
 
+// Moves a packed cell and its offset by less than a cell per axis: adds the
+// displacement d to f and steps the cell by `unit` (the axis's field of
+// pack_cell) where f leaves [0, 1). unit_fix sees to what that leaves outside:
+// a sum rounded to 1, -0, NaN, and longer moves.
+template <typename real>
+__device__ __forceinline__ void step_axis(int& c, real& f, real d, int unit) {
+  real t = f + d;
+  if (t >= (real)1) {
+    t -= (real)1;
+    c += unit;
+  }
+  if (t < (real)0) {
+    t += (real)1;
+    c -= unit;
+  }
+  f = t;
+}
+template <typename real>
+__device__ __forceinline__ void unit_fix(int& c, real& t, int unit) {
+  if (!off_unit(t)) return;
+  const real fl = floor(t);
+  c += (int)fl * unit;
+  t -= fl;
+  if (t >= (real)1) {
+    t = (real)0;
+    c += unit;
+  }
+}
+constexpr int kUnitX = 1 << (2 * kCellBits), kUnitY = 1 << kCellBits, kUnitZ = 1;
+template <typename real>
+__device__ __forceinline__ void step_cell(int& c, real& fx, real& fy, real& fz, real dx, real dy, real dz) {
+  step_axis(c, fx, dx, kUnitX);
+  step_axis(c, fy, dy, kUnitY);
+  step_axis(c, fz, dz, kUnitZ);
+}
+
+// Record B's fourth word after the main loop: what is left to do for the
+// particle (0 nothing, kLeftAll the whole push, kLeftEnd the density deposit
+// and sr_particle).
+constexpr int kLeftAll = 1, kLeftEnd = 2;
+template <typename real>
+__device__ __forceinline__ int left_of(const Parts<real>& P, int t) { return (int)P.rb[4 * (long long)t + 3]; }
+
+// The slots after the layout (particles without a hole in their group): the
+// slot-order push, in the grid's first blocks.
+template <typename real>
+__device__ __noinline__ void push_tail(const Parts<real>& P, const TileArgs& ta, const Fields<real>& F, const Geom& g,
+                                       const PushConst<real>& pc, unsigned long long* err) {
+  push_slots<real, PUSH_FUSED>(P, ta.tail + blockIdx.x * blockDim.x + threadIdx.x, ta.ntail * blockDim.x, *ta.count, F,
+                               g, pc, err);
+}
+
+// What the main loop left of particle t to the general path.
+template <typename real>
+__device__ __noinline__ void push_rest(const Parts<real>& P, int t, const Fields<real>& F, const Geom& g,
+                                       const PushConst<real>& pc, unsigned long long* err) {
+  const Rec<real> r = load_records(P, t);
+  const int left = left_of(P, t);
+  if (r.cell < 0 || left == 0) return;
+  if (left == kLeftAll) {
+    push_one<real, PUSH_FUSED>(P, t, r, F, g, pc, err);
+    return;
+  }
+  int i, j, k;
+  unpack_cell(r.cell, i, j, k);
+  if (in_array(g, i, j, k)) {
+    if (stencil_ok(g, i, j, k))
+      deposit_n(F, g, pc, axis_weights(i, r.o[0]), axis_weights(j, r.o[1]), axis_weights(k, r.o[2]));
+    else
+      count_err(err, ERR_DEPOSIT_OOB);
+  }
+  const int c = settle(g, pc.out, i, j, k, r.o[0], r.o[1], r.o[2], r.v[0], r.v[1], r.v[2], err);
+  store_records(P, t, c, r.o[0], r.o[1], r.o[2], r.v[0], r.v[1], r.v[2]);
+}
+
 // The fused particle part of one step (push, J deposit at x^{n+1/2}, drift,
 // n deposit at x^{n+1}, sr_particle) for one species over the tiled layout;
 // the same arithmetic as push_kernel<real, PUSH_FUSED> apart from the FP32
 // square roots and divisions and, in FP32, the fixed-point sums of the density
-// window. One CTA per tile, one warp per group.
+// window. One CTA per tile, one warp per group; the first ntail CTAs take the
+// slots after the layout (a launch of their own, 7 to 12 us per species for
+// next to no particles, before).
+//
+// The second species' launch may start before the first has finished (they
+// share nothing but the error counters): every CTA lets it go at once, and the
+// second's CTAs end with a wait for the first, so that whatever follows still
+// finds both done (0.068 -> 0.053 ms per step at 32^3 x 8, 0.336 -> 0.327 at
+// 64^3 x 16, the same at 128^3 x 64).
 //
 // J of a particle in its lane's home cell at x^{n+1/2} is summed in registers;
 // the others add theirs to global memory with reductions (a shared J window
 // taking every particle's 24 weights by FP32 shared atomics, which frees the
-// registers for 3 CTAs per SM, measured 1.7x slower). The density goes to the window with shared
-// reductions (every active lane at once): integer ones on fixed-point sums in
-// FP32, FP64 atomics in FP64.
-// FP64 at one CTA per SM: 254 registers and no spills, against 528 bytes of
-// spill stores per thread at two CTAs per SM (128 registers); measured 30.6 ->
-// 27.2 ms per step for the FP64 push at 128^3 cells x 64 particles/cell/species.
+// registers for 3 CTAs per SM, measured 1.7x slower). The density goes to the
+// window with shared reductions (every active lane at once): integer ones on
+// fixed-point sums in FP32, FP64 atomics in FP64.
+//
+// Bound by instruction issue (16 warps per SM, 55 % of the slots issue; DRAM at
+// 17 %), so the loop is written for few instructions: cells stay packed while
+// they move (step_cell), one range test says that a particle needs no bounds
+// checks, window addresses come from one multiply-add chain and the lanes
+// without a particle run along with zero currents instead of branching. What
+// the test refuses -- a particle wrapped to the other side of the domain, or
+// more than a cell outside its tile -- goes to push_rest after the loop.
+// Against the checks and branches per particle that this replaces, push per
+// step of both species: 7.06 -> 6.55 ms at 128^3 x 64, 0.327 -> 0.309 at
+// 64^3 x 16, 0.203 -> 0.183 at 41 x 22 x 70 x 30 (sides that no tile divides),
+// FP64 64^3 x 32 1.72 -> 1.61. Rows loaded into registers one ahead, without
+// the ring: 7.7 ms at 128^3 x 64.
+// FP64 runs one CTA per SM: 254 registers and no spills, against 528 bytes of
+// spill stores per thread at two (128 registers); 27.2 against 30.6 ms per step
+// at 128^3 x 64. That leaves room for the field window and the J queue.
 #ifndef PB_PUSH64_MIN_BLOCKS
 #define PB_PUSH64_MIN_BLOCKS 1
 #endif
-template <typename real, bool VEC_FLUSH>
+template <typename real, bool VEC>
 __global__ void __launch_bounds__(kTileX * kTileY * 32, sizeof(real) == 4 ? 2 : PB_PUSH64_MIN_BLOCKS)
-push_tiled_kernel(Parts<real> P, TileArgs ta, Fields<real> F, Geom g, PushConst<real> pc, unsigned long long* err) {
+push_tiled_kernel(const __grid_constant__ Parts<real> P, const __grid_constant__ TileArgs ta,
+                  const __grid_constant__ Fields<real> F, const __grid_constant__ Geom g,
+                  const __grid_constant__ PushConst<real> pc, unsigned long long* err) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if ((int)blockIdx.x < ta.ntail) {
+    push_tail(P, ta, F, g, pc, err);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    return;
+  }
   using S = PushSmem<real>;
-  constexpr int WY = S::WY, WZ = S::WZ, WN = S::WN, WX = S::WX;
+  constexpr int WY = S::WY, WZ = S::WZ, WN = S::WN, WX = S::WX, NS = kStages<real>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  real* win = reinterpret_cast<real*>(smem_raw);  // [4][WN]: jx, jy, jz, n
-  const int tile = blockIdx.x;
+  real* wn = reinterpret_cast<real*>(smem_raw);                // [WN]: n
+  real* wj = reinterpret_cast<real*>(smem_raw + S::ring_off);  // [3][WN]: jx, jy, jz, after the last row
+  real* fw = reinterpret_cast<real*>(smem_raw + S::fwin_off);  // [6][WN]: E, B
+  const int tile = blockIdx.x - ta.ntail;
   const TileGeom& t = ta.t;
   const int tz = tile % t.ntz, ty = (tile / t.ntz) % t.nty, tx = tile / (t.ntz * t.nty);
   // window origin: two nodes below the tile's first interior cell (2 + tx*TX)
   const int wx0 = tx * kTileX, wy0 = ty * kTileY, wz0 = tz * kLanes;
-  for (int q = threadIdx.x; q < 4 * WN; q += blockDim.x) win[q] = (real)0;
-  // FP32: E and B over the window, one plane per component
-  float* fw = reinterpret_cast<float*>(smem_raw + S::fwin_off);
-  // the interior cells: a particle in one needs none of the array bounds,
-  // ballistic or sr_particle checks (below), wherever it sits relative to the
-  // tile (testing the tile's own cells instead sent every particle that had
-  // crossed into a neighbouring tile down those paths)
-  const InteriorBox tb{2, 2, 2, (unsigned)g.nx, (unsigned)g.ny, (unsigned)g.nz};
-  if constexpr (S::kFieldWin) fill_win<WX, WY, WZ, VEC_FLUSH>(fw, F, g, wx0, wy0, wz0);
+  for (int q = threadIdx.x; q < WN; q += blockDim.x) wn[q] = (real)0;
+  fill_win<real, WX, WY, WZ, VEC>(fw, F, g, wx0, wy0, wz0);
   __syncthreads();
+  // the interior cells whose stencils lie in the window: a particle in one
+  // needs no check of the array's bounds and none of sr_particle's
+  CellRange near;
+  near.lx = max(wx0 + 1, 2);
+  near.ly = max(wy0 + 1, 2);
+  near.lz = max(wz0 + 1, 2);
+  near.ex = (unsigned)(min(wx0 + WX - 1, g.nx + 2) - near.lx);
+  near.ey = (unsigned)(min(wy0 + WY - 1, g.ny + 2) - near.ly);
+  near.ez = (unsigned)(min(wz0 + WZ - 1, g.nz + 2) - near.lz);
+  if (pc.long_moves) near.ex = 0;  // nobody takes the short path
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int G = tile * (kTileX * kTileY) + warp;
   const int base = ta.goff[G], jmax = ta.gtop[G];
   // home cell of this lane
-  const int hi = wx0 + 2 + warp / kTileY, hj = wy0 + 2 + warp % kTileY, hk = wz0 + 2 + lane;
+  const int hi = wx0 + 2 + warp / kTileY, hj = wy0 + 2 + warp % kTileY;
+  const int nv = tile_cells(g, tz), hk = wz0 + 2 + lane_cell(nv, lane).z;
   const int hcell = pack_cell(hi, hj, hk);
-  real* wn = win + 3 * WN;
-  // FP32: the density window holds fixed-point sums (scatter8_win_fixed) at a
-  // scale that no node of this tile can overflow
+  const int wcell0 = (wx0 * WY + wy0) * WZ + wz0;  // window node of a cell: (i WY + j) WZ + k less this
+  // FP32: the density window holds fixed-point sums (add_density) at a scale
+  // that no node of this tile can overflow
   constexpr bool kFixedN = sizeof(real) == 4;
-  float nscale = 0.f;
+  real nscale = pc.nw;
   if (kFixedN) {
     int slots = 0;
 #pragma unroll
     for (int w = 0; w < kTileX * kTileY; ++w) slots += ta.gtop[tile * (kTileX * kTileY) + w];
-    // below 2^23 as well, where scatter8_win_fixed's rounding by an added 2^23 is exact
-    nscale = fminf(4294967295.f / (float)(slots * kLanes + 1), 8388607.f);
+    // below 2^23 as well, where add_density's rounding by an added 2^23 is exact
+    nscale = (real)fminf(4294967295.f / (float)(slots * kLanes + 1), 8388607.f);
   }
   HomeJ<real> acc;
   acc.zero();
@@ -296,151 +489,149 @@ push_tiled_kernel(Parts<real> P, TileArgs ta, Fields<real> F, Geom g, PushConst<
   // They go to the planes with global reductions (into the shared J window by
   // FP32 shared atomics, where the stencil allowed, measured 0.7 ms per step
   // slower; z-adjacent pairs as 16-byte vector reductions, 0.2 ms slower)
-  float* jq = reinterpret_cast<float*>(smem_raw + S::jq_off) + warp * S::kQ * 7;
+  real* jq = reinterpret_cast<real*>(smem_raw + S::jq_off) + warp * S::kQ * 7;
   int nq = 0;
   auto deposit_queued = [&](int q) {
-    const float* e = jq + q * 7;
+    const real* e = jq + q * 7;
     int qi, qj, qk;
-    unpack_cell(__float_as_int(e[0]), qi, qj, qk);
-    const Axis<real> X = axis_weights(qi, (real)e[1]), Y = axis_weights(qj, (real)e[2]), Z = axis_weights(qk, (real)e[3]);
-    deposit_j(F, g, pc, X, Y, Z, (real)e[4], (real)e[5], (real)e[6]);
+    unpack_cell(word_int(e[0]), qi, qj, qk);
+    const Axis<real> X = axis_weights(qi, e[1]), Y = axis_weights(qj, e[2]), Z = axis_weights(qk, e[3]);
+    deposit_j(F, g, pc, X, Y, Z, e[4], e[5], e[6]);
   };
+  // slots left to push_rest: the first kRest of them in a list
+  int* rest = reinterpret_cast<int*>(smem_raw + S::slow_off) + warp * S::kRest;
+  int nrest = 0;
   // ring of particle rows fetched ahead; each lane copies and reads only its
   // own slots, so the per-thread cp.async groups need no warp barrier. A
   // stage holds the row's 32 records A, then its 32 records B, so that the
   // lanes' 16-byte reads of one record fall on consecutive banks.
-  real* prec = reinterpret_cast<real*>(smem_raw + S::prec_off) + warp * kStages * kLanes * 8;
+  real* ring = reinterpret_cast<real*>(smem_raw + S::ring_off) + warp * NS * kLanes * 8;
   auto fetch = [&](int row) {
     if (row < jmax) {
-      real* stage = prec + (row % kStages) * kLanes * 8;
+      real* stage = ring + (row % NS) * kLanes * 8;
       fetch_records(stage + lane * 4, stage + (kLanes + lane) * 4, P, base + row * kLanes + lane);
     }
     cp_async_commit();
   };
 #pragma unroll
-  for (int s = 0; s < kStages - 1; ++s) fetch(s);
-  unsigned pushed = 0;
+  for (int s = 0; s < NS - 1; ++s) fetch(s);
+  unsigned pushed = 0, nbad = 0;
   for (int jj = 0; jj < jmax; ++jj) {
-    fetch(jj + kStages - 1);
-    cp_async_wait<kStages - 1>();
-    const int t = base + jj * kLanes + lane;
-    const int st = jj % kStages;
+    fetch(jj + NS - 1);
+    cp_async_wait<NS - 1>();
+    const int slot = base + jj * kLanes + lane;
+    const real* stage = ring + (jj % NS) * kLanes * 8;
     real ra[4], rb[4];
-    read_record(prec + st * kLanes * 8 + lane * 4, ra);
-    read_record(prec + st * kLanes * 8 + (kLanes + lane) * 4, rb);
-    int c;
-    if constexpr (sizeof(real) == 4) c = __float_as_int((float)ra[0]);
-    else c = __double2loint((double)ra[0]);
-    const bool act = c >= 0;
-    int i = 0, j = 0, k = 0;
-    real fx = 0, fy = 0, fz = 0, vx = 0, vy = 0, vz = 0;
-    bool enq = false;  // J at x^{n+1/2} goes to the warp's queue
-    int chalf = 0;     // the packed cell at x^{n+1/2}
-    if (act) {
-      ++pushed;
+    read_record(stage + lane * 4, ra);
+    read_record(stage + (kLanes + lane) * 4, rb);
+    int c = word_int(ra[0]);
+    real fx = ra[1], fy = ra[2], fz = ra[3];
+    real vx = rb[0], vy = rb[1], vz = rb[2];
+    pushed += c >= 0;
+    int i, j, k;
+    unpack_cell(c, i, j, k);
+    bool quick = near.has(i, j, k);  // never for an empty slot
+    bool push = quick;
+    if (pc.bal_interior && quick && ballistic(pc, i, j, k, fx, fy, fz)) {
+      push = false;
+      // a velocity that Boris has not bounded by c
+      quick = fabs(vx * pc.hdt) < (real)1 && fabs(vy * pc.hdt) < (real)1 && fabs(vz * pc.hdt) < (real)1;
+    }
+    int left = c >= 0 && !quick ? kLeftAll : 0;
+    if (push) {
+      const WinAxis<real> X = win_axis(fx, WY * WZ), Y = win_axis(fy, WZ), Z = win_axis(fz, 1);
+      const real* n = fw + ((i * WY + j) * WZ + k - wcell0);
+      boris4_fast(pc, gather6_win<WY, WZ, WN>(n, X, Y, Z), vx, vy, vz);
+      // one test for the three: |v| < c, so the sum of finite components is finite
+      nbad += !isfinite(vx + vy + vz);
+    }
+    // From here to the density every lane runs, with no branch: a lane without
+    // a particle, or whose particle is off its home cell, adds zero currents
+    // (weights of offsets in [0, 1], whatever an empty slot holds).
+    if (!quick) fx = fy = fz = (real)0.5;
+    const real dx = vx * pc.hdt, dy = vy * pc.hdt, dz = vz * pc.hdt;
+    // an offset rounded to 1 or -0 deposits the same current as in the cell it
+    // belongs to; the second half step puts it there
+    step_cell(c, fx, fy, fz, dx, dy, dz);
+    const bool home = quick && c == hcell;
+    {
+      const W3<real> bx = home3(fx), by = home3(fy), bz = home3(fz);
+      acc.add(home ? pc.qn * vx : (real)0, home ? pc.qn * vy : (real)0, home ? pc.qn * vz : (real)0, fx, fy, fz, bx, by,
+              bz);
+    }
+    // the others' currents go to the warp's queue: the row's queued lanes take
+    // consecutive entries; a full warp's worth is deposited by all 32 lanes at
+    // once (less than a cell from the interior, their stencils lie in the array)
+    const bool enq = quick && !home;
+    const unsigned em = __ballot_sync(0xffffffffu, enq);
+    if (em) {
+      if (enq) {
+        real* e = jq + (nq + __popc(em & ((1u << lane) - 1u))) * 7;
+        e[0] = int_word<real>(c);
+        e[1] = fx; e[2] = fy; e[3] = fz;
+        e[4] = vx; e[5] = vy; e[6] = vz;
+      }
+      nq += __popc(em);
+      if (nq >= kLanes) {
+        __syncwarp();
+        deposit_queued(nq - kLanes + lane);
+        nq -= kLanes;
+        __syncwarp();
+      }
+    }
+    step_cell(c, fx, fy, fz, dx, dy, dz);
+    if (quick) {
+      if (off_unit(fx) || off_unit(fy) || off_unit(fz)) {
+        unit_fix(c, fx, kUnitX);
+        unit_fix(c, fy, kUnitY);
+        unit_fix(c, fz, kUnitZ);
+      }
       unpack_cell(c, i, j, k);
-      fx = ra[1]; fy = ra[2]; fz = ra[3];
-      vx = rb[0]; vy = rb[1]; vz = rb[2];
-      // a particle in an interior cell has its stencils in the array, and it
-      // is ballistic only when the Absorb_grid2 layer reaches interior cells
-      const bool inside = tb.has(i, j, k);
-      bool bal = (pc.bal_interior || !inside) && ballistic(pc, i, j, k, fx, fy, fz);
-      if (!bal && !inside && !stencil_ok(g, i, j, k)) {
-        count_err(err, ERR_DEPOSIT_OOB);
-        bal = true;
+      int cnew = c;
+      bool dep = near.has(i, j, k);
+      if (!dep) {
+        // past the interior (sr_particle's business), or out of the window too
+        dep = (unsigned)(i - wx0 - 1) < WX - 2 && (unsigned)(j - wy0 - 1) < WY - 2 && (unsigned)(k - wz0 - 1) < WZ - 2 &&
+              stencil_ok(g, i, j, k);
+        if (dep) cnew = settle(g, pc.out, i, j, k, fx, fy, fz, vx, vy, vz, err);
+        else left = kLeftEnd;
       }
-      if (!bal) {
-        const Axis<real> X = axis_weights(i, fx), Y = axis_weights(j, fy), Z = axis_weights(k, fz);
-        if constexpr (S::kFieldWin) {
-          // the window covers the stencils of particles within two halo nodes of the tile
-          const bool in_win = i - 1 >= wx0 && i + 1 < wx0 + WX && j - 1 >= wy0 && j + 1 < wy0 + WY &&
-                              k - 1 >= wz0 && k + 1 < wz0 + WZ;
-          if (in_win)
-            boris4_fast(pc, gather6_win<WY, WZ, WN>(fw, wx0, wy0, wz0, X, Y, Z), vx, vy, vz);
-          else
-            boris4_fast(pc, gather6(F, g, X, Y, Z), vx, vy, vz);
-        } else {
-          boris4_fast(pc, gather6(F, g, X, Y, Z), vx, vy, vz);
-        }
-        // one test for the three: |v| < c, so the sum of finite components is finite
-        if (!isfinite(vx + vy + vz)) count_err(err, ERR_NONFINITE);
+      if (dep) {  // n at x^{n+1}
+        const int w = ((c >> (2 * kCellBits)) * WY + ((c >> kCellBits) & kCellMask)) * WZ + (c & kCellMask) - wcell0;
+        const WinAxis<real> X = win_axis(fx, WY * WZ), Y = win_axis(fy, WZ), Z = win_axis(fz, 1);
+        add_density<WY, WZ>(wn + w + X.s + Y.s + Z.s, nscale, X, Y, Z);
       }
-      advance(i, fx, vx * pc.hdt);
-      advance(j, fy, vy * pc.hdt);
-      advance(k, fz, vz * pc.hdt);
-      // J at x^{n+1/2}
-      // compared packed: a half step moves an index at most a cell past the
-      // padded array, where a -1 packs negative and a kMaxDim sets a bit that
-      // only an index 0 or 1 next to it could match, and home cells have indices >= 2
-      chalf = pack_cell(i, j, k);
-      if (chalf == hcell) {
-        const Axis<real> X = axis_weights(i, fx), Y = axis_weights(j, fy), Z = axis_weights(k, fz);
-        const W3<real> bx = home3(X, hi), by = home3(Y, hj), bz = home3(Z, hk);
-        acc.add(pc.qn * vx, pc.qn * vy, pc.qn * vz, X, Y, Z, bx, by, bz);
-      } else if (in_array(g, i, j, k)) {
-        if (stencil_ok(g, i, j, k)) {
-          if constexpr (S::kJQueue) {
-            enq = true;
-          } else {
-            const Axis<real> X = axis_weights(i, fx), Y = axis_weights(j, fy), Z = axis_weights(k, fz);
-            deposit_j(F, g, pc, X, Y, Z, vx, vy, vz);
-          }
-        } else {
-          count_err(err, ERR_DEPOSIT_OOB);
-        }
-      }
+      store_records(P, slot, cnew, fx, fy, fz, vx, vy, vz, (real)left);
+    } else if (left) {
+      P.rb[4 * (long long)slot + 3] = (real)kLeftAll;
     }
-    if constexpr (S::kJQueue) {
-      // warp-uniform: the row's queued lanes take consecutive entries; a full
-      // warp's worth is deposited by all 32 lanes at once
-      const unsigned em = __ballot_sync(0xffffffffu, enq);
-      if (em) {
-        if (enq) {
-          float* e = jq + (nq + __popc(em & ((1u << lane) - 1u))) * 7;
-          e[0] = __int_as_float(chalf);
-          e[1] = (float)fx; e[2] = (float)fy; e[3] = (float)fz;
-          e[4] = (float)vx; e[5] = (float)vy; e[6] = (float)vz;
-        }
-        nq += __popc(em);
-        if (nq >= kLanes) {
-          __syncwarp();
-          deposit_queued(nq - kLanes + lane);
-          nq -= kLanes;
-          __syncwarp();
-        }
-      }
-    }
-    if (act) {
-      advance(i, fx, vx * pc.hdt);
-      advance(j, fy, vy * pc.hdt);
-      advance(k, fz, vz * pc.hdt);
-      // n at x^{n+1}
-      const bool inside1 = tb.has(i, j, k);
-      if (inside1 || in_array(g, i, j, k)) {
-        if (inside1 || stencil_ok(g, i, j, k)) {
-          const Axis<real> X = axis_weights(i, fx), Y = axis_weights(j, fy), Z = axis_weights(k, fz);
-          if constexpr (kFixedN)
-            scatter8_win_fixed(reinterpret_cast<unsigned*>(wn), wx0, wy0, wz0, F.f[pc.pn], g, X.b, Y.b, Z.b,
-                               pc.nw, nscale, X.b0, X.b1, Y.b0, Y.b1, Z.b0, Z.b1);
-          else
-            scatter8_win(wn, wx0, wy0, wz0, F.f[pc.pn], g, X.b, Y.b, Z.b, pc.nw, X.b0, X.b1, Y.b0, Y.b1, Z.b0, Z.b1);
-        } else {
-          count_err(err, ERR_DEPOSIT_OOB);
-        }
-      }
-      // sr_particle keeps a particle of an interior cell where it is
-      const int cnew = inside1 ? pack_cell(i, j, k) : settle(g, pc.out, i, j, k, fx, fy, fz, vx, vy, vz, err);
-      store_records(P, t, cnew, fx, fy, fz, vx, vy, vz);
+    const unsigned lm = __ballot_sync(0xffffffffu, left != 0);
+    if (lm) {
+      const int q = nrest + __popc(lm & ((1u << lane) - 1u));
+      if (left && q < S::kRest) rest[q] = slot;
+      nrest += __popc(lm);
     }
   }
-  if constexpr (S::kJQueue) {
-    __syncwarp();
-    if (lane < nq) deposit_queued(lane);
-  }
+  if (nbad) atomicAdd(err + ERR_NONFINITE, (unsigned long long)nbad);
+  __syncwarp();
+  if (lane < nq) deposit_queued(lane);
   for (int o = 16; o > 0; o >>= 1) pushed += __shfl_down_sync(0xffffffffu, pushed, o);
   if (lane == 0 && pushed) atomicAdd(err + CNT_PUSHED, (unsigned long long)pushed);
+  // what the loop left: the list (particles that have crossed the periodic
+  // faces of x and y since the last re-layout, mostly), or every row when the
+  // list overflowed
+  if (nrest > S::kRest) {
+    for (int jj = 0; jj < jmax; ++jj) push_rest(P, base + jj * kLanes + lane, F, g, pc, err);
+  } else {
+    for (int q = lane; q < nrest; q += kLanes) push_rest(P, rest[q], F, g, pc, err);
+  }
   // the lane's home-cell sums into the window (nodes h-1 .. h+1 around it)
-  if (jmax > 0) {
+  cp_async_wait<0>();
+  __syncthreads();
+  for (int q = threadIdx.x; q < 3 * WN; q += blockDim.x) wj[q] = (real)0;
+  __syncthreads();
+  if (nv < kLanes) merge_lanes(acc, nv, lane);
+  if (jmax > 0 && lane < nv) {
     const int la = hi - 1 - wx0, lb = hj - 1 - wy0, lc = hk - 1 - wz0;  // window index of node h-1
 #pragma unroll
     for (int a = 0; a < 3; ++a)
@@ -449,9 +640,9 @@ push_tiled_kernel(Parts<real> P, TileArgs ta, Fields<real> F, Geom g, PushConst<
 #pragma unroll
         for (int cc = 0; cc < 3; ++cc) {
           const int s = ((la + a) * WY + (lb + b)) * WZ + (lc + cc);
-          if (a < 2) atomicAdd(win + s + WY * WZ, acc.x(a, b, cc));       // x nodes h, h+1
-          if (b < 2) atomicAdd(win + WN + s + WZ, acc.y(a, b, cc));       // y nodes h, h+1
-          if (cc < 2) atomicAdd(win + 2 * WN + s + 1, acc.z(a, b, cc));   // z nodes h, h+1
+          if (a < 2) atomicAdd(wj + s + WY * WZ, acc.x(a, b, cc));       // x nodes h, h+1
+          if (b < 2) atomicAdd(wj + WN + s + WZ, acc.y(a, b, cc));       // y nodes h, h+1
+          if (cc < 2) atomicAdd(wj + 2 * WN + s + 1, acc.z(a, b, cc));   // z nodes h, h+1
         }
   }
   __syncthreads();
@@ -464,16 +655,16 @@ push_tiled_kernel(Parts<real> P, TileArgs ta, Fields<real> F, Geom g, PushConst<
     const int a = r / (WY * NZ4), b = (r / NZ4) % WY, c4 = r % NZ4;
     const int ga = wx0 + a, gb = wy0 + b, gc = wz0 + 4 * c4;
     if (ga >= g.gx || gb >= g.gy || gc >= g.gz) continue;
-    const real* src = win + q * WN + (a * WY + b) * WZ + 4 * c4;
+    const real* src = (q == 3 ? wn : wj + q * WN) + (a * WY + b) * WZ + 4 * c4;
     real v0 = src[0], v1 = src[1], v2 = src[2], v3 = src[3];
     if (kFixedN && q == 3) {  // fixed-point density sums back to weights
       const unsigned* u = reinterpret_cast<const unsigned*>(src);
-      const real back = pc.nw / (real)nscale;
+      const real back = pc.nw / nscale;
       v0 = (real)u[0] * back; v1 = (real)u[1] * back; v2 = (real)u[2] * back; v3 = (real)u[3] * back;
     }
     if (v0 == (real)0 && v1 == (real)0 && v2 == (real)0 && v3 == (real)0) continue;
     real* dst = F.f[planes[q]] + ga * g.sx + gb * g.gz + gc;
-    if (VEC_FLUSH) {
+    if (VEC && sizeof(real) == 4) {
       red_add_v4(reinterpret_cast<float*>(dst), (float)v0, (float)v1, (float)v2, (float)v3);
     } else {
       const real v[4] = {v0, v1, v2, v3};
@@ -482,6 +673,7 @@ push_tiled_kernel(Parts<real> P, TileArgs ta, Fields<real> F, Geom g, PushConst<
         if (gc + e < g.gz && v[e] != (real)0) atomicAdd(dst + e, v[e]);
     }
   }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 

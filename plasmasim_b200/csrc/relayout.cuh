@@ -52,7 +52,8 @@ __global__ void classify_kernel(Parts<real> P, Geom g, TileGeom t, const int* __
   const int lane = threadIdx.x & 31;
   if (G >= t.ngroups) return;  // warp-uniform
   const unsigned below = (1u << lane) - 1u;
-  const int home = home_key(g, t, G, lane);
+  LaneCell lc;
+  const int home = home_key(g, t, G, lane, lc);
   const int base = goff[G], m = gmax[G];
   int nh = 0, top = 0;
   int blk = 0, used = kAppendBlock;  // current block of append slots (warp-uniform)
@@ -174,11 +175,13 @@ __global__ void place_fill_kernel(Parts<real> P, int first, Geom g, TileGeom t, 
   const int lane = threadIdx.x & 31;
   if (G >= t.ngroups) return;  // warp-uniform
   const unsigned below = (1u << lane) - 1u;
-  const int home = home_key(g, t, G, lane);
-  const int arr = home >= 0 ? arrivals[home] : 0;
+  LaneCell lc;
+  const int home = home_key(g, t, G, lane, lc);
+  // this lane's entries of its cell's bucket: o, o + lc.n, ...
+  const int arr = home >= 0 ? lane_share(arrivals[home], lc) : 0;
   const int narr = warp_sum(arr);
   if (narr == 0) return;
-  const int o = home >= 0 ? off[home] : 0;
+  const int o = home >= 0 ? off[home] + lc.m : 0;
   const int nh = nholes[G * kLanes + lane];
   const int base = goff[G], rows = gmax[G];
   const int level = min(rows, group_level(rows * kLanes - warp_sum(nh) + narr));
@@ -192,7 +195,7 @@ __global__ void place_fill_kernel(Parts<real> P, int first, Geom g, TileGeom t, 
     for (int u = 0; u < U; ++u) {
       const int k = k0 + u;
       const int row = k < n ? holes[base + k * kLanes + lane] : level;
-      src[u] = row < level ? first + bucket[o + k] : -1;
+      src[u] = row < level ? first + bucket[o + k * lc.n] : -1;
       dst[u] = base + row * kLanes + lane;
       if (row < level) {
         top = max(top, row + 1);
@@ -205,7 +208,7 @@ __global__ void place_fill_kernel(Parts<real> P, int first, Geom g, TileGeom t, 
       if (src[u] >= 0) copy_record(P, src[u], P, dst[u], P.cell[src[u]]);
     if (!__any_sync(0xffffffffu, more)) break;
   }
-  // strangers: number s of the group is entry used + (s - pre) of its lane's bucket
+  // strangers: number s of the group is entry used + (s - pre) of its lane's
   const int rest = arr - used;
   const int pre = warp_scan(rest) - rest;
   const int nrest = warp_sum(rest);
@@ -219,7 +222,7 @@ __global__ void place_fill_kernel(Parts<real> P, int first, Geom g, TileGeom t, 
 #pragma unroll
     for (int q = 16; q > 0; q >>= 1)
       if (__shfl_sync(0xffffffffu, pre, b + q) <= s) b += q;
-    const int e = __shfl_sync(0xffffffffu, o + used - pre, b) + s;
+    const int e = __shfl_sync(0xffffffffu, o, b) + (__shfl_sync(0xffffffffu, used - pre, b) + s) * __shfl_sync(0xffffffffu, lc.n, b);
     if (row < level && s < nrest) {
       const int src = first + bucket[e];
       top = max(top, row + 1);
@@ -234,7 +237,7 @@ __global__ void place_fill_kernel(Parts<real> P, int first, Geom g, TileGeom t, 
 #pragma unroll
     for (int q = 16; q > 0; q >>= 1)
       if (__shfl_sync(0xffffffffu, pre, b + q) <= s) b += q;
-    const int e = __shfl_sync(0xffffffffu, o + used - pre, b) + s;
+    const int e = __shfl_sync(0xffffffffu, o, b) + (__shfl_sync(0xffffffffu, used - pre, b) + s) * __shfl_sync(0xffffffffu, lc.n, b);
     int sb = 0;
     if (lane == 0) sb = atomicAdd(nspill, min(kLanes, nrest - s0));
     sb = __shfl_sync(0xffffffffu, sb, 0);

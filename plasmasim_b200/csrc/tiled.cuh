@@ -69,6 +69,9 @@ struct TileArgs {
   TileGeom t;
   const int* goff;  // first slot of each group
   const int* gtop;  // rows of each group up to the last one that holds a particle
+  int ntail;        // CTAs of the grid that take the slots from `tail` to *count instead of a tile
+  int tail;
+  const int* count;
 };
 
 // Group and lane of an interior cell (absolute indices), -1 outside the interior.
@@ -83,16 +86,50 @@ __device__ __forceinline__ int group_of(const Geom& g, const TileGeom& t, int i,
   return tile * (kTileX * kTileY) + wx * kTileY + wy;
 }
 
-// Interior cell key of group G's lane, or -1 when the lane has no cell.
-__device__ __forceinline__ int home_key(const Geom& g, const TileGeom& t, int G, int lane) {
+// The cell that a lane of z tile tz owns. Where the interior ends inside the
+// tile (nv < 32 cells), the lanes past its last cell own the tile's cells over
+// again: cell z has the lanes z, z + nv, z + 2 nv, ..., n of them, and this is
+// number m. (Where such lanes held nothing but strangers, the push of both
+// species took 0.180, 0.464, 0.186 and 0.249 ms per step with nz = 20, 45, 70
+// and 36, this way 0.137, 0.404, 0.180 and 0.244.)
+struct LaneCell {
+  int z, m, n;
+};
+__device__ __forceinline__ int tile_cells(const Geom& g, int tz) { return min(kLanes, g.nz - tz * kLanes); }
+__device__ __forceinline__ int lanes_of(int nv, int z) { return nv == kLanes ? 1 : (kLanes - 1 - z) / nv + 1; }
+__device__ __forceinline__ LaneCell lane_cell(int nv, int lane) {
+  if (nv == kLanes) return {lane, 0, 1};
+  const int z = lane % nv;
+  return {z, lane / nv, lanes_of(nv, z)};
+}
+// This lane's part of the c particles of its cell: those ranked m, m + n, ...
+__device__ __forceinline__ int lane_share(int c, const LaneCell& l) { return (c + l.n - 1 - l.m) / l.n; }
+
+// Absolute indices of the cell that group G's lane owns; false when it owns none.
+__device__ __forceinline__ bool home_cell(const Geom& g, const TileGeom& t, int G, int lane, int& i, int& j, int& k,
+                                          LaneCell& l) {
   const int tile = G / (kTileX * kTileY), w = G % (kTileX * kTileY);
   const int tz = tile % t.ntz, ty = (tile / t.ntz) % t.nty, tx = tile / (t.ntz * t.nty);
-  const int i = tx * kTileX + w / kTileY, j = ty * kTileY + w % kTileY, k = tz * kLanes + lane;
-  if (i >= g.nx || j >= g.ny || k >= g.nz) return -1;
-  return (i * g.ny + j) * g.nz + k;
+  l = lane_cell(tile_cells(g, tz), lane);
+  i = tx * kTileX + w / kTileY;
+  j = ty * kTileY + w % kTileY;
+  k = tz * kLanes + l.z;
+  const bool ok = i < g.nx && j < g.ny;
+  i += 2; j += 2; k += 2;
+  return ok;
 }
 
-// Group and lane of an interior cell key.
+// Interior cell key of group G's lane, or -1 when the lane has no cell.
+__device__ __forceinline__ int home_key(const Geom& g, const TileGeom& t, int G, int lane, LaneCell& l) {
+  int i, j, k;
+  return home_cell(g, t, G, lane, i, j, k, l) ? ((i - 2) * g.ny + (j - 2)) * g.nz + (k - 2) : -1;
+}
+
+__device__ __forceinline__ int cells_of_group(const Geom& g, const TileGeom& t, int G) {
+  return tile_cells(g, G / (kTileX * kTileY) % t.ntz);
+}
+
+// Group and (first) lane of an interior cell key.
 __device__ __forceinline__ int group_of_key(const Geom& g, const TileGeom& t, int key, int& lane) {
   const int k = key % g.nz, j = (key / g.nz) % g.ny, i = key / (g.nz * g.ny);
   return group_of(g, t, i + 2, j + 2, k + 2, lane);
@@ -107,7 +144,9 @@ __global__ void tiled_count_kernel(Parts<real> P, Geom g, TileGeom t, const int*
   const int G = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (G >= t.ngroups) return;
-  const int home = home_key(g, t, G, lane);
+  LaneCell lc;
+  int home = home_key(g, t, G, lane, lc);
+  if (lc.n > 1) home = -1;  // the lanes of one cell have no common order: all movers
   const int base = goff[G], m = gmax[G];
   int nstay = 0;
   constexpr int U = 8;  // rows whose loads are in flight together
@@ -123,7 +162,7 @@ __global__ void tiled_count_kernel(Parts<real> P, Geom g, TileGeom t, const int*
       else atomicAdd(moved + key, 1);
     }
   }
-  if (home >= 0) stay[home] = nstay;
+  if (home >= 0) stay[home] = nstay;  // cleared before: cells of several lanes keep 0
 }
 
 template <typename real>
@@ -136,27 +175,15 @@ __global__ void append_count_kernel(Parts<real> P, int first, const int* __restr
   }
 }
 
-// Absolute indices of group G's lane cell; false when the lane has no cell.
-__device__ __forceinline__ bool home_cell(const Geom& g, const TileGeom& t, int G, int lane, int& i,
-                                          int& j, int& k) {
-  const int tile = G / (kTileX * kTileY), w = G % (kTileX * kTileY);
-  const int tz = tile % t.ntz, ty = (tile / t.ntz) % t.nty, tx = tile / (t.ntz * t.nty);
-  i = tx * kTileX + w / kTileY;
-  j = ty * kTileY + w % kTileY;
-  k = tz * kLanes + lane;
-  const bool ok = i < g.nx && j < g.ny && k < g.nz;
-  i += 2; j += 2; k += 2;
-  return ok;
-}
-
 // Rows a lane column keeps for the boundary refill of its cell: the refill's
 // particle count plus an eighth and four, so that the refill fits into the
 // column's empty slots without moving other particles.
 __device__ __forceinline__ int refill_reserve(const SourceParams& sp, const Geom& g, const TileGeom& t,
                                               int G, int lane) {
   int i, j, k;
-  if (!home_cell(g, t, G, lane, i, j, k)) return 0;
-  const int need = slab_need(sp, i, j, k);
+  LaneCell l;
+  if (!home_cell(g, t, G, lane, i, j, k, l)) return 0;
+  const int need = lane_share(slab_need(sp, i, j, k), l);
   return need > 0 ? need + need / 8 + 4 : 0;
 }
 
@@ -190,8 +217,9 @@ __global__ void group_size_kernel(Geom g, TileGeom t, const int* __restrict__ st
   const int G = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (G >= t.ngroups) return;
-  const int home = home_key(g, t, G, lane);
-  const int c = home >= 0 ? stay[home] + moved[home] : 0;
+  LaneCell lc;
+  const int home = home_key(g, t, G, lane, lc);
+  const int c = home >= 0 ? lane_share(stay[home] + moved[home], lc) : 0;
   const int level = group_level(warp_sum(c));
   const int room = group_level(warp_sum(max(c, refill_reserve(refill, g, t, G, lane))));
   const int rows = room > 0 ? room + room / kSlackDiv + kSlackRows : 0;
@@ -213,8 +241,9 @@ __global__ void group_pad_kernel(Geom g, TileGeom t, const int* __restrict__ sta
   const int G = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (G >= t.ngroups) return;
-  const int home = home_key(g, t, G, lane);
-  const int c = min(home >= 0 ? stay[home] + moved[home] : 0, gtop[G]);
+  LaneCell lc;
+  const int home = home_key(g, t, G, lane, lc);
+  const int c = min(home >= 0 ? lane_share(stay[home] + moved[home], lc) : 0, gtop[G]);
   const int m = gmax[G], base = goff[G];
   for (int r = c; r < m; ++r) cell[base + r * kLanes + lane] = -1;
 }
@@ -229,12 +258,14 @@ struct NewLayout {
   int* gcursor;       // per group: strangers placed so far
 };
 
-// Slot of the particle ranked `rank` of the cell of group G, lane l: its own
-// column below the level, else the group's next free slot (the slots below
-// the level hold the whole group, so every stranger finds one).
-__device__ __forceinline__ int layout_slot(const NewLayout& nl, int G, int l, int rank) {
+// Slot of the particle ranked `rank` of cell z of group G, whose z tile has nv
+// cells: one of its own columns below the level, else the group's next free
+// slot (the slots below the level hold the whole group, so every stranger
+// finds one).
+__device__ __forceinline__ int layout_slot(const NewLayout& nl, int nv, int G, int z, int rank) {
   const int base = nl.goff[G];
-  if (rank < nl.level[G]) return base + rank * kLanes + l;
+  const int n = lanes_of(nv, z), row = rank / n;
+  if (row < nl.level[G]) return base + row * kLanes + z + (rank - row * n) * nv;
   const int q = atomicAdd(nl.gcursor + G, 1);
   const int2* f = nl.free + G * kLanes;
   int b = 0;  // the last lane whose strangers start at or before number q: it has free slots
@@ -258,7 +289,9 @@ __global__ void tiled_scatter_kernel(Parts<real> P, Geom g, TileGeom t, const in
   const int G = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (G >= t.ngroups) return;
-  const int home = home_key(g, t, G, lane);
+  LaneCell lc;
+  int home = home_key(g, t, G, lane, lc);
+  if (lc.n > 1) home = -1;  // as in tiled_count_kernel
   const int base = goff_old[G], m = gmax_old[G];
   int rnew = 0;
   constexpr int U = 4;  // rows whose loads are in flight together
@@ -282,12 +315,12 @@ __global__ void tiled_scatter_kernel(Parts<real> P, Geom g, TileGeom t, const in
       if (key < 0) continue;
       int d;
       if (key == home) {
-        d = layout_slot(nl, G, lane, rnew);
+        d = layout_slot(nl, kLanes, G, lane, rnew);  // a cell of one lane
         ++rnew;
       } else {
         int l2;
         const int G2 = group_of_key(g, t, key, l2);
-        d = layout_slot(nl, G2, l2, nl.stay[key] + atomicAdd(nl.cursor + key, 1));
+        d = layout_slot(nl, cells_of_group(g, t, G2), G2, l2, nl.stay[key] + atomicAdd(nl.cursor + key, 1));
       }
       Q.cell[d] = cell[u];
 #pragma unroll
@@ -309,7 +342,8 @@ __global__ void append_scatter_kernel(Parts<real> P, int first, const int* __res
     if (key < 0) continue;
     int l2;
     const int G2 = group_of_key(g, t, key, l2);
-    copy_particle(P, s, Q, layout_slot(nl, G2, l2, nl.stay[key] + atomicAdd(nl.cursor + key, 1)), c);
+    copy_particle(P, s, Q, layout_slot(nl, cells_of_group(g, t, G2), G2, l2, nl.stay[key] + atomicAdd(nl.cursor + key, 1)),
+                  c);
   }
 }
 
@@ -323,104 +357,80 @@ __device__ __forceinline__ void red_add_v4(float* p, float a, float b, float c, 
                :: "l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 
-// Window deposit of the 2x2x2 stencil at global base node (a, b, c); falls
-// back to global atomics when the stencil leaves the window.
-template <typename real>
-__device__ __forceinline__ void scatter8_win(real* win, int wx0, int wy0, int wz0, real* gplane,
-                                             const Geom& g, int a, int b, int c, real v, real x0,
-                                             real x1, real y0, real y1, real z0, real z1) {
-  constexpr int WY = kTileY + 4, WZ = kWinZ, WX = kTileX + 4;
-  const int la = a - wx0, lb = b - wy0, lc = c - wz0;
-  if (la >= 0 && la <= WX - 2 && lb >= 0 && lb <= WY - 2 && lc >= 0 && lc <= WZ - 2) {
-    const int s = (la * WY + lb) * WZ + lc;
-    const real a0 = v * x0, a1 = v * x1;
-    const real a00 = a0 * y0, a01 = a0 * y1, a10 = a1 * y0, a11 = a1 * y1;
-    atomicAdd(win + s, a00 * z0);
-    atomicAdd(win + s + 1, a00 * z1);
-    atomicAdd(win + s + WZ, a01 * z0);
-    atomicAdd(win + s + WZ + 1, a01 * z1);
-    atomicAdd(win + s + WY * WZ, a10 * z0);
-    atomicAdd(win + s + WY * WZ + 1, a10 * z1);
-    atomicAdd(win + s + WY * WZ + WZ, a11 * z0);
-    atomicAdd(win + s + WY * WZ + WZ + 1, a11 * z1);
-  } else {
-    scatter8(gplane, a * g.sx + b * g.gz + c, g.sx, g.gz, v, x0, x1, y0, y1, z0, z1);
-  }
-}
-
-// Density deposit into a fixed-point window: the 2x2x2 area weights (each in
-// [0, 1], summing to 1) scaled by `scale` and rounded, added with integer
-// shared-memory reductions, which need no compare-and-swap loop and give a sum
-// that does not depend on the order of the particles. The caller picks `scale`
-// so that no node can overflow: a node collects at most one unit of weight from
-// each particle of the tile, so scale = (2^32 - 1) / (slots + 1) is safe; it is
-// also kept below 2^23 for the rounding below. With 64 particles per cell this
-// resolves 2^-17.7 of a particle's weight, as fine as an FP32 sum of the same
-// node. The stencil falls back to FP32 global
-// atomics (weight v) when it leaves the window.
+// Density deposit into the window at node s, the base of the particle's 2x2x2
+// stencil (X, Y, Z hold the half-shifted weights). FP64 adds the weight. FP32
+// sums in fixed point: the 2x2x2 area weights (each in [0, 1], summing to 1)
+// scaled by `scale` and rounded, added with integer shared-memory reductions,
+// which need no compare-and-swap loop and give a sum that does not depend on
+// the order of the particles. The caller picks `scale` so that no node can
+// overflow: a node collects at most one unit of weight from each particle of
+// the tile, so scale = (2^32 - 1) / (slots + 1) is safe; it is also kept below
+// 2^23 for the rounding below. With 64 particles per cell this resolves
+// 2^-17.7 of a particle's weight, as fine as an FP32 sum of the same node.
 __device__ __forceinline__ void red_shared_u32(const unsigned* p, unsigned v) {
   asm volatile("red.shared.add.u32 [%0], %1;" :: "r"((unsigned)__cvta_generic_to_shared(p)), "r"(v) : "memory");
 }
-
-__device__ __forceinline__ void scatter8_win_fixed(unsigned* win, int wx0, int wy0, int wz0, float* gplane,
-                                                   const Geom& g, int a, int b, int c, float v, float scale,
-                                                   float x0, float x1, float y0, float y1, float z0, float z1) {
-  constexpr int WY = kTileY + 4, WZ = kWinZ, WX = kTileX + 4;
-  const int la = a - wx0, lb = b - wy0, lc = c - wz0;
-  if (la >= 0 && la <= WX - 2 && lb >= 0 && lb <= WY - 2 && lc >= 0 && lc <= WZ - 2) {
-    const unsigned* s = win + (la * WY + lb) * WZ + lc;
-    // the eight node weights (each in [0, scale], scale < 2^23) rounded to
-    // integers by adding 2^23 in the FMA: the sum's low mantissa bits are then
-    // the rounded weight, with no float-to-integer conversion; the two x
-    // planes travel as one packed pair
-    constexpr float kM = 8388608.f;                 // 2^23
-    constexpr unsigned kMBits = 0x4B000000u;        // its bit pattern
-    const float2 M = make_float2(kM, kM);
-    const float2 ax = __fmul2_rn(make_float2(x0, x1), make_float2(scale, scale));
-    const float2 ay0 = __fmul2_rn(ax, make_float2(y0, y0));  // (a00, a10)
-    const float2 ay1 = __fmul2_rn(ax, make_float2(y1, y1));  // (a01, a11)
-    const float2 Z0 = make_float2(z0, z0), Z1 = make_float2(z1, z1);
-    const float2 t00 = __ffma2_rn(ay0, Z0, M), t01 = __ffma2_rn(ay0, Z1, M);
-    const float2 t10 = __ffma2_rn(ay1, Z0, M), t11 = __ffma2_rn(ay1, Z1, M);
-    red_shared_u32(s, __float_as_uint(t00.x) - kMBits);
-    red_shared_u32(s + 1, __float_as_uint(t01.x) - kMBits);
-    red_shared_u32(s + WZ, __float_as_uint(t10.x) - kMBits);
-    red_shared_u32(s + WZ + 1, __float_as_uint(t11.x) - kMBits);
-    red_shared_u32(s + WY * WZ, __float_as_uint(t00.y) - kMBits);
-    red_shared_u32(s + WY * WZ + 1, __float_as_uint(t01.y) - kMBits);
-    red_shared_u32(s + WY * WZ + WZ, __float_as_uint(t10.y) - kMBits);
-    red_shared_u32(s + WY * WZ + WZ + 1, __float_as_uint(t11.y) - kMBits);
-  } else {
-    scatter8(gplane, a * g.sx + b * g.gz + c, g.sx, g.gz, v, x0, x1, y0, y1, z0, z1);
-  }
+template <int WY, int WZ, typename W>
+__device__ __forceinline__ void add_density(float* win, float scale, const W& X, const W& Y, const W& Z) {
+  // the eight node weights rounded to integers by adding 2^23 in the FMA: the
+  // sum's low mantissa bits are then the rounded weight, with no
+  // float-to-integer conversion; the two x planes travel as one packed pair
+  const unsigned* s = reinterpret_cast<const unsigned*>(win);
+  constexpr float kM = 8388608.f;       // 2^23
+  constexpr unsigned kMBits = 0x4B000000u;  // its bit pattern
+  const float2 M = make_float2(kM, kM);
+  const float2 ax = __fmul2_rn(make_float2(X.b0, X.b1), make_float2(scale, scale));
+  const float2 ay0 = __fmul2_rn(ax, make_float2(Y.b0, Y.b0));  // (a00, a10)
+  const float2 ay1 = __fmul2_rn(ax, make_float2(Y.b1, Y.b1));  // (a01, a11)
+  const float2 Z0 = make_float2(Z.b0, Z.b0), Z1 = make_float2(Z.b1, Z.b1);
+  const float2 t00 = __ffma2_rn(ay0, Z0, M), t01 = __ffma2_rn(ay0, Z1, M);
+  const float2 t10 = __ffma2_rn(ay1, Z0, M), t11 = __ffma2_rn(ay1, Z1, M);
+  red_shared_u32(s, __float_as_uint(t00.x) - kMBits);
+  red_shared_u32(s + 1, __float_as_uint(t01.x) - kMBits);
+  red_shared_u32(s + WZ, __float_as_uint(t10.x) - kMBits);
+  red_shared_u32(s + WZ + 1, __float_as_uint(t11.x) - kMBits);
+  red_shared_u32(s + WY * WZ, __float_as_uint(t00.y) - kMBits);
+  red_shared_u32(s + WY * WZ + 1, __float_as_uint(t01.y) - kMBits);
+  red_shared_u32(s + WY * WZ + WZ, __float_as_uint(t10.y) - kMBits);
+  red_shared_u32(s + WY * WZ + WZ + 1, __float_as_uint(t11.y) - kMBits);
+}
+template <int WY, int WZ, typename W>
+__device__ __forceinline__ void add_density(double* s, double weight, const W& X, const W& Y, const W& Z) {
+  const double a0 = weight * X.b0, a1 = weight * X.b1;
+  const double a00 = a0 * Y.b0, a01 = a0 * Y.b1, a10 = a1 * Y.b0, a11 = a1 * Y.b1;
+  atomicAdd(s, a00 * Z.b0);
+  atomicAdd(s + 1, a00 * Z.b1);
+  atomicAdd(s + WZ, a01 * Z.b0);
+  atomicAdd(s + WZ + 1, a01 * Z.b1);
+  atomicAdd(s + WY * WZ, a10 * Z.b0);
+  atomicAdd(s + WY * WZ + 1, a10 * Z.b1);
+  atomicAdd(s + WY * WZ + WZ, a11 * Z.b0);
+  atomicAdd(s + WY * WZ + WZ + 1, a11 * Z.b1);
 }
 
-// Half-shifted weights of a particle in its home cell h as a 3-vector over the
-// nodes h-1, h, h+1 (its base is h-1 for an offset below 1/2, h otherwise).
+// Half-shifted weights of a particle at offset f of its home cell h (an
+// interior cell) as a 3-vector over the nodes h-1, h, h+1: with g = f - 1/2
+// they are (max(-g, 0), 1 - |g|, max(g, 0)).
 template <typename real>
 struct W3 {
   real w[3];
 };
-template <typename real>
-__device__ __forceinline__ W3<real> home3(const Axis<real>& A, int h) {
-  W3<real> r;
-  const bool up = A.b == h;
-  r.w[0] = up ? (real)0 : A.b0;
-  r.w[1] = up ? A.b0 : A.b1;
-  r.w[2] = up ? A.b1 : (real)0;
-  return r;
-}
-// FP32: the same three weights straight from the offset f = A.a1 of a
-// particle in its home cell (an interior cell, so never cell 0): with
-// g = f - 1/2 they are (max(-g, 0), 1 - |g|, max(g, 0)), equal to the form
-// above to within a rounding, in four instructions instead of the base
-// choice and three selects.
-__device__ __forceinline__ W3<float> home3(const Axis<float>& A, int) {
-  const float g = A.a1 - 0.5f;
+__device__ __forceinline__ W3<float> home3(float f) {
+  const float g = f - 0.5f;
   W3<float> r;
   r.w[0] = fmaxf(-g, 0.f);
   r.w[1] = 1.f - fabsf(g);
   r.w[2] = fmaxf(g, 0.f);
+  return r;
+}
+// FP64: the same from the reference's base and weights, rounded as it rounds.
+__device__ __forceinline__ W3<double> home3(double f) {
+  const bool up = f >= 0.5;
+  const double b1 = up ? f - 0.5 : f + 0.5, b0 = 1.0 - b1;
+  W3<double> r;
+  r.w[0] = up ? 0.0 : b0;
+  r.w[1] = up ? b0 : b1;
+  r.w[2] = up ? b1 : 0.0;
   return r;
 }
 

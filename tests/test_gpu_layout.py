@@ -62,3 +62,43 @@ def test_layout_keeps_particles_and_their_sums(n, speed, precision):
             if precision == 64:
                 assert rel_norm(ordered(np.round(a, 9)), ordered(np.round(b, 9))) < 1e-8
         assert T.status()[0] == 0
+
+
+@pytest.mark.parametrize("case", ["long moves", "ballistic at 3 c", "ballistic at 9 c", "wraps"])
+def test_particles_off_the_short_path(case):
+    """Moves of a cell and more per half step, ballistic particles that Boris
+    has not slowed, and more particles wrapped round the x faces than a warp's
+    list holds: the tiled push hands them to the general one (FP64; a step
+    rounds a value a few times, so 1e-11 covers three)."""
+    n = (12, 9, 40)
+    kw = {"long moves": dict(dt=2.5), "wraps": {}}.get(case, dict(absorb_grid2=5))
+    speed = {"ballistic at 3 c": 3.0, "ballistic at 9 c": 9.0, "wraps": 0.95}.get(case, 0.3)
+    rng = np.random.default_rng(len(case))
+    xyz = 2 + rng.random((6000, 3)) * np.array(n)
+    if case == "wraps":
+        xyz[:, 0] = n[0] + 1 + rng.random(6000)
+        xyz[:, 1] = 3 + rng.random(6000)
+    v = rng.normal(0, 0.1 * speed, xyz.shape) + [0.9 * speed, 0, 0.1]
+    if case == "wraps":
+        v[:] = [0.94, 0, 0.05]
+    rows = np.column_stack([xyz, v, np.full(len(xyz), 0.01 / 4)])
+    P = []
+    for slot_order in (0, 1):
+        P.append(Pic3D(PicConfig.normalized(*n, 4, precision=64, diag_every_step=0, sort_interval=1000,
+                                            add_interval=1000, slot_order=slot_order, capacity=200000, **kw)))
+        P[-1].init_grid()
+        for s in (ION, ELECTRON):
+            P[-1].set_particles(s, rows)
+    for _ in range(3 if case != "wraps" else 8):
+        for p in P:
+            p.step(1)
+        g, h = P[0].grid(), P[1].grid()
+        for q in range(18):
+            assert rel_norm(g[..., q], h[..., q]) < 1e-11 or np.abs(g[..., q] - h[..., q]).max() < 1e-15
+    for s in (ION, ELECTRON):
+        a, b = P[0].particles(s), P[1].particles(s)
+        assert len(a) == len(b) and rel_norm(ordered(np.round(a, 8)), ordered(np.round(b, 8))) < 1e-7
+    (ra, ca), (rb, cb) = P[0].status(), P[1].status()
+    assert ra == rb and np.array_equal(ca, cb)
+    for p in P:
+        p.close()
