@@ -208,7 +208,7 @@ int adj_compact(pic_ctx* c, AdjRun& R, int s, int* map) {
                                                                         R.sslot[0], parts<real>(c, s, 1 - st.cur),
                                                                         map, st.count_dev);
   CKL();
-  CK(cudaMemcpyAsync(c->host_pin + 2 + s, st.count_dev, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaMemcpyAsync(c->host_pin + 4 + s, st.count_dev, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaEventRecord(st.readback, c->stream));
   st.cur = 1 - st.cur;
   c->tiled[s] = false;
@@ -248,7 +248,7 @@ int adj_resolve(pic_ctx* c, AdjRun& R, AdjSnap* rec) {
     Store& st = c->sp[s];
     CK(cudaEventSynchronize(st.readback));
     R.pend[s] = false;
-    const long long kept = c->host_pin[2 + s];  // read back before the appends
+    const long long kept = c->host_pin[4 + s];  // read back before the appends
     st.count = kept + R.pend_added[s];
     if (rec) {
       rec->kept[s] = kept;

@@ -9,6 +9,7 @@
 #include <map>
 #include <new>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include <cudaTypedefs.h>
@@ -50,7 +51,8 @@ struct Store {
   cudaEvent_t readback = nullptr;
   int* holes = nullptr;   // per-slot scratch: hole rows of every lane column
   int* nholes = nullptr;  // per lane of every group: holes of its column
-  int* nonhome = nullptr; // a particle outside its home cell stayed in the layout
+  int* nspill = nullptr;  // a placement's particles without a hole
+  int* nonhome = nullptr; // a particle outside its home cell stayed in the layout (after nspill)
   // a refill's shell deletion over the layout is left to the next classify pass
   bool shell_pending = false;
 };
@@ -125,7 +127,8 @@ struct pic_ctx {
   int mig_cap = 0;
   unsigned long long* err = nullptr;  // ERR_COUNT
   DevPool adj_pool;                   // the adjoint's work and snapshot memory
-  int* host_pin = nullptr;            // pinned read-back slots: per species the spill count, the non-home flag
+  int* host_pin = nullptr;            // pinned read-back slots: per species the spill count and the non-home flag
+                                      // (0 to 3), the adjoint's counts (4, 5)
   // import/export staging
   void* stage = nullptr;
   size_t stage_bytes = 0;
@@ -204,6 +207,24 @@ int particle_blocks(long long n) {
   if (b > cap) b = cap;
   if (b < 1) b = 1;
   return (int)b;
+}
+
+// Launches k on the context's stream so that it may start while the kernel
+// before it is still running (after_prior in common.cuh, which every kernel
+// launched here calls first).
+template <typename... K, typename... A>
+cudaError_t launch_after(const pic_ctx* c, void (*k)(K...), long long grid, int block, size_t smem, A&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c->stream;
+  cudaLaunchAttribute early{};
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &early;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
 }
 
 __global__ void set_int_kernel(int* p, int v) { *p = v; }
@@ -571,12 +592,13 @@ int do_renew_b(pic_ctx* c, int ride = RIDE_NONE) {
     constexpr int TX = StShape<real>::TX, TY = StShape<real>::TY;
     const int ty = (c->g.ny + TY - 1) / TY, tz = (c->g.nz + kStZ - 1) / kStZ, tx = (c->g.nx + TX - 1) / TX;
     rider.first = tx * ty * tz;
-    renew_b_tma_kernel<real, TX, TY><<<tx * ty * tz + extra, kStThreads, StTile<real>::bytes, c->stream>>>(
-        c->tm_e[0], c->tm_e[1], c->tm_e[2], fields<real>(c), c->g, ramps(c), p, ty, tz, ghosts, rider, c->err);
+    CK(launch_after(c, renew_b_tma_kernel<real, TX, TY>, tx * ty * tz + extra, kStThreads, StTile<real>::bytes,
+                    c->tm_e[0], c->tm_e[1], c->tm_e[2], fields<real>(c), c->g, ramps(c), p, ty, tz, ghosts, rider,
+                    c->err));
   } else {
     rider.first = grid_blocks((long long)c->g.nx * c->g.ny * c->g.nz);
-    renew_b_kernel<real><<<rider.first + extra, kThreads, 0, c->stream>>>(fields<real>(c), c->g, ramps(c), p, ghosts,
-                                                                         rider);
+    CK(launch_after(c, renew_b_kernel<real>, rider.first + extra, kThreads, 0, fields<real>(c), c->g, ramps(c), p,
+                    ghosts, rider));
   }
   CKL();
   if (c->has_xport) {
@@ -601,11 +623,12 @@ int do_renew_e(pic_ctx* c) {
   if (c->staged) {
     constexpr int TX = StShape<real>::TX, TY = StShape<real>::TY;
     const int ty = (c->g.ny + TY - 1) / TY, tz = (c->g.nz + kStZ - 1) / kStZ, tx = (c->g.nx + TX - 1) / TX;
-    renew_e_tma_kernel<real, TX, TY><<<tx * ty * tz, kStThreads, StTile<real>::bytes, c->stream>>>(
-        c->tm_db[0], c->tm_db[1], c->tm_db[2], fields<real>(c), c->g, ramps(c), p, ty, tz, ghosts, c->err);
+    CK(launch_after(c, renew_e_tma_kernel<real, TX, TY>, tx * ty * tz, kStThreads, StTile<real>::bytes, c->tm_db[0],
+                    c->tm_db[1], c->tm_db[2], fields<real>(c), c->g, ramps(c), p, ty, tz, ghosts, c->err));
   } else {
     const long long nint = (long long)c->g.nx * c->g.ny * c->g.nz;
-    renew_e_kernel<real><<<grid_blocks(nint), kThreads, 0, c->stream>>>(fields<real>(c), c->g, ramps(c), p, ghosts);
+    CK(launch_after(c, renew_e_kernel<real>, grid_blocks(nint), kThreads, 0, fields<real>(c), c->g, ramps(c), p,
+                    ghosts));
   }
   CKL();
   static const int ids[3] = {F_EX, F_EY, F_EZ};
@@ -736,8 +759,6 @@ int do_push(pic_ctx* c, int s, long long first = 0) {
   return PIC_OK;
 }
 
-__global__ void copy_int_kernel(int* dst, const int* src) { *dst = *src; }
-
 // The push of species s. `overlap`: the launch just before on the stream is the
 // other species' tiled push, which this one may run beside (push_tiled.cuh).
 template <typename real>
@@ -747,23 +768,11 @@ int do_push_tiled(pic_ctx* c, int s, bool overlap = false) {
   // a CTA per SM for the tail, whose length only the device may know
   const long long tail = slot_bound(c, s) - c->tiled_end[s];
   const int ntail = (int)std::min<long long>((std::max<long long>(tail, 0) + kThreads - 1) / kThreads, 148);
-  const TileArgs ta{c->tg, c->goff[s][c->lay[s]], c->gtop[s], ntail, (int)c->tiled_end[s], c->sp[s].count_dev};
+  const TileArgs ta{c->tg, c->goff[s][c->lay[s]], c->gtop[s], ntail, (int)c->tiled_end[s], c->sp[s].count_dev, overlap};
   const bool vec = c->g.gz * sizeof(real) % 16 == 0;
-  cudaLaunchConfig_t k{};
-  k.gridDim = dim3(ntail + ntiles);
-  k.blockDim = dim3(kTileX * kTileY * 32);
-  k.dynamicSmemBytes = PushSmem<real>::bytes;
-  k.stream = c->stream;
-  cudaLaunchAttribute early{};
-  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  early.val.programmaticStreamSerializationAllowed = 1;
-  k.attrs = &early;
-  k.numAttrs = overlap ? 1 : 0;
-  const Parts<real> P = parts<real>(c, s);
-  const Fields<real> F = fields<real>(c);
-  const PushConst<real> pc = push_const<real>(c, s);
-  CK(vec ? cudaLaunchKernelEx(&k, push_tiled_kernel<real, true>, P, ta, F, c->g, pc, c->err)
-         : cudaLaunchKernelEx(&k, push_tiled_kernel<real, false>, P, ta, F, c->g, pc, c->err));
+  CK(launch_after(c, vec ? push_tiled_kernel<real, true> : push_tiled_kernel<real, false>, ntail + ntiles,
+                  kTileX * kTileY * 32, PushSmem<real>::bytes, parts<real>(c, s), ta, fields<real>(c), c->g,
+                  push_const<real>(c, s), c->err));
   CKL();
   return PIC_OK;
 }
@@ -794,11 +803,11 @@ int do_sr_particle(pic_ctx* c) {
 int scan_exclusive(pic_ctx* c, const int* in, int* out, long long n, int* tmp, size_t tmp_len) {
   const long long tiles = (n + kScanTile - 1) / kScanTile;
   if ((size_t)tiles + 1 > tmp_len) return PIC_ERR_STATE;
-  scan_tile_kernel<<<(unsigned)tiles, kScanThreads, 0, c->stream>>>(in, out, tmp, n);
+  CK(launch_after(c, scan_tile_kernel, tiles, kScanThreads, 0, in, out, tmp, n));
   CKL();
   if (tiles > 1) {
     CKR(scan_exclusive(c, tmp, tmp, tiles, tmp + tiles + 1, tmp_len - (size_t)tiles - 1));
-    scan_add_kernel<<<(unsigned)tiles, 256, 0, c->stream>>>(out, tmp, n);
+    CK(launch_after(c, scan_add_kernel, tiles, 256, 0, out, tmp, n));
     CKL();
   }
   return PIC_OK;
@@ -882,8 +891,6 @@ int do_sort_species(pic_ctx* c, int s) {
 // spill count back into pinned memory without waiting; check_spill acts on
 // that read-back when it has landed (a full sort when many particles found no
 // hole), sync_count reads the count itself when the host needs it.
-__global__ void spill_count_kernel(int* count, int first, const int* nspill) { *count = first + *nspill; }
-
 // The placement of the particles in [tiled_end, *count_dev) into the holes
 // that st.holes / st.nholes list (place_launch).
 template <typename real>
@@ -894,26 +901,23 @@ int place_launch(pic_ctx* c, int s) {
   const Parts<real> P = parts<real>(c, s);
   const long long first = c->tiled_end[s];
   const Parts<real> Q = parts<real>(c, s, 1 - st.cur);
-  CK(cudaMemsetAsync(c->cursor, 0, sizeof(int) * c->ncells, c->stream));
-  CK(cudaMemsetAsync(c->total_dev, 0, sizeof(int), c->stream));  // spill count
-  place_count_kernel<real><<<particle_blocks(st.cap - first), kThreads, 0, c->stream>>>(
-      P, (int)first, st.count_dev, c->g, c->cursor, c->rank);
+  const int pblocks = particle_blocks(st.cap - first);
+  CK(launch_after(c, place_count_kernel<real>, pblocks, kThreads, 0, P, (int)first, c->append_dev, (int)st.cap, c->g,
+                  c->cursor, c->rank));
   CKL();
   int* off = c->offs;  // per cell: bucket offset of its arrivals
   CKR(scan_exclusive(c, c->cursor, off, c->ncells, c->scan_tmp, c->scan_tmp_len));
-  place_bucket_kernel<real><<<particle_blocks(st.cap - first), kThreads, 0, c->stream>>>(
-      P, (int)first, st.count_dev, c->g, off, c->rank, c->bucket);
+  CK(launch_after(c, place_bucket_kernel<real>, pblocks, kThreads, 0, P, (int)first, c->append_dev, (int)st.cap, c->g,
+                  off, c->rank, c->bucket));
   CKL();
-  place_fill_kernel<real><<<gblocks, kThreads, 0, c->stream>>>(
-      P, (int)first, c->g, tg, c->goff[s][c->lay[s]], c->gmax[s][c->lay[s]], c->gtop[s], st.holes, c->cursor,
-      st.nholes, off, c->bucket, c->total_dev, Q);
+  CK(launch_after(c, place_fill_kernel<real>, gblocks, kThreads, 0, P, (int)first, c->g, tg, c->goff[s][c->lay[s]],
+                  c->gmax[s][c->lay[s]], c->gtop[s], st.holes, c->cursor, st.nholes, off, c->bucket, st.nspill, Q));
   CKL();
-  unspill_kernel<real><<<particle_blocks(st.cap), kThreads, 0, c->stream>>>(Q, c->total_dev, P, (int)first);
+  CK(launch_after(c, unspill_kernel<real>, particle_blocks(st.cap), kThreads, 0, Q, st.nspill, P, (int)first,
+                  st.count_dev));
   CKL();
-  spill_count_kernel<<<1, 1, 0, c->stream>>>(st.count_dev, (int)first, c->total_dev);
-  CKL();
-  CK(cudaMemcpyAsync(c->host_pin + s, c->total_dev, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaMemcpyAsync(c->host_pin + 2 + s, st.nonhome, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  // the spill count and the non-home flag, side by side
+  CK(cudaMemcpyAsync(c->host_pin + 2 * s, st.nspill, 2 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaEventRecord(st.readback, c->stream));
   st.pending = true;
   st.spill_pending = true;
@@ -928,17 +932,14 @@ int relayout_launch(pic_ctx* c, int s) {
   const TileGeom& tg = c->tg;
   const int gblocks = grid_blocks((long long)tg.ngroups * 32);
   const Parts<real> P = parts<real>(c, s);
-  CK(cudaMemsetAsync(st.nonhome, 0, sizeof(int), c->stream));
-  copy_int_kernel<<<1, 1, 0, c->stream>>>(c->append_dev, st.count_dev);
+  CK(launch_after(c, relayout_begin_kernel, particle_blocks(c->ncells / 8), kThreads, 0, st.count_dev, c->append_dev,
+                  st.nspill, st.nonhome, c->cursor, c->ncells));
   CKL();
-  classify_kernel<real><<<gblocks, kThreads, 0, c->stream>>>(P, c->g, tg, c->goff[s][c->lay[s]],
-                                                             c->gmax[s][c->lay[s]], c->gtop[s], (int)st.cap, st.holes,
-                                                             st.nholes, c->append_dev, st.nonhome,
-                                                             st.shell_pending ? 1 : 0);
+  CK(launch_after(c, classify_kernel<real>, gblocks, kThreads, 0, P, c->g, tg, c->goff[s][c->lay[s]],
+                  c->gmax[s][c->lay[s]], c->gtop[s], (int)st.cap, st.holes, st.nholes, c->append_dev, st.nonhome,
+                  st.shell_pending ? 1 : 0));
   CKL();
   st.shell_pending = false;
-  clamp_count_kernel<<<1, 1, 0, c->stream>>>(c->append_dev, (int)st.cap, st.count_dev);
-  CKL();
   return place_launch<real>(c, s);
 }
 
@@ -974,7 +975,7 @@ int check_spill(pic_ctx* c, int s, bool wait) {
   }
   st.spill_pending = false;
   const long long first = c->tiled_end[s];
-  if (c->host_pin[s] > first / 50 || c->host_pin[2 + s]) {
+  if (c->host_pin[2 * s] > first / 50 || c->host_pin[2 * s + 1]) {
     CKR(sync_count(c, s));
     return do_sort_species<real>(c, s);
   }
@@ -1077,6 +1078,7 @@ int do_source(pic_ctx* c, int s, const Slab* slabs, int nslab, int init_form = 0
 }
 
 __global__ void grow_count_kernel(int* count, long long add, int cap) {
+  after_prior();
   const long long n = (long long)*count + add;
   *count = (int)(n < cap ? n : (long long)cap);
 }
@@ -1093,9 +1095,9 @@ int do_source_dev(pic_ctx* c, int s, const Slab* slabs, int nslab) {
   Store& st = c->sp[s];
   sp.dst_dev = st.count_dev;
   sp.cap = (int)st.cap;
-  source_kernel<real><<<grid_blocks(total), kThreads, 0, c->stream>>>(parts<real>(c, s), sp, c->err);
+  CK(launch_after(c, source_kernel<real>, grid_blocks(total), kThreads, 0, parts<real>(c, s), sp, c->err));
   CKL();
-  grow_count_kernel<<<1, 1, 0, c->stream>>>(st.count_dev, total, (int)st.cap);
+  CK(launch_after(c, grow_count_kernel, 1, 1, 0, st.count_dev, total, (int)st.cap));
   CKL();
   c->ctr_p += 3 * total;
   c->ctr_v += 6 * total;
@@ -1126,8 +1128,8 @@ int do_add_flat(pic_ctx* c, bool fused = false) {
     }
     const long long first = defer ? c->tiled_end[s] : 0;
     if (nowait || st.count > first) {
-      delete_shell_kernel<real><<<particle_blocks((nowait ? st.cap : st.count) - first), kThreads, 0, c->stream>>>(
-          P, (int)first, st.count_dev, c->g);
+      CK(launch_after(c, delete_shell_kernel<real>, particle_blocks((nowait ? st.cap : st.count) - first), kThreads, 0,
+                      P, (int)first, st.count_dev, c->g));
       CKL();
     }
     if (defer) {
@@ -1265,7 +1267,7 @@ int do_thrust_sums(pic_ctx* c, bool mean = false) {
   a.nfar = (int)std::min<long long>(far, 148 * 2);
   const int nodes = (int)std::min<long long>(grid_blocks((long long)k.nx * k.ny * k.nz), 148);
   const size_t smem = sizeof(real) == 4 ? 6 * ThrustPlan::WN * sizeof(float) : 0;
-  thrust_kernel<real><<<a.sp[0].near + a.sp[1].near + 2 * a.nfar + nodes, kThreads, smem, c->stream>>>(a);
+  CK(launch_after(c, thrust_kernel<real>, a.sp[0].near + a.sp[1].near + 2 * a.nfar + nodes, kThreads, smem, a));
   CKL();
   if (!c->has_xport) return PIC_OK;
   // thrust_f's MPI_Allreduce of F and E over the ranks (:5103-5108)
@@ -1801,8 +1803,9 @@ int pic_create(const pic_config* cfg, pic_ctx** out) {
       for (int s = 0; s < 2; ++s) {  // each species' hole lists live from its push to its next placement
         if (cudaMalloc(&c->sp[s].holes, sizeof(int) * (size_t)cap) != cudaSuccess) return fail(PIC_ERR_CUDA);
         if (cudaMalloc(&c->sp[s].nholes, sizeof(int) * kLanes * t.ngroups) != cudaSuccess) return fail(PIC_ERR_CUDA);
-        if (cudaMalloc(&c->sp[s].nonhome, sizeof(int)) != cudaSuccess) return fail(PIC_ERR_CUDA);
-        cudaMemsetAsync(c->sp[s].nonhome, 0, sizeof(int), c->stream);
+        if (cudaMalloc(&c->sp[s].nspill, 2 * sizeof(int)) != cudaSuccess) return fail(PIC_ERR_CUDA);
+        c->sp[s].nonhome = c->sp[s].nspill + 1;
+        cudaMemsetAsync(c->sp[s].nspill, 0, 2 * sizeof(int), c->stream);
       }
       if (cudaMalloc(&c->rank, sizeof(int) * (size_t)cap) != cudaSuccess) return fail(PIC_ERR_CUDA);
       if (cudaMalloc(&c->bucket, sizeof(int) * (size_t)cap) != cudaSuccess) return fail(PIC_ERR_CUDA);
@@ -1858,7 +1861,7 @@ int pic_destroy(pic_ctx* c) {
   for (int s = 0; s < 2; ++s) {
     cudaFree(c->sp[s].holes);
     cudaFree(c->sp[s].nholes);
-    cudaFree(c->sp[s].nonhome);
+    cudaFree(c->sp[s].nspill);
   }
   cudaFree(c->rank);
   cudaFree(c->bucket);

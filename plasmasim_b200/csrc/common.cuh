@@ -31,6 +31,26 @@ __host__ __device__ __forceinline__ void unpack_cell(int c, int& i, int& j, int&
   k = c & kCellMask;
 }
 
+// Programmatic dependent launch. A kernel launched with launch_after (api.cu)
+// may start while the one before it on the stream is still running, once all
+// of that one's CTAs have called after_prior; its own call then waits until
+// the earlier kernel has ended and its writes can be seen. Every thread of
+// every such kernel calls after_prior before it touches memory, so that a
+// kernel's end still implies that of all before it. (What such a kernel loads
+// in the same breath is not marked __restrict__, so that no load can be taken
+// for one of constant memory and moved ahead of the wait.) It saves the gap
+// between two kernels (with a re-layout's clears and counts folded into its
+// passes: 0.144 -> 0.141 ms per step at 32^3 x 8, 0.306 -> 0.288 at 41 x 22 x 70
+// x 30, the re-layout 0.035 -> 0.025 and 0.084 -> 0.074 of it).
+#ifdef __CUDACC__
+__device__ __forceinline__ void wait_prior() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void after_prior() {
+  wait_prior();
+  release_next();
+}
+#endif
+
 struct Geom {
   int nx, ny, nz;   // interior cells
   int gx, gy, gz;   // padded extents (n + 4)

@@ -175,6 +175,7 @@ __device__ __forceinline__ Rec<double> load_record_a(const Parts<double>& P, int
 // counter: 0.099, 0.034, 0.316.)
 template <typename real>
 __global__ void __launch_bounds__(256, 3) thrust_kernel(const __grid_constant__ ThrustArgs<real> a) {
+  after_prior();
   using S = ThrustPlan;
   constexpr int U = sizeof(real) == 4 ? 4 : 2;
   constexpr bool kWin = sizeof(real) == 4;

@@ -245,6 +245,7 @@ __device__ __forceinline__ void e_coeffs(double s, const EParams& p, double& ca,
 template <typename real>
 __global__ void __launch_bounds__(256) renew_b_kernel(Fields<real> F, Geom g, Ramps rp, BParams p, bool ghosts,
                                                       Rider<real> rider) {
+  after_prior();
   if (rider.mode && (int)blockIdx.x >= rider.first) return ride(rider, g);
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int nint = g.nx * g.ny * g.nz;
@@ -300,6 +301,7 @@ __global__ void __launch_bounds__(256) renew_b_kernel(Fields<real> F, Geom g, Ra
 // ca = (1 - mu0 s t/2)/(1 + mu0 s t/2), cb = t/(1 + mu0 s t/2), t = c^2 dt.
 template <typename real>
 __global__ void __launch_bounds__(256) renew_e_kernel(Fields<real> F, Geom g, Ramps rp, EParams p, bool ghosts) {
+  after_prior();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int nint = g.nx * g.ny * g.nz;
   if (t >= nint) return;

@@ -161,6 +161,7 @@ __global__ void __launch_bounds__(kStThreads, sizeof(real) == 4 ? 3 : 2)
                        const __grid_constant__ CUtensorMap tez, Fields<real> F, Geom g, Ramps rp, BParams p,
                        int tiles_y, int tiles_z, bool ghosts, const __grid_constant__ Rider<real> rider,
                        unsigned long long* err) {
+  after_prior();
   using T = StencilTile<real, TX, TY>;
   if (rider.mode && (int)blockIdx.x >= rider.first) return ride(rider, g);
   extern __shared__ __align__(128) unsigned char fsm[];
@@ -282,6 +283,7 @@ __global__ void __launch_bounds__(kStThreads, sizeof(real) == 4 ? 3 : 2)
     renew_e_tma_kernel(const __grid_constant__ CUtensorMap tbx, const __grid_constant__ CUtensorMap tby,
                        const __grid_constant__ CUtensorMap tbz, Fields<real> F, Geom g, Ramps rp, EParams p,
                        int tiles_y, int tiles_z, bool ghosts, unsigned long long* err) {
+  after_prior();
   using T = StencilTile<real, TX, TY>;
   extern __shared__ __align__(128) unsigned char fsm[];
   int k0, l0, m0;

@@ -455,7 +455,8 @@ __device__ __forceinline__ bool in_refill_shell(const Parts<real>& P, const Geom
 }
 
 template <typename real>
-__global__ void delete_shell_kernel(Parts<real> P, int first, const int* __restrict__ count, Geom g) {
+__global__ void delete_shell_kernel(Parts<real> P, int first, const int* count, Geom g) {
+  after_prior();
   const int n = *count;
   for (int t = first + blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     const int c = P.cell[t];
@@ -555,6 +556,7 @@ __device__ __forceinline__ int slab_need(const SourceParams& sp, int i, int j, i
 // The call's particles, one thread each, into slots [dst, dst + total).
 template <typename real>
 __global__ void source_kernel(Parts<real> P, SourceParams sp, unsigned long long* err) {
+  after_prior();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= sp.total) return;
   int s = 0;
@@ -612,8 +614,9 @@ constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 4;
 constexpr int kScanTile = kScanThreads * kScanItems;
 
-static __global__ void __launch_bounds__(kScanThreads) scan_tile_kernel(const int* __restrict__ in, int* out,
+static __global__ void __launch_bounds__(kScanThreads) scan_tile_kernel(const int* in, int* out,
                                                                  int* sums, long long n) {
+  after_prior();
   __shared__ int warp_tot[32];
   const long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanItems;
   int v[kScanItems];
@@ -651,7 +654,8 @@ static __global__ void __launch_bounds__(kScanThreads) scan_tile_kernel(const in
   if (threadIdx.x == kScanThreads - 1) sums[blockIdx.x] = run;
 }
 
-static __global__ void scan_add_kernel(int* out, const int* __restrict__ add, long long n) {
+static __global__ void scan_add_kernel(int* out, const int* add, long long n) {
+  after_prior();
   const long long base = (long long)blockIdx.x * kScanTile;
   const int a = add[blockIdx.x];
   for (int q = threadIdx.x; q < kScanTile; q += blockDim.x) {

@@ -47,6 +47,7 @@ template <typename real>
 __global__ void classify_kernel(Parts<real> P, Geom g, TileGeom t, const int* __restrict__ goff,
                                 const int* __restrict__ gmax, int* gtop, int cap, int* holes, int* nholes,
                                 int* append_at, int* nonhome, int shell) {
+  after_prior();
   constexpr int U = 4;  // rows whose loads are in flight together (8 measured no faster)
   const int G = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -122,17 +123,28 @@ __global__ void classify_kernel(Parts<real> P, Geom g, TileGeom t, const int* __
   if (lane == 0) gtop[G] = top;
 }
 
-__global__ void clamp_count_kernel(const int* append_at, int cap, int* count_dev) {
-  *count_dev = min(*append_at, cap);
+// Before a re-layout: the append region starts at the count, and no spills, no
+// particle left outside its home, no arrivals yet.
+__global__ void relayout_begin_kernel(const int* count, int* append_at, int* nspill, int* nonhome, int* cursor,
+                                      long long ncells) {
+  after_prior();
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  for (long long c = t; c < ncells; c += (long long)gridDim.x * blockDim.x) cursor[c] = 0;
+  if (t == 0) {
+    *append_at = *count;
+    *nspill = 0;
+    *nonhome = 0;
+  }
 }
 
 // Placement, pass 1: the particle's rank among the appended particles of its
 // new cell (from the per-cell counter `cursor`); -1 for an empty slot or a
 // particle outside the interior (dropped).
 template <typename real>
-__global__ void __launch_bounds__(256) place_count_kernel(Parts<real> P, int first, const int* __restrict__ count,
-                                                          Geom g, int* cursor, int* rank) {
-  const int span = *count - first;
+__global__ void __launch_bounds__(256) place_count_kernel(Parts<real> P, int first, const int* append_at,
+                                                          int cap, Geom g, int* cursor, int* rank) {
+  after_prior();
+  const int span = min(*append_at, cap) - first;
   const int lane = threadIdx.x & 31;
   const int stride = gridDim.x * blockDim.x;
   for (int w0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; w0 < span; w0 += stride) {  // warp-uniform
@@ -146,10 +158,11 @@ __global__ void __launch_bounds__(256) place_count_kernel(Parts<real> P, int fir
 // Pass 2 (after an exclusive scan of the arrivals into bucket offsets): every
 // particle writes its index to its bucket slot.
 template <typename real>
-__global__ void __launch_bounds__(256) place_bucket_kernel(Parts<real> P, int first, const int* __restrict__ count,
-                                                           Geom g, const int* __restrict__ off,
+__global__ void __launch_bounds__(256) place_bucket_kernel(Parts<real> P, int first, const int* append_at,
+                                                           int cap, Geom g, const int* __restrict__ off,
                                                            const int* __restrict__ rank, int* bucket) {
-  const int span = *count - first;
+  after_prior();
+  const int span = min(*append_at, cap) - first;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < span; q += gridDim.x * blockDim.x) {
     const int r = rank[q];
     if (r >= 0) bucket[off[interior_key(g, P.cell[first + q])] + r] = q;
@@ -170,6 +183,7 @@ __global__ void place_fill_kernel(Parts<real> P, int first, Geom g, TileGeom t, 
                                   const int* __restrict__ arrivals, const int* __restrict__ nholes,
                                   const int* __restrict__ off, const int* __restrict__ bucket, int* nspill,
                                   Parts<real> Q) {
+  after_prior();
   constexpr int U = 4;  // holes per lane in flight together
   const int G = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -251,10 +265,13 @@ __global__ void place_fill_kernel(Parts<real> P, int first, Geom g, TileGeom t, 
   if (lane == 0) gtop[G] = top;
 }
 
-// The particles without a hole back to slots [first, first + n).
+// The particles without a hole back to slots [first, first + n), where the
+// count then ends.
 template <typename real>
-__global__ void unspill_kernel(Parts<real> Q, const int* __restrict__ nspill, Parts<real> P, int first) {
+__global__ void unspill_kernel(Parts<real> Q, const int* nspill, Parts<real> P, int first, int* count) {
+  after_prior();
   const int n = *nspill;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *count = first + n;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x)
     copy_slot(Q, q, P, first + q, Q.cell[q]);
 }

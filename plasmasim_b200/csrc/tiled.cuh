@@ -72,6 +72,7 @@ struct TileArgs {
   int ntail;        // CTAs of the grid that take the slots from `tail` to *count instead of a tile
   int tail;
   const int* count;
+  int overlap;      // the launch before is the other species' push: no need to wait for its end
 };
 
 // Group and lane of an interior cell (absolute indices), -1 outside the interior.
