@@ -50,7 +50,7 @@ struct Store {
   bool spill_pending = false;
   cudaEvent_t readback = nullptr;
   int* holes = nullptr;   // per-slot scratch: hole rows of every lane column
-  int* nholes = nullptr;  // per lane of every group: holes of its column
+  int* nholes = nullptr;  // per lane of every group: holes of its column, then how many of them are filled
   int* nspill = nullptr;  // a placement's particles without a hole
   int* nonhome = nullptr; // a particle outside its home cell stayed in the layout (after nspill)
   // a refill's shell deletion over the layout is left to the next classify pass
@@ -90,6 +90,7 @@ struct pic_ctx {
   int* goff[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
   int* gmax[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
   int* gtop[2] = {nullptr, nullptr};  // rows in use of each group of the current layout
+  int* glevel[2] = {nullptr, nullptr};  // its level when it was last sorted or re-laid
   int2* gfree = nullptr;              // a full sort's free slots (NewLayout)
   int* gcursor = nullptr;             // and its per-group cursor
   int lay[2] = {0, 0};                // current layout buffer
@@ -850,7 +851,7 @@ int do_sort_species(pic_ctx* c, int s) {
   Slab slabs[5];
   refill_slabs(c, slabs);
   group_size_kernel<<<gblocks, kThreads, 0, c->stream>>>(c->g, tg, stay, moved, source_params(c, s, slabs, 5, 0),
-                                                         c->gmax[s][nw], c->gtop[s], c->gfree, c->gcap);
+                                                         c->gmax[s][nw], c->glevel[s], c->gtop[s], c->gfree, c->gcap);
   CKL();
   CKR(scan_exclusive(c, c->gcap, c->goff[s][nw], tg.ngroups, c->scan_tmp, c->scan_tmp_len));
   tiled_total_kernel<<<1, 1, 0, c->stream>>>(c->goff[s][nw], c->gcap, tg.ngroups, c->total_dev);
@@ -911,7 +912,8 @@ int place_launch(pic_ctx* c, int s) {
                   off, c->rank, c->bucket));
   CKL();
   CK(launch_after(c, place_fill_kernel<real>, gblocks, kThreads, 0, P, (int)first, c->g, tg, c->goff[s][c->lay[s]],
-                  c->gmax[s][c->lay[s]], c->gtop[s], st.holes, c->cursor, st.nholes, off, c->bucket, st.nspill, Q));
+                  c->gmax[s][c->lay[s]], c->glevel[s], c->gtop[s], st.holes, c->cursor, st.nholes,
+                  st.nholes + (size_t)kLanes * tg.ngroups, off, c->bucket, st.nspill, Q));
   CKL();
   CK(launch_after(c, unspill_kernel<real>, particle_blocks(st.cap), kThreads, 0, Q, st.nspill, P, (int)first,
                   st.count_dev));
@@ -935,8 +937,9 @@ int relayout_launch(pic_ctx* c, int s) {
   CK(launch_after(c, relayout_begin_kernel, particle_blocks(c->ncells / 8), kThreads, 0, st.count_dev, c->append_dev,
                   st.nspill, st.nonhome, c->cursor, c->ncells));
   CKL();
-  CK(launch_after(c, classify_kernel<real>, gblocks, kThreads, 0, P, c->g, tg, c->goff[s][c->lay[s]],
-                  c->gmax[s][c->lay[s]], c->gtop[s], (int)st.cap, st.holes, st.nholes, c->append_dev, st.nonhome,
+  CK(launch_after(c, classify_kernel<real>, gblocks, kThreads, sizeof(Pending<real>) * (kThreads / 32), P, c->g, tg,
+                  c->goff[s][c->lay[s]], c->gmax[s][c->lay[s]], c->glevel[s], c->gtop[s], (int)st.cap, st.holes,
+                  st.nholes, st.nholes + (size_t)kLanes * tg.ngroups, c->append_dev, st.nonhome,
                   st.shell_pending ? 1 : 0));
   CKL();
   st.shell_pending = false;
@@ -1790,19 +1793,21 @@ int pic_create(const pic_config* cfg, pic_ctx** out) {
         if (cudaMalloc(&c->gmax[s][b], sizeof(int) * t.ngroups) != cudaSuccess) return fail(PIC_ERR_CUDA);
       }
     }
-    // gfree, gtop of both species and gcursor in one block
-    if (cudaMalloc(&c->gfree, (sizeof(int2) * kLanes + sizeof(int) * 3) * t.ngroups) != cudaSuccess)
+    // gfree, gtop and glevel of both species and gcursor in one block
+    if (cudaMalloc(&c->gfree, (sizeof(int2) * kLanes + sizeof(int) * 5) * t.ngroups) != cudaSuccess)
       return fail(PIC_ERR_CUDA);
     c->gtop[0] = (int*)(c->gfree + (size_t)kLanes * t.ngroups);
     c->gtop[1] = c->gtop[0] + t.ngroups;
-    c->gcursor = c->gtop[1] + t.ngroups;
+    c->glevel[0] = c->gtop[1] + t.ngroups;
+    c->glevel[1] = c->glevel[0] + t.ngroups;
+    c->gcursor = c->glevel[1] + t.ngroups;
     if (cudaMalloc(&c->gcap, sizeof(int) * t.ngroups) != cudaSuccess) return fail(PIC_ERR_CUDA);
     if (cudaMalloc(&c->total_dev, sizeof(int)) != cudaSuccess) return fail(PIC_ERR_CUDA);
     if (cudaMalloc(&c->append_dev, sizeof(int)) != cudaSuccess) return fail(PIC_ERR_CUDA);
     if (tiled) {  // re-layout scratch
       for (int s = 0; s < 2; ++s) {  // each species' hole lists live from its push to its next placement
         if (cudaMalloc(&c->sp[s].holes, sizeof(int) * (size_t)cap) != cudaSuccess) return fail(PIC_ERR_CUDA);
-        if (cudaMalloc(&c->sp[s].nholes, sizeof(int) * kLanes * t.ngroups) != cudaSuccess) return fail(PIC_ERR_CUDA);
+        if (cudaMalloc(&c->sp[s].nholes, sizeof(int) * 2 * kLanes * t.ngroups) != cudaSuccess) return fail(PIC_ERR_CUDA);
         if (cudaMalloc(&c->sp[s].nspill, 2 * sizeof(int)) != cudaSuccess) return fail(PIC_ERR_CUDA);
         c->sp[s].nonhome = c->sp[s].nspill + 1;
         cudaMemsetAsync(c->sp[s].nspill, 0, 2 * sizeof(int), c->stream);
@@ -1810,6 +1815,9 @@ int pic_create(const pic_config* cfg, pic_ctx** out) {
       if (cudaMalloc(&c->rank, sizeof(int) * (size_t)cap) != cudaSuccess) return fail(PIC_ERR_CUDA);
       if (cudaMalloc(&c->bucket, sizeof(int) * (size_t)cap) != cudaSuccess) return fail(PIC_ERR_CUDA);
     }
+    if (cudaFuncSetAttribute(classify_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(Pending<double>) * (kThreads / 32)) != cudaSuccess)
+      return fail(PIC_ERR_CUDA);
     const int pb_f = (int)PushSmem<float>::bytes, pb_d = (int)PushSmem<double>::bytes;
     if (cudaFuncSetAttribute(push_tiled_kernel<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, pb_d) !=
             cudaSuccess ||

@@ -2,14 +2,14 @@
 //
 // Between two sorts most particles stay in their home cell. A re-layout
 // leaves those where they are and moves only the rest:
-//  1. classify (one warp per group): a particle whose cell is not its lane's
-//     home cell (it moved, or sits in another lane's free slot) is copied to
-//     the append region after `count` and its slot becomes a hole (cell = -1);
-//     each lane lists the rows of its holes, in row order, in a scratch array
-//     laid out like the slots themselves. A warp takes append slots 64 at a
-//     time from the shared counter and marks the slots of its last block it
-//     does not use empty, so the counter sees one atomic per 64 movers instead
-//     of one per row;
+//  1. classify (one warp per group): a particle whose cell belongs to another
+//     lane of its group is handed to that lane on the spot; one that has left
+//     the group is copied to the append region after `count` and its slot
+//     becomes a hole (cell = -1); each lane lists the rows of its holes, in row
+//     order, in a scratch array laid out like the slots themselves. A warp
+//     takes append slots 64 at a time from the shared counter and marks the
+//     slots of its last block it does not use empty, so the counter sees one
+//     atomic per 64 movers instead of one per row;
 //  2. place (movers and refilled particles, all appended after `count`): the
 //     particles are bucketed by their new cell -- a rank per particle from a
 //     per-cell counter, an exclusive scan of the arrivals, the particle's
@@ -40,29 +40,108 @@ __device__ __forceinline__ void copy_slot(const Parts<real>& S, int s, const Par
   copy_record(S, s, D, d, c);
 }
 
+// A warp's particles on their way to another lane of their group: up to
+// kPending for each lane.
+constexpr int kPending = 4;
+template <typename real>
+struct Pending {
+  real a[kPending][kLanes][4], b[kPending][kLanes][4];  // records A, B
+  int n[kLanes];
+};
+__device__ __forceinline__ void put_record(float (&a)[4], float (&b)[4], const Rec<float>& r) {
+  *reinterpret_cast<float4*>(a) = make_float4(__int_as_float(r.cell), r.o[0], r.o[1], r.o[2]);
+  *reinterpret_cast<float4*>(b) = make_float4(r.v[0], r.v[1], r.v[2], 0.f);
+}
+__device__ __forceinline__ void put_record(double (&a)[4], double (&b)[4], const Rec<double>& r) {
+  double2* pa = reinterpret_cast<double2*>(a);
+  double2* pb = reinterpret_cast<double2*>(b);
+  pa[0] = make_double2(__hiloint2double(0, r.cell), r.o[0]);
+  pa[1] = make_double2(r.o[1], r.o[2]);
+  pb[0] = make_double2(r.v[0], r.v[1]);
+  pb[1] = make_double2(r.v[2], 0.0);
+}
+template <typename real>
+__device__ __forceinline__ Rec<real> get_record(const real (&a)[4], const real (&b)[4]) {
+  return Rec<real>{word_int(a[0]), {a[1], a[2], a[3]}, {b[0], b[1], b[2]}};
+}
+
+// One warp per group walks its rows, kRowsTogether at a time. A particle in
+// its lane's home cell stays. One whose cell belongs to another lane of the
+// group -- most of those that leave their cell do so along z, the drift's axis
+// -- goes to that lane's pending list in shared memory, and after each batch
+// of rows every lane copies its pending particles into its holes below the
+// group's level that lie in the rows read so far; where the list is full the
+// particle stays as a stranger. The others, and what is pending at the end,
+// go to the append region, from where the placement takes them. Each lane
+// lists the rows of its holes in order; the first hfirst of them are filled.
 // With `shell` set (the re-layout after a refill), a particle of the layout
 // that lies in a refill shell is deleted here, as add_*_flat's removal
 // (:6015-6031) would have: one pass over the layout for both.
+//
+// Bound by the latency of a batch (cells, then the movers' records, then the
+// pending lists) and its instructions; the next batch's cells are loaded ahead,
+// and 24 warps per SM (80 registers) were faster than 16 or 32. With every
+// mover in the append region the re-layout of both species took 2.00 ms per
+// step at 128^3 x 64, this way 1.41; 0.092 -> 0.084 at 64^3 x 16, FP64 64^3 x 32
+// 0.185 -> 0.165.
+constexpr int kRowsTogether = 4;
 template <typename real>
-__global__ void classify_kernel(Parts<real> P, Geom g, TileGeom t, const int* __restrict__ goff,
-                                const int* __restrict__ gmax, int* gtop, int cap, int* holes, int* nholes,
-                                int* append_at, int* nonhome, int shell) {
+__global__ void __launch_bounds__(256, sizeof(real) == 4 ? 3 : 2) classify_kernel(Parts<real> P, Geom g, TileGeom t, const int* __restrict__ goff,
+                                                       const int* __restrict__ gmax, const int* glevel, int* gtop,
+                                                       int cap, int* holes, int* nholes, int* hfirst, int* append_at,
+                                                       int* nonhome, int shell) {
   after_prior();
-  constexpr int U = 4;  // rows whose loads are in flight together (8 measured no faster)
+  constexpr int U = kRowsTogether;
+  extern __shared__ __align__(16) unsigned char pending_raw[];
   const int G = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (G >= t.ngroups) return;  // warp-uniform
+  Pending<real>& pend = reinterpret_cast<Pending<real>*>(pending_raw)[threadIdx.x >> 5];
   const unsigned below = (1u << lane) - 1u;
+  int hi, hj, hk;
   LaneCell lc;
-  const int home = home_key(g, t, G, lane, lc);
-  const int base = goff[G], m = gmax[G];
-  int nh = 0, top = 0;
-  int blk = 0, used = kAppendBlock;  // current block of append slots (warp-uniform)
-  for (int r0 = 0; r0 < m; r0 += U) {
-    int c[U], d[U];
-    bool moved[U];
+  const bool owns = home_cell(g, t, G, lane, hi, hj, hk, lc);
+  const int home = owns ? pack_cell(hi, hj, hk) : -2;
+  const int nv = cells_of_group(g, t, G);
+  const int column = hi << (2 * kCellBits) | hj << kCellBits, z0 = hk - lc.z;  // the group's cells: column | z0 .. z0 + nv - 1
+  const int base = goff[G], m = gmax[G], level = glevel[G];
+  int nh = 0, hu = 0, top = 0;
+  int nexth = 0;                          // row of hole hu, when hu < nh
+  int blk = 0, used = kAppendBlock;       // current block of append slots (warp-uniform)
+  pend.n[lane] = 0;
+  __syncwarp();
+  // Append slots for the lanes with `want`, -1 for the others; warp-uniform control.
+  const auto append = [&](bool want) {
+    const unsigned mm = __ballot_sync(0xffffffffu, want);
+    const int nm = __popc(mm);
+    if (nm > kAppendBlock - used) {  // close the block, take a new one
+      for (int q = used + lane; q < kAppendBlock; q += kLanes)
+        if (blk + q < cap) P.cell[blk + q] = -1;
+      int nb = 0;
+      if (lane == 0) nb = atomicAdd(append_at, kAppendBlock);
+      blk = __shfl_sync(0xffffffffu, nb, 0);
+      used = 0;
+    }
+    const int d = blk + used + __popc(mm & below);
+    used += nm;
+    return want ? d : -1;
+  };
+  const auto add_hole = [&](int r) {
+    holes[base + nh * kLanes + lane] = r;
+    if (nh == hu) nexth = r;
+    ++nh;
+  };
+  int next[U];  // the next batch's cells, on their way
+  const auto fetch = [&](int r0) {
 #pragma unroll
-    for (int u = 0; u < U; ++u) c[u] = r0 + u < m ? P.cell[base + (r0 + u) * kLanes + lane] : -1;
+    for (int u = 0; u < U; ++u) next[u] = r0 + u < m ? P.cell[base + (r0 + u) * kLanes + lane] : -1;
+  };
+  fetch(0);
+  for (int r0 = 0; r0 < m; r0 += U) {
+    int c[U], d[U], k[U], to[U];  // cell; append slot, pending entry and lane, -1 none
+#pragma unroll
+    for (int u = 0; u < U; ++u) c[u] = next[u];
+    fetch(r0 + U);
     if (shell) {
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -75,49 +154,81 @@ __global__ void classify_kernel(Parts<real> P, Geom g, TileGeom t, const int* __
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int r = r0 + u;
-      const int key = interior_key(g, c[u]);
-      const bool leaves = c[u] >= 0 && (key < 0 || key != home);
-      const bool mover = leaves && key >= 0;
-      const unsigned mm = __ballot_sync(0xffffffffu, mover);
-      const int nm = __popc(mm);
-      if (nm > kAppendBlock - used) {  // close the block, take a new one
-        for (int q = used + lane; q < kAppendBlock; q += kLanes)
-          if (blk + q < cap) P.cell[blk + q] = -1;
-        int nb = 0;
-        if (lane == 0) nb = atomicAdd(append_at, kAppendBlock);
-        blk = __shfl_sync(0xffffffffu, nb, 0);
-        used = 0;
+      const int r = r0 + u, slot = base + r * kLanes + lane;
+      d[u] = k[u] = -1;
+      to[u] = 0;
+      bool stays = c[u] == home, goes = false;
+      if (c[u] >= 0 && !stays) {
+        const int z = c[u] - (column | z0);  // below nv for the group's cells only
+        if ((unsigned)z < (unsigned)nv && owns) {
+          const int n = lanes_of(nv, z);
+          to[u] = n == 1 ? z : z + nv * (r % n);
+          k[u] = atomicAdd(&pend.n[to[u]], 1);
+          if (k[u] >= kPending) {
+            atomicSub(&pend.n[to[u]], 1);
+            k[u] = -1;
+            stays = true;
+          }
+        } else if (interior_key(g, c[u]) >= 0) {
+          goes = true;
+        } else {  // outside the interior: dropped
+          P.cell[slot] = -1;
+          c[u] = -1;
+        }
       }
-      d[u] = blk + used + __popc(mm & below);
-      used += nm;
-      // a mover that finds the append region full stays where it is
-      moved[u] = mover && d[u] < cap;
-      if (mover && !moved[u]) *nonhome = 1;
-      const bool hole = c[u] < 0 || (leaves && (moved[u] || !mover));
-      if (hole && c[u] >= 0 && !moved[u]) P.cell[base + r * kLanes + lane] = -1;
-      if (hole && r < m) {
-        holes[base + nh * kLanes + lane] = r;
-        ++nh;
+      d[u] = append(goes);
+      if (goes && d[u] >= cap) {  // the append region is full: it stays where it is
+        *nonhome = 1;
+        d[u] = -1;
+        stays = true;
       }
-      if (!hole) top = r + 1;  // a particle stays in this row
+      if (stays) top = r + 1;
+      else if (r < m) add_hole(r);
     }
-    // the movers of the U rows: their record loads issued together, then the copies
+    // the U rows' movers: their record loads issued together, then the copies
     Rec<real> rec[U];
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (moved[u]) rec[u] = load_records(P, base + (r0 + u) * kLanes + lane);
+      if (d[u] >= 0 || k[u] >= 0) rec[u] = load_records(P, base + (r0 + u) * kLanes + lane);
+    __syncwarp();
 #pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (moved[u]) {
-        const Rec<real>& q = rec[u];
-        store_records(P, d[u], c[u], q.o[0], q.o[1], q.o[2], q.v[0], q.v[1], q.v[2]);
-        P.cell[base + (r0 + u) * kLanes + lane] = -1;
-      }
+    for (int u = 0; u < U; ++u) {
+      const Rec<real>& q = rec[u];
+      if (d[u] >= 0) store_records(P, d[u], c[u], q.o[0], q.o[1], q.o[2], q.v[0], q.v[1], q.v[2]);
+      if (k[u] >= 0) put_record(pend.a[k[u]][to[u]], pend.b[k[u]][to[u]], q);
+      if (d[u] >= 0 || k[u] >= 0) P.cell[base + (r0 + u) * kLanes + lane] = -1;
+    }
+    __syncwarp();
+    int np = pend.n[lane];
+    while (np > 0 && hu < nh && nexth < level) {
+      --np;
+      const Rec<real> q = get_record(pend.a[np][lane], pend.b[np][lane]);
+      store_records(P, base + nexth * kLanes + lane, q.cell, q.o[0], q.o[1], q.o[2], q.v[0], q.v[1], q.v[2]);
+      top = max(top, nexth + 1);
+      if (++hu < nh) nexth = holes[base + hu * kLanes + lane];
+    }
+    pend.n[lane] = np;
+    __syncwarp();
+  }
+  // still pending: to the append region
+  const int np = pend.n[lane];
+#pragma unroll
+  for (int q = 0; q < kPending; ++q) {
+    int d = append(q < np);
+    if (d < 0) continue;
+    const Rec<real> p = get_record(pend.a[q][lane], pend.b[q][lane]);
+    if (d >= cap) {  // no room there: into one of the lane's holes, wherever that is
+      *nonhome = 1;
+      d = base + nexth * kLanes + lane;
+      top = max(top, nexth + 1);
+      if (++hu < nh) nexth = holes[base + hu * kLanes + lane];
+    }
+    store_records(P, d, p.cell, p.o[0], p.o[1], p.o[2], p.v[0], p.v[1], p.v[2]);
   }
   for (int q = used + lane; q < kAppendBlock; q += kLanes)
     if (blk + q < cap && used < kAppendBlock) P.cell[blk + q] = -1;
   nholes[G * kLanes + lane] = nh;
+  hfirst[G * kLanes + lane] = hu;
 #pragma unroll
   for (int s = 16; s > 0; s >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, s));
   if (lane == 0) gtop[G] = top;
@@ -179,8 +290,9 @@ __global__ void __launch_bounds__(256) place_bucket_kernel(Parts<real> P, int fi
 // last row that kept a particle and goes out covering the filled rows as well.
 template <typename real>
 __global__ void place_fill_kernel(Parts<real> P, int first, Geom g, TileGeom t, const int* __restrict__ goff,
-                                  const int* __restrict__ gmax, int* gtop, const int* __restrict__ holes,
-                                  const int* __restrict__ arrivals, const int* __restrict__ nholes,
+                                  const int* __restrict__ gmax, int* glevel, int* gtop,
+                                  const int* __restrict__ holes, const int* __restrict__ arrivals,
+                                  const int* __restrict__ nholes, const int* __restrict__ hfirst,
                                   const int* __restrict__ off, const int* __restrict__ bucket, int* nspill,
                                   Parts<real> Q) {
   after_prior();
@@ -196,9 +308,11 @@ __global__ void place_fill_kernel(Parts<real> P, int first, Geom g, TileGeom t, 
   const int narr = warp_sum(arr);
   if (narr == 0) return;
   const int o = home >= 0 ? off[home] + lc.m : 0;
-  const int nh = nholes[G * kLanes + lane];
+  const int hu = hfirst[G * kLanes + lane], nh = nholes[G * kLanes + lane] - hu;
   const int base = goff[G], rows = gmax[G];
+  const int* hole = holes + base + hu * kLanes + lane;  // the lane's k-th hole: hole[k * kLanes]
   const int level = min(rows, group_level(rows * kLanes - warp_sum(nh) + narr));
+  if (lane == 0) glevel[G] = level;
   const int n = min(arr, nh);
   int top = gtop[G];
   int used = 0;  // holes this lane has filled
@@ -208,7 +322,7 @@ __global__ void place_fill_kernel(Parts<real> P, int first, Geom g, TileGeom t, 
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int k = k0 + u;
-      const int row = k < n ? holes[base + k * kLanes + lane] : level;
+      const int row = k < n ? hole[k * kLanes] : level;
       src[u] = row < level ? first + bucket[o + k * lc.n] : -1;
       dst[u] = base + row * kLanes + lane;
       if (row < level) {
@@ -228,7 +342,7 @@ __global__ void place_fill_kernel(Parts<real> P, int first, Geom g, TileGeom t, 
   const int nrest = warp_sum(rest);
   int done = 0;
   for (int k = used; done < nrest; ++k) {
-    const int row = k < nh ? holes[base + k * kLanes + lane] : level;
+    const int row = k < nh ? hole[k * kLanes] : level;
     const unsigned m = __ballot_sync(0xffffffffu, row < level);
     if (!m) break;
     const int s = done + __popc(m & below);

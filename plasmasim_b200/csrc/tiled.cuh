@@ -214,6 +214,7 @@ __device__ __forceinline__ int group_level(int n) { return n > 0 ? (n + kLanes -
 // slots free below the level, numbered lane by lane (NewLayout::free).
 __global__ void group_size_kernel(Geom g, TileGeom t, const int* __restrict__ stay,
                                   const int* __restrict__ moved, SourceParams refill, int* gmax,
+                                  int* glevel,
                                   int* gtop, int2* free, int* gcap) {
   const int G = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -228,7 +229,7 @@ __global__ void group_size_kernel(Geom g, TileGeom t, const int* __restrict__ st
   free[G * kLanes + lane] = make_int2(warp_scan(free_below) - free_below, min(c, level));
   if (lane == 0) {
     gmax[G] = rows;
-    gtop[G] = level;
+    gtop[G] = glevel[G] = level;
     gcap[G] = rows * kLanes;
   }
 }
