@@ -760,30 +760,54 @@ int do_push(pic_ctx* c, int s, long long first = 0) {
   return PIC_OK;
 }
 
-// The push of species s. `overlap`: the launch just before on the stream is the
-// other species' tiled push, which this one may run beside (push_tiled.cuh).
-template <typename real>
-int do_push_tiled(pic_ctx* c, int s, bool overlap = false) {
-  if (!c->layout[s]) return do_push<real, PUSH_FUSED>(c, s);
-  const int ntiles = c->tg.ntx * c->tg.nty * c->tg.ntz;
-  // a CTA per SM for the tail, whose length only the device may know
-  const long long tail = slot_bound(c, s) - c->tiled_end[s];
+// Whether species s's tail (the slots after its layout) is long enough for a
+// launch of its own: a refill that the reference's loop leaves unsorted for
+// many steps, not the few slots that a re-layout leaves.
+bool long_tail(const pic_ctx* c, int s) {
+  return !c->sp[s].pending && c->sp[s].count - c->tiled_end[s] > 148LL * 2 * kThreads;
+}
+
+// The tiles of species s's layout and, when it is not long, a CTA per SM for
+// its tail, whose length only the device may know. `overlap`: the launch just before on the stream is
+// the same kernel for the other species, which this one may run beside
+// (push_tiled.cuh).
+TileArgs tile_args(const pic_ctx* c, int s, bool overlap) {
+  const long long tail = long_tail(c, s) ? 0 : slot_bound(c, s) - c->tiled_end[s];
   const int ntail = (int)std::min<long long>((std::max<long long>(tail, 0) + kThreads - 1) / kThreads, 148);
-  const TileArgs ta{c->tg, c->goff[s][c->lay[s]], c->gtop[s], ntail, (int)c->tiled_end[s], c->sp[s].count_dev, overlap};
+  return TileArgs{c->tg, c->goff[s][c->lay[s]], c->gtop[s], ntail, (int)c->tiled_end[s], c->sp[s].count_dev, overlap};
+}
+
+// The push of species s, of every part (PUSH_FUSED) or up to the J deposit.
+template <typename real, int MODE>
+int do_push_tiled(pic_ctx* c, int s, bool overlap = false) {
+  if (!c->layout[s]) return do_push<real, MODE>(c, s);
+  if (long_tail(c, s)) CKR((do_push<real, MODE>(c, s, c->tiled_end[s])));
+  const TileArgs ta = tile_args(c, s, overlap && !long_tail(c, s));
   const bool vec = c->g.gz * sizeof(real) % 16 == 0;
-  CK(launch_after(c, vec ? push_tiled_kernel<real, true> : push_tiled_kernel<real, false>, ntail + ntiles,
-                  kTileX * kTileY * 32, PushSmem<real>::bytes, parts<real>(c, s), ta, fields<real>(c), c->g,
-                  push_const<real>(c, s), c->err));
+  CK(launch_after(c, vec ? push_tiled_kernel<real, true, MODE> : push_tiled_kernel<real, false, MODE>,
+                  ta.ntail + c->tg.ntx * c->tg.nty * c->tg.ntz, kTileX * kTileY * 32, PushSmem<real>::bytes,
+                  parts<real>(c, s), ta, fields<real>(c), c->g, push_const<real>(c, s), c->err));
   CKL();
   return PIC_OK;
 }
 
 template <typename real>
-int do_drift_n(pic_ctx* c, int s) {
+int do_drift_n(pic_ctx* c, int s, bool overlap = false) {
   if (c->sp[s].count == 0) return PIC_OK;
-  drift_n_kernel<real><<<particle_blocks(c->sp[s].count), kThreads, 0, c->stream>>>(
-      parts<real>(c, s), c->sp[s].count_dev, fields<real>(c), c->g, push_const<real>(c, s), c->err);
-  CKL();
+  const bool tiles = c->layout[s], apart = !tiles || long_tail(c, s);
+  if (apart) {
+    const long long first = tiles ? c->tiled_end[s] : 0;
+    drift_n_kernel<real><<<particle_blocks(c->sp[s].count - first), kThreads, 0, c->stream>>>(
+        parts<real>(c, s), (int)first, c->sp[s].count_dev, fields<real>(c), c->g, push_const<real>(c, s), c->err);
+    CKL();
+  }
+  if (tiles) {
+    const TileArgs ta = tile_args(c, s, overlap && !apart);
+    CK(launch_after(c, c->g.gz % 4 == 0 ? drift_tiled_kernel<real, true> : drift_tiled_kernel<real, false>,
+                    ta.ntail + c->tg.ntx * c->tg.nty * c->tg.ntz, kTileX * kTileY * 32, 0, parts<real>(c, s), ta,
+                    fields<real>(c), c->g, push_const<real>(c, s), c->err));
+    CKL();
+  }
   return PIC_OK;
 }
 
@@ -1344,7 +1368,7 @@ int do_step(pic_ctx* c) {
   // the counts stay on the device: the push and the diagnostics cover the
   // slots up to the capacity and stop at the device count, and the host reads
   // a count back only when an entry point needs it
-  for (int s = 0; s < 2; ++s) CKR(do_push_tiled<real>(c, s, s == 1 && c->layout[0]));
+  for (int s = 0; s < 2; ++s) CKR((do_push_tiled<real, PUSH_FUSED>(c, s, s == 1 && c->layout[0])));
   if (c->has_xport) CKR(do_migrate<real>(c));  // sr_particle's exchange between ranks
   CKR(phase_mark(c, PH_PUSH));
   CKR(phase_mark(c, PH_FIELD));
@@ -1819,14 +1843,17 @@ int pic_create(const pic_config* cfg, pic_ctx** out) {
                              (int)sizeof(Pending<double>) * (kThreads / 32)) != cudaSuccess)
       return fail(PIC_ERR_CUDA);
     const int pb_f = (int)PushSmem<float>::bytes, pb_d = (int)PushSmem<double>::bytes;
-    if (cudaFuncSetAttribute(push_tiled_kernel<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, pb_d) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(push_tiled_kernel<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, pb_d) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(push_tiled_kernel<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, pb_f) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(push_tiled_kernel<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, pb_f) !=
-            cudaSuccess)
+    const auto allow = [](const void* k, int bytes) {
+      return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
+    };
+    if (!allow((const void*)push_tiled_kernel<double, false, PUSH_FUSED>, pb_d) ||
+        !allow((const void*)push_tiled_kernel<double, true, PUSH_FUSED>, pb_d) ||
+        !allow((const void*)push_tiled_kernel<float, false, PUSH_FUSED>, pb_f) ||
+        !allow((const void*)push_tiled_kernel<float, true, PUSH_FUSED>, pb_f) ||
+        !allow((const void*)push_tiled_kernel<double, false, PUSH_J>, pb_d) ||
+        !allow((const void*)push_tiled_kernel<double, true, PUSH_J>, pb_d) ||
+        !allow((const void*)push_tiled_kernel<float, false, PUSH_J>, pb_f) ||
+        !allow((const void*)push_tiled_kernel<float, true, PUSH_J>, pb_f))
       return fail(PIC_ERR_CUDA);
   }
   if (cudaMalloc(&c->acc, sizeof(double) * 64) != cudaSuccess) return fail(PIC_ERR_CUDA);
@@ -1932,7 +1959,8 @@ int pic_push_deposit_j(pic_ctx* c, int species) {
   if (species < -1 || species > 1) return PIC_ERR_ARG;
   for (int s = 0; s < 2; ++s) {
     if (species >= 0 && s != species) continue;
-    CKR((c->prec == 64 ? do_push<double, PUSH_J>(c, s) : do_push<float, PUSH_J>(c, s)));
+    const bool overlap = species < 0 && s == 1 && c->layout[0] && c->layout[1];
+    CKR((c->prec == 64 ? do_push_tiled<double, PUSH_J>(c, s, overlap) : do_push_tiled<float, PUSH_J>(c, s, overlap)));
   }
   return PIC_OK;
 }
@@ -1942,7 +1970,8 @@ int pic_drift_deposit_n(pic_ctx* c, int species) {
   if (species < -1 || species > 1) return PIC_ERR_ARG;
   for (int s = 0; s < 2; ++s) {
     if (species >= 0 && s != species) continue;
-    CKR((c->prec == 64 ? do_drift_n<double>(c, s) : do_drift_n<float>(c, s)));
+    const bool overlap = species < 0 && s == 1 && c->layout[0] && c->layout[1] && c->sp[0].count > 0;
+    CKR((c->prec == 64 ? do_drift_n<double>(c, s, overlap) : do_drift_n<float>(c, s, overlap)));
   }
   return PIC_OK;
 }

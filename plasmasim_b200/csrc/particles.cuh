@@ -396,33 +396,48 @@ __global__ void __launch_bounds__(256) push_kernel(Parts<real> P, int first, con
                          err);
 }
 
-// Drift to x^{n+1} and density deposit (fdtd :818-867).
+// The density of a particle at (i, j, k) + offsets, where its stencil lies in
+// the array.
 template <typename real>
-__global__ void __launch_bounds__(256) drift_n_kernel(Parts<real> P, const int* __restrict__ count,
+__device__ __forceinline__ void drift_density(const Fields<real>& F, const Geom& g, const PushConst<real>& pc, int i,
+                                              int j, int k, real fx, real fy, real fz, unsigned long long* err) {
+  if (!in_array(g, i, j, k)) return;
+  if (stencil_ok(g, i, j, k)) deposit_n(F, g, pc, axis_weights(i, fx), axis_weights(j, fy), axis_weights(k, fz));
+  else count_err(err, ERR_DEPOSIT_OOB);
+}
+
+__device__ __forceinline__ void store_position(const Parts<float>& P, int t, int c, float fx, float fy, float fz) {
+  reinterpret_cast<float4*>(P.ra)[t] = make_float4(__int_as_float(c), fx, fy, fz);
+}
+__device__ __forceinline__ void store_position(const Parts<double>& P, int t, int c, double fx, double fy, double fz) {
+  double2* a = reinterpret_cast<double2*>(P.ra + 4 * (long long)t);
+  a[0] = make_double2(__hiloint2double(0, c), fx);
+  a[1] = make_double2(fy, fz);
+}
+
+// Drift to x^{n+1} and density deposit (fdtd :818-867) of slots first,
+// first + stride, ... below n.
+template <typename real>
+__device__ __forceinline__ void drift_slots(const Parts<real>& P, int first, int stride, int n, const Fields<real>& F,
+                                            const Geom& g, const PushConst<real>& pc, unsigned long long* err) {
+  for (int t = first; t < n; t += stride) {
+    const Rec<real> r = load_records(P, t);
+    if (r.cell < 0) continue;
+    int i, j, k;
+    unpack_cell(r.cell, i, j, k);
+    real fx = r.o[0], fy = r.o[1], fz = r.o[2];
+    advance(i, fx, r.v[0] * pc.hdt);
+    advance(j, fy, r.v[1] * pc.hdt);
+    advance(k, fz, r.v[2] * pc.hdt);
+    drift_density(F, g, pc, i, j, k, fx, fy, fz, err);
+    store_position(P, t, repack(i, j, k, err), fx, fy, fz);
+  }
+}
+template <typename real>
+__global__ void __launch_bounds__(256) drift_n_kernel(Parts<real> P, int first, const int* __restrict__ count,
                                                       Fields<real> F, Geom g, PushConst<real> pc,
                                                       unsigned long long* err) {
-  const int n = *count;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-    const int c = P.cell[t];
-    if (c < 0) continue;
-    int i, j, k;
-    unpack_cell(c, i, j, k);
-    real fx = P.o[0][t], fy = P.o[1][t], fz = P.o[2][t];
-    const real vx = P.v[0][t], vy = P.v[1][t], vz = P.v[2][t];
-    advance(i, fx, vx * pc.hdt);
-    advance(j, fy, vy * pc.hdt);
-    advance(k, fz, vz * pc.hdt);
-    if (in_array(g, i, j, k)) {
-      if (stencil_ok(g, i, j, k)) {
-        const Axis<real> X = axis_weights(i, fx), Y = axis_weights(j, fy), Z = axis_weights(k, fz);
-        deposit_n(F, g, pc, X, Y, Z);
-      } else {
-        count_err(err, ERR_DEPOSIT_OOB);
-      }
-    }
-    P.cell[t] = repack(i, j, k, err);
-    P.o[0][t] = fx; P.o[1][t] = fy; P.o[2][t] = fz;
-  }
+  drift_slots(P, first + blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, *count, F, g, pc, err);
 }
 
 // sr_particle at size 1 on its own.

@@ -350,6 +350,39 @@ __device__ __forceinline__ void step_cell(int& c, real& fx, real& fy, real& fz, 
   step_axis(c, fz, dz, kUnitZ);
 }
 
+// The scale of a tile's density window (add_density): FP32 sums fixed-point
+// weights at a scale that no node of a tile of `slots` rows can overflow, below
+// 2^23 as well, where the rounding by an added 2^23 is exact.
+__device__ __forceinline__ double window_scale(double weight, int) { return weight; }
+__device__ __forceinline__ float window_scale(float, int slots) {
+  return fminf(4294967295.f / (float)(slots * kLanes + 1), 8388607.f);
+}
+// Four consecutive nodes of the window as densities.
+template <typename real>
+struct Four {
+  real v[4];
+};
+__device__ __forceinline__ Four<double> window_density(const double* s, double, double) {
+  return Four<double>{{s[0], s[1], s[2], s[3]}};
+}
+__device__ __forceinline__ Four<float> window_density(const float* s, float weight, float scale) {
+  const unsigned* u = reinterpret_cast<const unsigned*>(s);
+  const float back = weight / scale;
+  return Four<float>{{(float)u[0] * back, (float)u[1] * back, (float)u[2] * back, (float)u[3] * back}};
+}
+// Adds them to a plane: one reduction where the rows allow, `left` nodes to the row's end.
+template <bool VEC, typename real>
+__device__ __forceinline__ void flush_nodes(real* dst, int left, const Four<real>& f) {
+  if (f.v[0] == (real)0 && f.v[1] == (real)0 && f.v[2] == (real)0 && f.v[3] == (real)0) return;
+  if constexpr (VEC && sizeof(real) == 4) {
+    red_add_v4(dst, f.v[0], f.v[1], f.v[2], f.v[3]);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (e < left && f.v[e] != (real)0) atomicAdd(dst + e, f.v[e]);
+  }
+}
+
 // Record B's fourth word after the main loop: what is left to do for the
 // particle (0 nothing, kLeftAll the whole push, kLeftEnd the density deposit
 // and sr_particle).
@@ -359,22 +392,22 @@ __device__ __forceinline__ int left_of(const Parts<real>& P, int t) { return (in
 
 // The slots after the layout (particles without a hole in their group): the
 // slot-order push, in the grid's first blocks.
-template <typename real>
+template <typename real, int MODE>
 __device__ __noinline__ void push_tail(const Parts<real>& P, const TileArgs& ta, const Fields<real>& F, const Geom& g,
                                        const PushConst<real>& pc, unsigned long long* err) {
-  push_slots<real, PUSH_FUSED>(P, ta.tail + blockIdx.x * blockDim.x + threadIdx.x, ta.ntail * blockDim.x, *ta.count, F,
+  push_slots<real, MODE>(P, ta.tail + blockIdx.x * blockDim.x + threadIdx.x, ta.ntail * blockDim.x, *ta.count, F,
                                g, pc, err);
 }
 
 // What the main loop left of particle t to the general path.
-template <typename real>
+template <typename real, int MODE>
 __device__ __noinline__ void push_rest(const Parts<real>& P, int t, const Fields<real>& F, const Geom& g,
                                        const PushConst<real>& pc, unsigned long long* err) {
   const Rec<real> r = load_records(P, t);
   const int left = left_of(P, t);
   if (r.cell < 0 || left == 0) return;
-  if (left == kLeftAll) {
-    push_one<real, PUSH_FUSED>(P, t, r, F, g, pc, err);
+  if (MODE == PUSH_J || left == kLeftAll) {
+    push_one<real, MODE>(P, t, r, F, g, pc, err);
     return;
   }
   int i, j, k;
@@ -390,7 +423,8 @@ __device__ __noinline__ void push_rest(const Parts<real>& P, int t, const Fields
 }
 
 // The fused particle part of one step (push, J deposit at x^{n+1/2}, drift,
-// n deposit at x^{n+1}, sr_particle) for one species over the tiled layout;
+// n deposit at x^{n+1}, sr_particle), or with MODE = PUSH_J its first two
+// parts, for one species over the tiled layout;
 // the same arithmetic as push_kernel<real, PUSH_FUSED> apart from the FP32
 // square roots and divisions and, in FP32, the fixed-point sums of the density
 // window. One CTA per tile, one warp per group; the first ntail CTAs take the
@@ -428,7 +462,7 @@ __device__ __noinline__ void push_rest(const Parts<real>& P, int t, const Fields
 #ifndef PB_PUSH64_MIN_BLOCKS
 #define PB_PUSH64_MIN_BLOCKS 1
 #endif
-template <typename real, bool VEC>
+template <typename real, bool VEC, int MODE>
 __global__ void __launch_bounds__(kTileX * kTileY * 32, sizeof(real) == 4 ? 2 : PB_PUSH64_MIN_BLOCKS)
 push_tiled_kernel(const __grid_constant__ Parts<real> P, const __grid_constant__ TileArgs ta,
                   const __grid_constant__ Fields<real> F, const __grid_constant__ Geom g,
@@ -436,7 +470,7 @@ push_tiled_kernel(const __grid_constant__ Parts<real> P, const __grid_constant__
   if (!ta.overlap) wait_prior();
   release_next();
   if ((int)blockIdx.x < ta.ntail) {
-    push_tail(P, ta, F, g, pc, err);
+    push_tail<real, MODE>(P, ta, F, g, pc, err);
     wait_prior();
     return;
   }
@@ -472,17 +506,10 @@ push_tiled_kernel(const __grid_constant__ Parts<real> P, const __grid_constant__
   const int nv = tile_cells(g, tz), hk = wz0 + 2 + lane_cell(nv, lane).z;
   const int hcell = pack_cell(hi, hj, hk);
   const int wcell0 = (wx0 * WY + wy0) * WZ + wz0;  // window node of a cell: (i WY + j) WZ + k less this
-  // FP32: the density window holds fixed-point sums (add_density) at a scale
-  // that no node of this tile can overflow
-  constexpr bool kFixedN = sizeof(real) == 4;
-  real nscale = pc.nw;
-  if (kFixedN) {
-    int slots = 0;
+  int slots = 0;
 #pragma unroll
-    for (int w = 0; w < kTileX * kTileY; ++w) slots += ta.gtop[tile * (kTileX * kTileY) + w];
-    // below 2^23 as well, where add_density's rounding by an added 2^23 is exact
-    nscale = (real)fminf(4294967295.f / (float)(slots * kLanes + 1), 8388607.f);
-  }
+  for (int w = 0; w < kTileX * kTileY; ++w) slots += ta.gtop[tile * (kTileX * kTileY) + w];
+  const real nscale = window_scale(pc.nw, slots);
   HomeJ<real> acc;
   acc.zero();
   // the warp's queue of J deposits off the home cells: entries [0, nq), 7
@@ -580,7 +607,7 @@ push_tiled_kernel(const __grid_constant__ Parts<real> P, const __grid_constant__
         __syncwarp();
       }
     }
-    step_cell(c, fx, fy, fz, dx, dy, dz);
+    if (MODE == PUSH_FUSED) step_cell(c, fx, fy, fz, dx, dy, dz);
     if (quick) {
       if (off_unit(fx) || off_unit(fy) || off_unit(fz)) {
         unit_fix(c, fx, kUnitX);
@@ -589,8 +616,8 @@ push_tiled_kernel(const __grid_constant__ Parts<real> P, const __grid_constant__
       }
       unpack_cell(c, i, j, k);
       int cnew = c;
-      bool dep = near.has(i, j, k);
-      if (!dep) {
+      bool dep = MODE == PUSH_FUSED && near.has(i, j, k);
+      if (MODE == PUSH_FUSED && !dep) {
         // past the interior (sr_particle's business), or out of the window too
         dep = (unsigned)(i - wx0 - 1) < WX - 2 && (unsigned)(j - wy0 - 1) < WY - 2 && (unsigned)(k - wz0 - 1) < WZ - 2 &&
               stencil_ok(g, i, j, k);
@@ -622,9 +649,9 @@ push_tiled_kernel(const __grid_constant__ Parts<real> P, const __grid_constant__
   // faces of x and y since the last re-layout, mostly), or every row when the
   // list overflowed
   if (nrest > S::kRest) {
-    for (int jj = 0; jj < jmax; ++jj) push_rest(P, base + jj * kLanes + lane, F, g, pc, err);
+    for (int jj = 0; jj < jmax; ++jj) push_rest<real, MODE>(P, base + jj * kLanes + lane, F, g, pc, err);
   } else {
-    for (int q = lane; q < nrest; q += kLanes) push_rest(P, rest[q], F, g, pc, err);
+    for (int q = lane; q < nrest; q += kLanes) push_rest<real, MODE>(P, rest[q], F, g, pc, err);
   }
   // the lane's home-cell sums into the window (nodes h-1 .. h+1 around it)
   cp_async_wait<0>();
@@ -650,32 +677,102 @@ push_tiled_kernel(const __grid_constant__ Parts<real> P, const __grid_constant__
   // flush the window: one reduction per 4 consecutive z nodes
   const int planes[4] = {pc.pjx, pc.pjy, pc.pjz, pc.pn};
   constexpr int NZ4 = WZ / 4;
-  for (int q4 = threadIdx.x; q4 < 4 * WX * WY * NZ4; q4 += blockDim.x) {
+  for (int q4 = threadIdx.x; q4 < (MODE == PUSH_FUSED ? 4 : 3) * WX * WY * NZ4; q4 += blockDim.x) {
     const int q = q4 / (WX * WY * NZ4);
     const int r = q4 % (WX * WY * NZ4);
     const int a = r / (WY * NZ4), b = (r / NZ4) % WY, c4 = r % NZ4;
     const int ga = wx0 + a, gb = wy0 + b, gc = wz0 + 4 * c4;
     if (ga >= g.gx || gb >= g.gy || gc >= g.gz) continue;
-    const real* src = (q == 3 ? wn : wj + q * WN) + (a * WY + b) * WZ + 4 * c4;
-    real v0 = src[0], v1 = src[1], v2 = src[2], v3 = src[3];
-    if (kFixedN && q == 3) {  // fixed-point density sums back to weights
-      const unsigned* u = reinterpret_cast<const unsigned*>(src);
-      const real back = pc.nw / nscale;
-      v0 = (real)u[0] * back; v1 = (real)u[1] * back; v2 = (real)u[2] * back; v3 = (real)u[3] * back;
-    }
-    if (v0 == (real)0 && v1 == (real)0 && v2 == (real)0 && v3 == (real)0) continue;
-    real* dst = F.f[planes[q]] + ga * g.sx + gb * g.gz + gc;
-    if (VEC && sizeof(real) == 4) {
-      red_add_v4(reinterpret_cast<float*>(dst), (float)v0, (float)v1, (float)v2, (float)v3);
+    Four<real> v;
+    if (q == 3) {
+      v = window_density(wn + (a * WY + b) * WZ + 4 * c4, pc.nw, nscale);
     } else {
-      const real v[4] = {v0, v1, v2, v3};
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (gc + e < g.gz && v[e] != (real)0) atomicAdd(dst + e, v[e]);
+      const real* src = wj + q * WN + (a * WY + b) * WZ + 4 * c4;
+      v = Four<real>{{src[0], src[1], src[2], src[3]}};
     }
+    flush_nodes<VEC>(F.f[planes[q]] + ga * g.sx + gb * g.gz + gc, g.gz - gc, v);
   }
   wait_prior();
 }
 
+// The drift loop of fdtd (:818-867) over the tiled layout: each particle to
+// x^{n+1} and its density, into the tile's window as in push_tiled_kernel; a
+// cell whose stencil leaves the window or the array goes the general way. One
+// CTA per tile, one warp per group, U rows' records in flight; the first ntail
+// CTAs take the slots after the layout. Bound by the records' latency and the
+// shared reductions; with PUSH_J in tiles as well, against a thread per slot and
+// atomics on the planes: four loop bodies of 48^3 x 16 by single functions
+// took 3.9 ms, now 2.7, 0.7 of either to read the grid back.
+template <typename real, bool VEC>
+__global__ void __launch_bounds__(kTileX * kTileY * 32)
+drift_tiled_kernel(const __grid_constant__ Parts<real> P, const __grid_constant__ TileArgs ta,
+                   const __grid_constant__ Fields<real> F, const __grid_constant__ Geom g,
+                   const __grid_constant__ PushConst<real> pc, unsigned long long* err) {
+  using S = PushSmem<real>;
+  constexpr int WY = S::WY, WZ = S::WZ, WN = S::WN, WX = S::WX, U = sizeof(real) == 4 ? 4 : 2;
+  if (!ta.overlap) wait_prior();
+  release_next();
+  if ((int)blockIdx.x < ta.ntail) {
+    drift_slots(P, ta.tail + blockIdx.x * blockDim.x + threadIdx.x, ta.ntail * blockDim.x, *ta.count, F, g, pc, err);
+    wait_prior();
+    return;
+  }
+  __shared__ real wn[WN];
+  const int tile = blockIdx.x - ta.ntail;
+  const TileGeom& t = ta.t;
+  const int tz = tile % t.ntz, ty = (tile / t.ntz) % t.nty, tx = tile / (t.ntz * t.nty);
+  const int wx0 = tx * kTileX, wy0 = ty * kTileY, wz0 = tz * kLanes;
+  for (int q = threadIdx.x; q < WN; q += blockDim.x) wn[q] = (real)0;
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int G = tile * (kTileX * kTileY) + warp;
+  const int base = ta.goff[G] + lane, jmax = ta.gtop[G];
+  int slots = 0;
+#pragma unroll
+  for (int w = 0; w < kTileX * kTileY; ++w) slots += ta.gtop[tile * (kTileX * kTileY) + w];
+  const real nscale = window_scale(pc.nw, slots);
+  // cells whose stencils lie in the window and the array
+  CellRange near;
+  near.lx = wx0 + 1;
+  near.ly = wy0 + 1;
+  near.lz = wz0 + 1;
+  near.ex = (unsigned)(min(wx0 + WX - 1, g.gx - 1) - near.lx);
+  near.ey = (unsigned)(min(wy0 + WY - 1, g.gy - 1) - near.ly);
+  near.ez = (unsigned)(min(wz0 + WZ - 1, g.gz - 1) - near.lz);
+  for (int r0 = 0; r0 < jmax; r0 += U) {
+    Rec<real> q[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      q[u].cell = -1;
+      if (r0 + u < jmax) q[u] = load_records(P, base + (r0 + u) * kLanes);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (q[u].cell < 0) continue;
+      int i, j, k;
+      unpack_cell(q[u].cell, i, j, k);
+      real fx = q[u].o[0], fy = q[u].o[1], fz = q[u].o[2];
+      advance(i, fx, q[u].v[0] * pc.hdt);
+      advance(j, fy, q[u].v[1] * pc.hdt);
+      advance(k, fz, q[u].v[2] * pc.hdt);
+      if (near.has(i, j, k)) {
+        const WinAxis<real> X = win_axis(fx, WY * WZ), Y = win_axis(fy, WZ), Z = win_axis(fz, 1);
+        add_density<WY, WZ>(wn + (((i - wx0) * WY + j - wy0) * WZ + k - wz0) + X.s + Y.s + Z.s, nscale, X, Y, Z);
+      } else {
+        drift_density(F, g, pc, i, j, k, fx, fy, fz, err);
+      }
+      store_position(P, base + (r0 + u) * kLanes, repack(i, j, k, err), fx, fy, fz);
+    }
+  }
+  __syncthreads();
+  constexpr int NZ4 = WZ / 4;
+  for (int q4 = threadIdx.x; q4 < WX * WY * NZ4; q4 += blockDim.x) {
+    const int a = q4 / (WY * NZ4), b = (q4 / NZ4) % WY, c4 = q4 % NZ4;
+    const int ga = wx0 + a, gb = wy0 + b, gc = wz0 + 4 * c4;
+    if (ga >= g.gx || gb >= g.gy || gc >= g.gz) continue;
+    flush_nodes<VEC>(F.f[pc.pn] + ga * g.sx + gb * g.gz + gc, g.gz - gc, window_density(wn + (a * WY + b) * WZ + 4 * c4, pc.nw, nscale));
+  }
+  wait_prior();
+}
 
 }  // namespace pb

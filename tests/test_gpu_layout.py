@@ -102,3 +102,44 @@ def test_particles_off_the_short_path(case):
     assert ra == rb and np.array_equal(ca, cb)
     for p in P:
         p.close()
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("n", [(9, 8, 33), (10, 9, 64)])
+def test_single_functions_over_the_layout(n, precision):
+    """The push and drift loops called by themselves on a sorted store with a
+    refill behind the layout, against the same calls in slot order. FP64: 1e-11
+    as above. FP32: a step's velocities differ by the square roots' and
+    divisions' roundings (2e-7 each, a few of them: 2e-6), the sums of 8 to 300
+    such terms by as much."""
+    rng = np.random.default_rng(n[0])
+    rows = [crowd(n, rng, 0.2) for _ in range(2)]
+    P = [context(n, precision, slot_order) for slot_order in (0, 1)]
+    for p in P:
+        for s in (ION, ELECTRON):
+            p.set_particles(s, rows[s])
+        p.sorting()
+        p.add_flat()
+        for step in range(2):
+            p.renew_grid()
+            p.renew_b4_2()
+            if step == 0:
+                p.push_deposit_j()
+            else:  # one species at a time, the second first
+                p.push_deposit_j(ELECTRON)
+                p.push_deposit_j(ION)
+            p.renew_b4_2()
+            p.drift_deposit_n()
+            p.reduce_current()
+            p.renew_e4_2()
+            p.sr_particle()
+    g, h = P[0].grid(), P[1].grid()
+    tol = 1e-11 if precision == 64 else 1e-5
+    for q in range(18):
+        assert rel_norm(g[..., q], h[..., q]) < tol or np.abs(g[..., q] - h[..., q]).max() < 1e-15
+    for s in (ION, ELECTRON):
+        assert P[0].particle_count(s) == P[1].particle_count(s)
+    (ra, ca), (rb, cb) = P[0].status(), P[1].status()
+    assert ra == rb == 0 and np.array_equal(ca, cb)
+    for p in P:
+        p.close()
