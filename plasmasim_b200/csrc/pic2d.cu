@@ -35,6 +35,7 @@
 #include "../../include/plasma_b200.h"
 #include "common.cuh"
 #include "particles.cuh"
+#include "sine_gemm.cuh"
 
 using namespace pb;
 
@@ -76,6 +77,7 @@ struct Run {
   unsigned long long seed_p, seed_v;
   int add_interval;
   int sz_dst;             // offset of the run's sine tables (Nx then Nz)
+  int ev;                 // offset of its sin^2 eigenvalue terms (Nx, then Nz)
   long long roff;         // offset of the run's Poisson buffers (nx * nz)
   // tiled layout: group (i, b) holds cells (i, 2 + 32 b + lane); the run's
   // groups are [gbase, gbase + ngroups), nx rows of nzb = ceil(nz / 32)
@@ -151,10 +153,14 @@ struct Item {
 
 // ------------------------------------------------------------ grid
 // Rows of one item of the field updates: a block of 256 threads takes
-// kFieldRows rows of a run, so that a thread updates several nodes per item.
+// kFieldRows rows of a run, so that a thread updates several nodes per item,
+// or one row where the batch has fewer items than the SMs hold blocks (two
+// updates of B and one of E took 37 us for 8 runs of 64 to 96 a side with four
+// rows an item; with one, and the other changes of this size to the small
+// kernels of a step, the step went from 0.229 to 0.164 ms).
 constexpr int kFieldRows = 4;
 
-// The nodes (k, m) of one item, k0 <= k < k0 + kFieldRows (and < nx + 2), 2 <=
+// The nodes (k, m) of one item, k0 <= k < k0 + rows (and < nx + 2), 2 <=
 // m < nz + 2, flattened over the block's threads and walked without a
 // division per node.
 struct NodeWalk {
@@ -185,12 +191,12 @@ __device__ __forceinline__ real d4(const real* f, int n, int d, real inv24dx) {
 }
 
 // renew_b4 (:1391-1417) on the interior of every run; item = (run, first row
-// k0) for rows k0 .. k0 + kFieldRows - 1, in the field's precision. Away from
+// k0) for rows k0 .. k0 + rows - 1, in the field's precision. Away from
 // the damping layers s = 0, where the two factors are exactly 1 and dt / 2
 // and are taken without their divisions.
 template <typename real>
 __global__ void __launch_bounds__(256) renew_b4_kernel(real* F, const Run<real>* __restrict__ runs,
-                                                       const Item* __restrict__ items, int nitems) {
+                                                       const Item* __restrict__ items, int nitems, int rows) {
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
     const Run<real>& R = runs[items[it].run];
     const int k0 = items[it].first;
@@ -211,7 +217,7 @@ __global__ void __launch_bounds__(256) renew_b4_kernel(real* F, const Run<real>*
     // (1 - s t) / (1 + s t) and dt / 2 / (1 + s t)
     auto ca = [&](double s) { return s == 0. ? (real)1 : (real)((1. - s * t) / (1. + s * t)); };
     auto cb = [&](double s) { return s == 0. ? hdt : (real)(0.5 * R.dt / (1. + s * t)); };
-    const int kend = min(k0 + kFieldRows, nx + 2);
+    const int kend = min(k0 + rows, nx + 2);
     for (NodeWalk w(k0, nz, threadIdx.x, blockDim.x); w.k < kend; w.next(nz)) {
       const int k = w.k, m = w.m;
       const int n = k * G + m;
@@ -237,7 +243,7 @@ __global__ void __launch_bounds__(256) renew_b4_kernel(real* F, const Run<real>*
 // there. dB = B - B0 on both sides of each difference.
 template <typename real>
 __global__ void __launch_bounds__(256) renew_e4_kernel(real* F, const Run<real>* __restrict__ runs,
-                                                       const Item* __restrict__ items, int nitems) {
+                                                       const Item* __restrict__ items, int nitems, int rows) {
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
     const Run<real>& R = runs[items[it].run];
     const int k0 = items[it].first;
@@ -273,7 +279,7 @@ __global__ void __launch_bounds__(256) renew_e4_kernel(real* F, const Run<real>*
       return s == 0. ? (real)1 : (real)((1. - h) / (1. + h));
     };
     auto cb = [&](double s) { return s == 0. ? rcc : (real)(cc / (1. + 0.5 * mu0 * s * cc)); };
-    const int kend = min(k0 + kFieldRows, nx + 2);
+    const int kend = min(k0 + rows, nx + 2);
     for (NodeWalk w(k0, nz, threadIdx.x, blockDim.x); w.k < kend; w.next(nz)) {
       const int k = w.k, m = w.m;
       const int n = k * G + m;
@@ -297,51 +303,29 @@ __global__ void __launch_bounds__(256) renew_e4_kernel(real* F, const Run<real>*
 }
 
 // sr_grid at size 1 (:1021-1071): columns 0,1 <- N, N+1 and N+2, N+3 <- 2, 3
-// of every plane (the whole Grid record); one block per run.
+// of every plane (the whole Grid record); one block per run and plane. The
+// step's last one counts the step as well (`step`).
 template <typename real>
-__global__ void sr_grid_kernel(real* F, const Run<real>* __restrict__ runs, int nruns) {
-  for (int r = blockIdx.x; r < nruns; r += gridDim.x) {
-    const Run<real> R = runs[r];
-    const int G = R.gz, N = R.nx;
-    for (int q = threadIdx.x; q < P_COUNT * G; q += blockDim.x) {
-      real* a = plane(F, R, q / G);
-      const int m = q % G;
-      const real v0 = a[N * G + m], v1 = a[(N + 1) * G + m], v2 = a[2 * G + m], v3 = a[3 * G + m];
-      a[m] = v0;
-      a[G + m] = v1;
-      a[(N + 2) * G + m] = v2;
-      a[(N + 3) * G + m] = v3;
-    }
+__global__ void __launch_bounds__(128) sr_grid_kernel(real* F, const Run<real>* __restrict__ runs, int* step) {
+  const Run<real>& R = runs[blockIdx.x];
+  const int G = R.gz, N = R.nx;
+  real* a = plane(F, R, blockIdx.y);
+  for (int m = threadIdx.x; m < G; m += blockDim.x) {
+    const real v0 = a[N * G + m], v1 = a[(N + 1) * G + m], v2 = a[2 * G + m], v3 = a[3 * G + m];
+    a[m] = v0;
+    a[G + m] = v1;
+    a[(N + 2) * G + m] = v2;
+    a[(N + 3) * G + m] = v3;
   }
-}
-
-// sr_current / sr_density at size 1 (:1073-1209): column 2 += column N+2,
-// column N+1 += column 1, for planes [p0, p0 + np).
-template <typename real>
-__global__ void fold_kernel(real* F, const Run<real>* __restrict__ runs, int nruns, int p0, int np) {
-  for (int r = blockIdx.x; r < nruns; r += gridDim.x) {
-    const Run<real> R = runs[r];
-    const int G = R.gz, N = R.nx;
-    for (int q = threadIdx.x; q < np * G; q += blockDim.x) {
-      real* a = plane(F, R, p0 + q / G);
-      const int m = q % G;
-      a[2 * G + m] += a[(N + 2) * G + m];
-      a[(N + 1) * G + m] += a[G + m];
-    }
-  }
+  if (step && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *step += 1;
 }
 
 // external_current_perp (:2238-2268) at rank p/2 = 0: the coil's two line
 // currents, ramped up over the first 10000 steps.
 template <typename real>
-__global__ void coil_kernel(real* F, const Run<real>* __restrict__ runs, int nruns, const int* __restrict__ step) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= nruns) return;
-  const Run<real> R = runs[r];
-  const int c = *step;
+__device__ __forceinline__ void coil_current(real* jiy, const Run<real>& R, int c) {
   const double Pi = 3.14159265358979323846;
   const double w = Pi / 10000.;
-  real* jiy = plane(F, R, P_JIY);
   const int G = R.gz;
   const int lo = 3 * G + (R.nz + 4) / 2 - 3, hi = 3 * G + (R.nz + 4) / 2 + 2;
   if (c < 10000) {
@@ -353,19 +337,34 @@ __global__ void coil_kernel(real* F, const Run<real>* __restrict__ runs, int nru
   }
 }
 
-// renew_grid (:1348-1389): J, n and phi of every run to zero (the last nine
-// planes of each run's block); one block per run.
+// sr_current / sr_density at size 1 (:1073-1209): column 2 += column N+2,
+// column N+1 += column 1, for planes p0 + blockIdx.y, one block per run and
+// plane; with `step` (the current's planes), external_current_perp after it.
 template <typename real>
-__global__ void zero_sources_kernel(real* F, const Run<real>* __restrict__ runs, int nruns) {
-  for (int r = blockIdx.x; r < nruns; r += gridDim.x) {
-    const Run<real> R = runs[r];
-    real* base = F + R.foff + (long long)P_JIX * R.nodes;
-    const long long n = (long long)(P_COUNT - P_JIX) * R.nodes;
-    for (long long q = threadIdx.x; q < n; q += blockDim.x) base[q] = (real)0;
+__global__ void __launch_bounds__(128) fold_kernel(real* F, const Run<real>* __restrict__ runs, int p0,
+                                                   const int* step) {
+  const Run<real>& R = runs[blockIdx.x];
+  const int G = R.gz, N = R.nx, p = p0 + blockIdx.y;
+  real* a = plane(F, R, p);
+  for (int m = threadIdx.x; m < G; m += blockDim.x) {
+    a[2 * G + m] += a[(N + 2) * G + m];
+    a[(N + 1) * G + m] += a[G + m];
+  }
+  if (step && p == P_JIY) {
+    __syncthreads();  // the coil's column may be one of the fold's
+    if (threadIdx.x == 0) coil_current(a, R, *step);
   }
 }
 
-__global__ void step_advance_kernel(int* step) { *step += 1; }
+// renew_grid (:1348-1389): J, n and phi of every run to zero (the last nine
+// planes of each run's block), gridDim.y blocks per run.
+template <typename real>
+__global__ void __launch_bounds__(256) zero_sources_kernel(real* F, const Run<real>* __restrict__ runs) {
+  const Run<real>& R = runs[blockIdx.x];
+  real* base = F + R.foff + (long long)P_JIX * R.nodes;
+  const int n = (P_COUNT - P_JIX) * R.nodes;
+  for (int q = blockIdx.y * blockDim.x + threadIdx.x; q < n; q += gridDim.y * blockDim.x) base[q] = (real)0;
+}
 
 // ------------------------------------------------------------ particles
 // Bilinear weights of one axis in cell units (shape_func_*3, :1948-2016):
@@ -1034,107 +1033,67 @@ __global__ void phi_rho_kernel(real* F, const Run<real>* __restrict__ runs, cons
 }
 
 // Batched small GEMM C = alpha * op(A B) over every run (row-major, the run's
-// sizes): 64x64 output tiles, 256 threads of 4x4 outputs each (4 consecutive
-// rows by 4 consecutive columns, read from the staged tiles as 4-wide vector
-// loads), K staged through shared memory 32 at a time, both tiles k-major. mode selects the operands of the four
-// sine transforms:
+// sizes), T x T output tiles (sine_gemm.cuh). mode selects the operands of the
+// four sine transforms:
 //  0: C[nx][nz] = A[nx][nz] * S_nz        (transform along z)
 //  1: C[nx][nz] = S_nx * A[nx][nz], then / eigenvalue  (along x, solve)
 //  2: C[nx][nz] = (2/nx) S_nx * A          (inverse along x)
 //  3: C[nx][nz] = (2/nz) A * S_nz          (inverse along z)
 // S_n[i][j] = sin(pi i j / n); its row and column 0 vanish, so the transforms
 // skip the first element as the reference's sinft does (y[1] = 0, :2902).
-constexpr int kGemmTile = 64;
-__device__ __forceinline__ void ld4(const float* p, float (&v)[4]) {
-  const float4 q = *reinterpret_cast<const float4*>(p);
-  v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
-}
-__device__ __forceinline__ void ld4(const double* p, double (&v)[4]) {
-  const double2 q0 = reinterpret_cast<const double2*>(p)[0], q1 = reinterpret_cast<const double2*>(p)[1];
-  v[0] = q0.x; v[1] = q0.y; v[2] = q1.x; v[3] = q1.y;
-}
-template <typename real>
+// sin2 holds sin^2(pi i / 2 n), the terms of renew_phi's eigenvalues (:2680-2690).
+constexpr int kGemmTile = 64, kGemmSmall = 32;
+template <typename real, int T>
 __global__ void __launch_bounds__(256) dst_gemm_kernel(const Run<real>* __restrict__ runs, const Item* __restrict__ items,
                                                        int nitems, const real* __restrict__ A, real* C,
-                                                       const real* __restrict__ sines, int mode) {
-  constexpr int T = kGemmTile, KT = 32;
-  __shared__ __align__(16) real As[KT][T + 4];  // [k][row of C]
-  __shared__ __align__(16) real Bs[KT][T + 4];  // [k][col of C]
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;  // 16 x 16; outputs (4 ty + u, 4 tx + v)
+                                                       const real* __restrict__ sines, const double* __restrict__ sin2,
+                                                       int mode) {
+  constexpr int U = T / 16;
+  __shared__ __align__(16) GemmStage<real, T> stage;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
     const Run<real>& R = runs[items[it].run];
     const int nx = R.nx, nz = R.nz;
     const int tiles_n = (nz + T - 1) / T;
-    const int ti = items[it].first / tiles_n, tj = items[it].first % tiles_n;
+    const int row0 = items[it].first / tiles_n * T, col0 = items[it].first % tiles_n * T;
     const real* a = A + R.roff;
     real* cmat = C + R.roff;
     const real* Sx = sines + R.sz_dst;
     const real* Sz = sines + R.sz_dst + (long long)nx * nx;
-    const bool left = mode == 1 || mode == 2;  // S * A (K = nx) or A * S (K = nz)
-    const int K = left ? nx : nz;
-    real acc[4][4];
+    real acc[U][U];
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+    for (int u = 0; u < U; ++u)
 #pragma unroll
-      for (int v = 0; v < 4; ++v) acc[u][v] = 0;
-    for (int k0 = 0; k0 < K; k0 += KT) {
-      __syncthreads();  // the last tile's reads are done
-      // left operand tile [T rows of C][KT of K], right operand tile [KT of K][T cols of C]
-      for (int q = threadIdx.x; q < T * KT; q += blockDim.x) {
-        // left: a warp takes 4 rows x 8 consecutive k (coalesced reads; its
-        // transposed stores fall on 32 different banks)
-        const int ch = q >> 5, l = q & 31;
-        const int r = 4 * (ch % (T / 4)) + (l >> 3), kc = 8 * (ch / (T / 4)) + (l & 7);
-        const int row = ti * T + r, kk = k0 + kc;
-        real lv = 0;
-        if (left) {
-          if (row < nx && kk < nx) lv = Sx[(long long)row * nx + kk];
-        } else {
-          if (row < nx && kk < nz) lv = a[(long long)row * nz + kk];
-        }
-        As[kc][r] = lv;
-        const int kr = q / T, cc = q % T;  // right: row k0 + kr, column cc
-        const int krow = k0 + kr, col = tj * T + cc;
-        real rv = 0;
-        if (left) {
-          if (krow < nx && col < nz) rv = a[(long long)krow * nz + col];
-        } else {
-          if (krow < nz && col < nz) rv = Sz[(long long)krow * nz + col];
-        }
-        Bs[kr][cc] = rv;
-      }
-      __syncthreads();
-#pragma unroll 8
-      for (int kk = 0; kk < KT; ++kk) {
-        real av[4], bv[4];
-        ld4(&As[kk][4 * ty], av);
-        ld4(&Bs[kk][4 * tx], bv);
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-          for (int v = 0; v < 4; ++v) acc[u][v] += av[u] * bv[v];
-      }
+      for (int v = 0; v < U; ++v) acc[u][v] = 0;
+    const auto element = [&](const real* m, int rows, int cols, int r, int c) {
+      return r < rows && c < cols ? m[(long long)r * cols + c] : (real)0;
+    };
+    if (mode == 1 || mode == 2) {  // S * A
+      gemm_tile<real, T>(stage, nx, [&](int r, int k) { return element(Sx, nx, nx, row0 + r, k); },
+                         [&](int k, int c) { return element(a, nx, nz, k, col0 + c); }, acc);
+    } else {  // A * S
+      gemm_tile<real, T>(stage, nz, [&](int r, int k) { return element(a, nx, nz, row0 + r, k); },
+                         [&](int k, int c) { return element(Sz, nz, nz, k, col0 + c); }, acc);
     }
-    const double Pi = 3.14159265358979323846;
+    const double inv = mode == 2 ? 2. / nx : 2. / nz, h2 = (R.dx / 2.) * (R.dx / 2.);
+    const double* ex = sin2 + R.ev;
+    const double* ez = ex + nx;
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+    for (int u = 0; u < U; ++u)
 #pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        const int row = ti * T + 4 * ty + u, col = tj * T + 4 * tx + v;
+      for (int v = 0; v < U; ++v) {
+        const int row = row0 + U * ty + u, col = col0 + U * tx + v;
         if (row >= nx || col >= nz) continue;
         real w = acc[u][v];
-        if (mode == 1) {
-          // renew_phi's eigenvalue (:2680-2690): row = x wave number, col = z wave number
-          const double sz = sin(Pi * (double)col / (double)nz / 2.), sx = sin(Pi * (double)row / (double)nx / 2.);
-          const double Aev = -(sz * sz + sx * sx) / ((R.dx / 2.) * (R.dx / 2.));
-          w = Aev == 0. ? (real)0 : (real)((double)w / Aev);
-        } else if (mode == 2) {
-          w = (real)(2. * (double)w / nx);
-        } else if (mode == 3) {
-          w = (real)(2. * (double)w / nz);
+        if (mode == 1) {  // row = x wave number, col = z wave number
+          const double e = -(ez[col] + ex[row]) / h2;
+          w = e == 0. ? (real)0 : (real)((double)w / e);
+        } else if (mode >= 2) {
+          w = (real)(inv * (double)w);
         }
         cmat[(long long)row * nz + col] = w;
       }
+    __syncthreads();  // the next tile's stage may be written
   }
 }
 
@@ -1286,6 +1245,11 @@ struct pic2d_batch {
   int cur = 0;
   long long pool_slots = 0;
   void* sines = nullptr;
+  double* stage = nullptr;  // a grid's records on their way to the host
+  size_t stage_bytes = 0;
+  double* sin2 = nullptr;  // per run: sin^2(pi i / 2 n) of Nx, then of Nz
+  int gemm_tile = 64;      // output tile of the sine transforms
+  int field_rows = 4;      // rows per item of the field updates
   void* rho = nullptr;
   void* rho2 = nullptr;
   long long rho_len = 0;
@@ -1833,8 +1797,8 @@ int cellsort(pic2d_batch* b) {
 }
 
 template <typename real>
-int sr_grid(pic2d_batch* b) {
-  sr_grid_kernel<real><<<persistent(b->nruns), 256, 0, b->stream>>>((real*)b->field, runs_of<real>(b), b->nruns);
+int sr_grid(pic2d_batch* b, int* step = nullptr) {
+  sr_grid_kernel<real><<<dim3(b->nruns, P_COUNT), 128, 0, b->stream>>>((real*)b->field, runs_of<real>(b), step);
   CKL2();
   return PIC_OK;
 }
@@ -1847,13 +1811,14 @@ int renew_phi(pic2d_batch* b) {
   phi_rho_kernel<real><<<persistent(b->n_rhorow), 128, 0, b->stream>>>((real*)b->field, R, b->rho_items, b->n_rhorow, rho);
   CKL2();
   const real* S = (const real*)b->sines;
-  dst_gemm_kernel<real><<<persistent(b->n_tile), 256, 0, b->stream>>>(R, b->tile_items, b->n_tile, rho, tmp, S, 0);
+  const auto gemm = b->gemm_tile == kGemmTile ? dst_gemm_kernel<real, kGemmTile> : dst_gemm_kernel<real, kGemmSmall>;
+  gemm<<<persistent(b->n_tile), 256, 0, b->stream>>>(R, b->tile_items, b->n_tile, rho, tmp, S, b->sin2, 0);
   CKL2();
-  dst_gemm_kernel<real><<<persistent(b->n_tile), 256, 0, b->stream>>>(R, b->tile_items, b->n_tile, tmp, rho, S, 1);
+  gemm<<<persistent(b->n_tile), 256, 0, b->stream>>>(R, b->tile_items, b->n_tile, tmp, rho, S, b->sin2, 1);
   CKL2();
-  dst_gemm_kernel<real><<<persistent(b->n_tile), 256, 0, b->stream>>>(R, b->tile_items, b->n_tile, rho, tmp, S, 2);
+  gemm<<<persistent(b->n_tile), 256, 0, b->stream>>>(R, b->tile_items, b->n_tile, rho, tmp, S, b->sin2, 2);
   CKL2();
-  dst_gemm_kernel<real><<<persistent(b->n_tile), 256, 0, b->stream>>>(R, b->tile_items, b->n_tile, tmp, rho, S, 3);
+  gemm<<<persistent(b->n_tile), 256, 0, b->stream>>>(R, b->tile_items, b->n_tile, tmp, rho, S, b->sin2, 3);
   CKL2();
   phi_apply_kernel<real><<<persistent(b->n_rhorow), 128, 0, b->stream>>>((real*)b->field, R, b->rho_items, b->n_rhorow, rho);
   CKL2();
@@ -1904,7 +1869,8 @@ int set_tiles(pic2d_batch* b, int tx) {
 // Zero J, n and phi of every run (renew_grid, :1348-1389).
 template <typename real>
 int renew_grid(pic2d_batch* b) {
-  zero_sources_kernel<real><<<persistent(b->nruns), 256, 0, b->stream>>>((real*)b->field, runs_of<real>(b), b->nruns);
+  zero_sources_kernel<real><<<dim3(b->nruns, std::max(4, 148 * 8 / b->nruns)), 256, 0, b->stream>>>((real*)b->field,
+                                                                                               runs_of<real>(b));
   CKL2();
   return PIC_OK;
 }
@@ -1924,26 +1890,22 @@ int step_body(pic2d_batch* b, bool refill, bool sort = false) {
   } else if (sort) {
     CKR2(cellsort<real>(b));
   }
-  renew_b4_kernel<real><<<persistent(b->n_row), 256, 0, b->stream>>>(F, R, b->row_items, b->n_row);
+  renew_b4_kernel<real><<<persistent(b->n_row), 256, 0, b->stream>>>(F, R, b->row_items, b->n_row, b->field_rows);
   CKL2();
   CKR2(sr_grid<real>(b));
   CKR2(push<real>(b));
-  fold_kernel<real><<<persistent(b->nruns), 256, 0, b->stream>>>(F, R, b->nruns, P_JIX, 6);
+  fold_kernel<real><<<dim3(b->nruns, 6), 128, 0, b->stream>>>(F, R, P_JIX, b->step_dev);
   CKL2();
-  fold_kernel<real><<<persistent(b->nruns), 256, 0, b->stream>>>(F, R, b->nruns, P_NI, 2);
+  fold_kernel<real><<<dim3(b->nruns, 2), 128, 0, b->stream>>>(F, R, P_NI, nullptr);
   CKL2();
-  coil_kernel<real><<<(b->nruns + 127) / 128, 128, 0, b->stream>>>(F, R, b->nruns, b->step_dev);
-  CKL2();
-  renew_b4_kernel<real><<<persistent(b->n_row), 256, 0, b->stream>>>(F, R, b->row_items, b->n_row);
+  renew_b4_kernel<real><<<persistent(b->n_row), 256, 0, b->stream>>>(F, R, b->row_items, b->n_row, b->field_rows);
   CKL2();
   CKR2(sr_grid<real>(b));
-  renew_e4_kernel<real><<<persistent(b->n_row), 256, 0, b->stream>>>(F, R, b->row_items, b->n_row);
+  renew_e4_kernel<real><<<persistent(b->n_row), 256, 0, b->stream>>>(F, R, b->row_items, b->n_row, b->field_rows);
   CKL2();
   CKR2(sr_grid<real>(b));
   CKR2(renew_phi<real>(b));
-  CKR2(sr_grid<real>(b));
-  step_advance_kernel<<<1, 1, 0, b->stream>>>(b->step_dev);
-  CKL2();
+  CKR2(sr_grid<real>(b, b->step_dev));  // and the step counted
   return PIC_OK;
 }
 
@@ -2046,7 +2008,7 @@ int do_init(pic2d_batch* b) {
   density2d_kernel<real><<<persistent(b->n_part), 256, 0, b->stream>>>(b->pool[b->cur], F, R, b->st, b->part_items,
                                                                         b->n_part, kChunk);
   CKL2();
-  fold_kernel<real><<<persistent(b->nruns), 256, 0, b->stream>>>(F, R, b->nruns, P_NI, 2);
+  fold_kernel<real><<<dim3(b->nruns, 2), 128, 0, b->stream>>>(F, R, P_NI, nullptr);
   CKL2();
   CKR2(sr_grid<real>(b));
   CK2(cudaMemsetAsync(b->step_dev, 0, sizeof(int), b->stream));
@@ -2066,8 +2028,7 @@ int do_create(pic2d_batch* b) {
   b->runs_host.assign(sizeof(Run<real>) * n, 0);
   Run<real>* H = runs_host<real>(b);
   long long foff = 0, poff = 0, roff = 0;
-  int ngroups = 0;
-  std::vector<int> sine_sizes;
+  int ngroups = 0, ev = 0;
   std::vector<std::pair<int, long long>> sine_off;  // size -> offset
   std::vector<double> sines;
   auto sine_table = [&](int m) -> long long {
@@ -2118,6 +2079,8 @@ int do_create(pic2d_batch* b) {
     R.seed_v = k.seed_v;
     R.add_interval = k.add_interval;
     R.sz_dst = 0;
+    R.ev = ev;
+    ev += k.nx + k.nz;
     R.roff = roff;
     roff += (long long)k.nx * k.nz;
     const long long sx = sine_table(k.nx);
@@ -2170,13 +2133,32 @@ int do_create(pic2d_batch* b) {
   CK2(cudaMalloc(&b->rho, sizeof(real) * (size_t)roff));
   CK2(cudaMalloc(&b->rho2, sizeof(real) * (size_t)roff));
   // work lists
+  // a small batch takes smaller items, so that every SM has some
+  long long big = 0, cells = 0;
+  std::vector<double> sin2;
+  for (int r = 0; r < n; ++r) {
+    big += (long long)((H[r].nz + kGemmTile - 1) / kGemmTile) * ((H[r].nx + kGemmTile - 1) / kGemmTile);
+    cells += H[r].nx;
+  }
+  for (int r = 0; r < n; ++r)
+    for (int axis = 0; axis < 2; ++axis) {
+      const int m = axis == 0 ? H[r].nx : H[r].nz;
+      for (int i = 0; i < m; ++i) {
+        const double s = std::sin(3.14159265358979323846 * (double)i / (double)m / 2.);
+        sin2.push_back(s * s);
+      }
+    }
+  CK2(cudaMalloc(&b->sin2, sizeof(double) * std::max<size_t>(sin2.size(), 1)));
+  CK2(cudaMemcpy(b->sin2, sin2.data(), sizeof(double) * sin2.size(), cudaMemcpyHostToDevice));
+  b->gemm_tile = big >= 148 * 2 ? kGemmTile : kGemmSmall;
+  b->field_rows = cells >= 148LL * 8 * kFieldRows ? kFieldRows : 1;
   std::vector<Item> rows, rhos, parts, tiles;
   for (int r = 0; r < n; ++r) {
-    for (int k = 2; k < H[r].nx + 2; k += kFieldRows) rows.push_back({r, k});
+    for (int k = 2; k < H[r].nx + 2; k += b->field_rows) rows.push_back({r, k});
     for (int k = 0; k < H[r].nx; ++k) rhos.push_back({r, k});
     for (int s = 0; s < 2; ++s)
       for (long long q = 0; q < H[r].cap; q += kChunk) parts.push_back({2 * r + s, (int)q});
-    const int tn = (H[r].nz + kGemmTile - 1) / kGemmTile, tm = (H[r].nx + kGemmTile - 1) / kGemmTile;
+    const int T = b->gemm_tile, tn = (H[r].nz + T - 1) / T, tm = (H[r].nx + T - 1) / T;
     for (int t = 0; t < tn * tm; ++t) tiles.push_back({r, t});
   }
   auto upload = [&](const std::vector<Item>& v, Item** dst, int* cnt) -> int {
@@ -2227,7 +2209,7 @@ void free_batch(pic2d_batch* b) {
       for (int a = 0; a < 2; ++a) cudaFree(b->pool[p].o[s][a]);
       for (int a = 0; a < 3; ++a) cudaFree(b->pool[p].v[s][a]);
     }
-  cudaFree(b->sines); cudaFree(b->rho); cudaFree(b->rho2);
+  cudaFree(b->sines); cudaFree(b->sin2); cudaFree(b->stage); cudaFree(b->rho); cudaFree(b->rho2);
   cudaFree(b->row_items); cudaFree(b->rho_items); cudaFree(b->part_items); cudaFree(b->tile_items);
   for (int w = 0; w < 2; ++w)
     for (int s = 0; s < 2; ++s) { cudaFree(b->src_items[w][s]); cudaFree(b->sets[w][s]); }
@@ -2291,13 +2273,17 @@ int do_get_particles(pic2d_batch* b, int run, int s, double* rows, long long cap
 template <typename real>
 int do_get_grid(pic2d_batch* b, int run, double* rec) {
   const Run<real>& R = runs_host<real>(b)[run];
-  double* dev = nullptr;
-  CK2(cudaMalloc(&dev, sizeof(double) * 18 * (size_t)R.nodes));
-  grid2d_export_kernel<real><<<(R.nodes + 255) / 256, 256, 0, b->stream>>>((const real*)b->field, R, dev);
-  cudaError_t e = cudaMemcpyAsync(rec, dev, sizeof(double) * 18 * (size_t)R.nodes, cudaMemcpyDeviceToHost, b->stream);
-  cudaStreamSynchronize(b->stream);
-  cudaFree(dev);
-  CK2(e);
+  const size_t bytes = sizeof(double) * 18 * (size_t)R.nodes;
+  if (bytes > b->stage_bytes) {  // kept for the next call; a run's grid is the largest it grows to
+    cudaFree(b->stage);
+    b->stage = nullptr;
+    b->stage_bytes = 0;
+    CK2(cudaMalloc(&b->stage, bytes));
+    b->stage_bytes = bytes;
+  }
+  grid2d_export_kernel<real><<<(R.nodes + 255) / 256, 256, 0, b->stream>>>((const real*)b->field, R, b->stage);
+  CK2(cudaMemcpyAsync(rec, b->stage, bytes, cudaMemcpyDeviceToHost, b->stream));
+  CK2(cudaStreamSynchronize(b->stream));
   CK2(cudaGetLastError());
   return PIC_OK;
 }

@@ -17,6 +17,7 @@
 
 #include "common.cuh"
 #include "fields.cuh"
+#include "sine_gemm.cuh"
 
 namespace pb {
 
@@ -68,61 +69,39 @@ struct DstGemm {
   double h2;           // (dx/2)^2
 };
 
-constexpr int kDstTile = 64, kDstK = 16;
+constexpr int kDstTile = 64;
 
 template <typename real>
 __global__ void __launch_bounds__(256) dst3_gemm_kernel(DstGemm<real> a) {
-  __shared__ real Ls[kDstK][kDstTile + 1];
-  __shared__ real Rs[kDstK][kDstTile + 1];
-  const int tiles_m = (a.M + kDstTile - 1) / kDstTile, tiles_n = (a.N + kDstTile - 1) / kDstTile;
+  constexpr int T = kDstTile, U = T / 16;
+  __shared__ __align__(16) GemmStage<real, T> stage;
+  const int tiles_m = (a.M + T - 1) / T, tiles_n = (a.N + T - 1) / T;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   for (long long blk = blockIdx.x; blk < (long long)tiles_m * tiles_n * a.B; blk += gridDim.x) {
     const int b = (int)(blk / ((long long)tiles_m * tiles_n));
     const int r = (int)(blk % ((long long)tiles_m * tiles_n));
-    const int m0 = (r / tiles_n) * kDstTile, n0 = (r % tiles_n) * kDstTile;
+    const int m0 = (r / tiles_n) * T, n0 = (r % tiles_n) * T;
     const real* L = a.L + b * a.lb;
     const real* R = a.R + b * a.rb;
-    real acc[4][4];
+    real acc[U][U];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < U; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = (real)0;
-    for (int k0 = 0; k0 < a.K; k0 += kDstK) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int e = threadIdx.x + 256 * q;
-        const int lmi = e / kDstK, lki = e % kDstK;  // L tile: 64 rows x 16 k
-        const int gm = m0 + lmi, gk = k0 + lki;
-        Ls[lki][lmi] = (gm < a.M && gk < a.K) ? L[gm * a.lm + gk] : (real)0;
-        const int rki = e / kDstTile, rni = e % kDstTile;  // R tile: 16 k x 64 cols
-        const int gk2 = k0 + rki, gn = n0 + rni;
-        Rs[rki][rni] = (gk2 < a.K && gn < a.N) ? R[gk2 * a.rk + gn] : (real)0;
-      }
-      __syncthreads();
-#pragma unroll
-      for (int kk = 0; kk < kDstK; ++kk) {
-        real lv[4], rv[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) lv[i] = Ls[kk][ty + 16 * i];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) rv[j] = Rs[kk][tx + 16 * j];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) acc[i][j] += lv[i] * rv[j];
-      }
-      __syncthreads();
-    }
+      for (int j = 0; j < U; ++j) acc[i][j] = (real)0;
+    gemm_tile<real, T>(
+        stage, a.K, [&](int m, int k) { return m0 + m < a.M && k < a.K ? L[(m0 + m) * a.lm + k] : (real)0; },
+        [&](int k, int n) { return k < a.K && n0 + n < a.N ? R[k * a.rk + n0 + n] : (real)0; }, acc);
     real* C = a.C + b * a.cb;
+    const double scale = a.mul / a.div;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int gm = m0 + ty + 16 * i;
+    for (int i = 0; i < U; ++i) {
+      const int gm = m0 + U * ty + i;
       if (gm >= a.M) continue;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int gn = n0 + tx + 16 * j;
+      for (int j = 0; j < U; ++j) {
+        const int gn = n0 + U * tx + j;
         if (gn >= a.N) continue;
-        double v = a.mul * (double)acc[i][j] / a.div;
+        double v = scale * (double)acc[i][j];
         if (a.solve) {
           const int kx = gm, ky = gn / a.nz, kz = gn % a.nz;
           const double ev = -(a.sin2[a.nx + ky] + a.sin2[a.nx + a.ny + kz] + a.sin2[kx]) / a.h2;
@@ -131,6 +110,7 @@ __global__ void __launch_bounds__(256) dst3_gemm_kernel(DstGemm<real> a) {
         C[gm * a.cm + gn] = (real)v;
       }
     }
+    __syncthreads();  // the next tile's stage may be written
   }
 }
 
