@@ -214,16 +214,29 @@ __global__ void __launch_bounds__(256, sizeof(real) == 4 ? 3 : 2) classify_kerne
   const int np = pend.n[lane];
 #pragma unroll
   for (int q = 0; q < kPending; ++q) {
-    int d = append(q < np);
-    if (d < 0) continue;
-    const Rec<real> p = get_record(pend.a[q][lane], pend.b[q][lane]);
-    if (d >= cap) {  // no room there: into one of the lane's holes, wherever that is
-      *nonhome = 1;
-      d = base + nexth * kLanes + lane;
-      top = max(top, nexth + 1);
-      if (++hu < nh) nexth = holes[base + hu * kLanes + lane];
+    const int d = append(q < np);
+    const bool full = d >= cap;
+    if (full) *nonhome = 1;
+    if (d >= 0 && !full) {
+      const Rec<real> p = get_record(pend.a[q][lane], pend.b[q][lane]);
+      store_records(P, d, p.cell, p.o[0], p.o[1], p.o[2], p.v[0], p.v[1], p.v[2]);
     }
-    store_records(P, d, p.cell, p.o[0], p.o[1], p.o[2], p.v[0], p.v[1], p.v[2]);
+    // No room there: into the holes that are left in any lane. Every pending
+    // particle left a hole in the group and every filled hole took one, so
+    // there are as many holes as particles.
+    for (unsigned left = __ballot_sync(0xffffffffu, full); left;) {  // warp-uniform
+      const unsigned open = __ballot_sync(0xffffffffu, hu < nh);
+      if (!open) break;
+      int from = -1;
+      for (unsigned o = open; o && left; o &= o - 1, left &= left - 1)
+        if (lane == __ffs(o) - 1) from = __ffs(left) - 1;
+      if (from >= 0) {
+        const Rec<real> p = get_record(pend.a[q][from], pend.b[q][from]);
+        store_records(P, base + nexth * kLanes + lane, p.cell, p.o[0], p.o[1], p.o[2], p.v[0], p.v[1], p.v[2]);
+        top = max(top, nexth + 1);
+        if (++hu < nh) nexth = holes[base + hu * kLanes + lane];
+      }
+    }
   }
   for (int q = used + lane; q < kAppendBlock; q += kLanes)
     if (blk + q < cap && used < kAppendBlock) P.cell[blk + q] = -1;

@@ -5,7 +5,7 @@ rows between two full sorts."""
 import numpy as np
 import pytest
 
-from plasmasim_b200 import ELECTRON, ION, Pic3D, PicConfig
+from plasmasim_b200 import ELECTRON, ION, Pic3D, PicConfig, PicError
 from util import rel_norm
 
 pytestmark = pytest.mark.gpu
@@ -143,3 +143,47 @@ def test_single_functions_over_the_layout(n, precision):
     assert ra == rb == 0 and np.array_equal(ca, cb)
     for p in P:
         p.close()
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+def test_hand_over_without_append_slots(precision):
+    """Particles that change lanes while the buffer ends with the layout: a
+    crowd moves into a cell whose lane has fewer holes than arrivals, and no
+    slot is left outside the layout. None may be lost or changed against the
+    slot-order push (the sorted columns: three steps round values and sums of
+    order 1 a few times, 1e-6 in FP32; particles lie 0.01 apart)."""
+    n, ppc, weight = (8, 8, 64), 4, 0.01 / 4
+    cells = np.stack(np.meshgrid(*[np.arange(2, m - 2) for m in n], indexing="ij"), -1).reshape(-1, 1, 3)
+    xyz = 2 + np.broadcast_to(cells + 0.5, (len(cells), ppc, 3)) + np.linspace(-0.04, 0.04, ppc)[:, None]
+    z = np.broadcast_to(cells[..., 2] % 32, xyz.shape[:2])
+    xyz[..., 2] += 0.4 * np.sign(16 - z)  # about to leave
+    v = np.zeros(xyz.shape)
+    v[..., 2] = np.where(z < 16, 0.7, np.where(z > 16, -0.7, 0.0))  # towards the group's 17th cell
+    rows = np.concatenate([xyz, v, np.full(xyz.shape[:2] + (1,), weight)], -1).reshape(-1, 7)
+    cfg = dict(precision=precision, diag_every_step=0, sort_interval=1, add_interval=1000)
+
+    def load(capacity, slot_order=0):
+        P = Pic3D(PicConfig.normalized(*n, 4, capacity=capacity, slot_order=slot_order, **cfg))
+        P.init_grid()
+        for s in (ION, ELECTRON):
+            P.set_particles(s, rows)
+        return P
+
+    low, high = len(rows), 200000  # high: a capacity that holds the layout
+    while low < high:
+        mid = (low + high) // 2
+        with load(mid) as P:
+            try:
+                P.sorting()
+                high = mid
+            except PicError:
+                low = mid + 1
+    with load(high) as T, load(high, 1) as S:
+        T.sorting()
+        for _ in range(3):
+            T.step(1)
+            S.step(1)
+            for s in (ION, ELECTRON):
+                a, b = (np.sort(P.particles(s), axis=0) for P in (T, S))
+                assert len(a) == len(b) == len(rows)
+                assert np.abs(a - b).max() < 1e-4
