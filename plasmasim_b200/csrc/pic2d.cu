@@ -394,47 +394,71 @@ __device__ __forceinline__ real bil(const real* P, int G, int i, int k, real x0,
          (P[i * G + k + 1] * (x0 * z1) + P[(i + 1) * G + k + 1] * (x1 * z1));
 }
 
+// Weights along one axis of a particle at offset f of an interior cell (so
+// never cell 0), and the step from the cell's node to the half-shifted base.
+template <typename real>
+struct WinAxis2 {
+  real a0, a1, b0, b1;
+  int s;
+};
+template <typename real>
+__device__ __forceinline__ WinAxis2<real> win_axis2(real f, int stride) {
+  WinAxis2<real> w;
+  const bool up = f >= (real)0.5;
+  w.a1 = f;
+  w.a0 = (real)1 - f;
+  w.b1 = f + (up ? (real)-0.5 : (real)0.5);
+  w.b0 = (real)1 - w.b1;
+  w.s = up ? 0 : -stride;
+  return w;
+}
+
 // E and B at a particle from a window of one plane per component (ex ey ez
-// bx by bz, WN nodes each, z rows of WZ nodes; window coordinates of the
-// stencil bases): bil's arithmetic in FP64. In FP32 the two x nodes of each
-// stencil row travel as one packed pair through two-wide multiplies and FMAs
-// (0.2 ms per step off the 256-run batch against bil's scalar form).
+// bx by bz, WN nodes each, z rows of WZ nodes), n the window node of its cell:
+// bil's arithmetic in FP64. In FP32 the two x nodes of each stencil row travel
+// as one packed pair through two-wide multiplies and FMAs (0.2 ms per step off
+// the 256-run batch against bil's scalar form).
 template <typename real>
 struct EB2 {
   real ex, ey, ez, bx, by, bz;
 };
-template <int WZ, int WN>
-__device__ __forceinline__ EB2<double> gather_win2(const double* fw, int xa, int xb, int za, int zb,
-                                                   const Ax2<double>& X, const Ax2<double>& Z) {
-  EB2<double> r;
-  r.ex = bil(fw + 0 * WN, WZ, xa, zb, X.a0, X.a1, Z.b0, Z.b1);
-  r.ey = bil(fw + 1 * WN, WZ, xb, zb, X.b0, X.b1, Z.b0, Z.b1);
-  r.ez = bil(fw + 2 * WN, WZ, xb, za, X.b0, X.b1, Z.a0, Z.a1);
-  r.bx = bil(fw + 3 * WN, WZ, xb, za, X.b0, X.b1, Z.a0, Z.a1);
-  r.by = bil(fw + 4 * WN, WZ, xa, za, X.a0, X.a1, Z.a0, Z.a1);
-  r.bz = bil(fw + 5 * WN, WZ, xa, zb, X.a0, X.a1, Z.b0, Z.b1);
-  return r;
+template <int WZ>
+__device__ __forceinline__ double bil_win(const double* P, double x0, double x1, double z0, double z1) {
+  return (P[0] * (x0 * z0) + P[WZ] * (x1 * z0)) + (P[1] * (x0 * z1) + P[WZ + 1] * (x1 * z1));
 }
 template <int WZ>
-__device__ __forceinline__ float bil_pair(const float* P, int i, int k, float x0, float x1, float2 Z0, float2 Z1) {
-  const float2 n0 = make_float2(P[i * WZ + k], P[(i + 1) * WZ + k]);
-  const float2 n1 = make_float2(P[i * WZ + k + 1], P[(i + 1) * WZ + k + 1]);
-  const float2 cz = __ffma2_rn(n1, Z1, __fmul2_rn(n0, Z0));
+__device__ __forceinline__ float bil_win(const float* P, float x0, float x1, float z0, float z1) {
+  const float2 n0 = make_float2(P[0], P[WZ]), n1 = make_float2(P[1], P[WZ + 1]);
+  const float2 cz = __ffma2_rn(n1, make_float2(z1, z1), __fmul2_rn(n0, make_float2(z0, z0)));
   return cz.x * x0 + cz.y * x1;
 }
-template <int WZ, int WN>
-__device__ __forceinline__ EB2<float> gather_win2(const float* fw, int xa, int xb, int za, int zb,
-                                                  const Ax2<float>& X, const Ax2<float>& Z) {
-  const float2 za0 = make_float2(Z.a0, Z.a0), za1 = make_float2(Z.a1, Z.a1);
-  const float2 zb0 = make_float2(Z.b0, Z.b0), zb1 = make_float2(Z.b1, Z.b1);
-  EB2<float> r;
-  r.ex = bil_pair<WZ>(fw + 0 * WN, xa, zb, X.a0, X.a1, zb0, zb1);
-  r.ey = bil_pair<WZ>(fw + 1 * WN, xb, zb, X.b0, X.b1, zb0, zb1);
-  r.ez = bil_pair<WZ>(fw + 2 * WN, xb, za, X.b0, X.b1, za0, za1);
-  r.bx = bil_pair<WZ>(fw + 3 * WN, xb, za, X.b0, X.b1, za0, za1);
-  r.by = bil_pair<WZ>(fw + 4 * WN, xa, za, X.a0, X.a1, za0, za1);
-  r.bz = bil_pair<WZ>(fw + 5 * WN, xa, zb, X.a0, X.a1, zb0, zb1);
+template <int WZ, int WN, typename real>
+__device__ __forceinline__ EB2<real> gather_win2(const real* n, const WinAxis2<real>& X, const WinAxis2<real>& Z) {
+  EB2<real> r;
+  r.ex = bil_win<WZ>(n + Z.s, X.a0, X.a1, Z.b0, Z.b1);
+  r.ey = bil_win<WZ>(n + WN + X.s + Z.s, X.b0, X.b1, Z.b0, Z.b1);
+  r.ez = bil_win<WZ>(n + 2 * WN + X.s, X.b0, X.b1, Z.a0, Z.a1);
+  r.bx = bil_win<WZ>(n + 3 * WN + X.s, X.b0, X.b1, Z.a0, Z.a1);
+  r.by = bil_win<WZ>(n + 4 * WN, X.a0, X.a1, Z.a0, Z.a1);
+  r.bz = bil_win<WZ>(n + 5 * WN + Z.s, X.a0, X.a1, Z.b0, Z.b1);
   return r;
+}
+
+// Adds the displacement d (in cells) to (i, f): advance's result, with the
+// moves of less than a cell in selects instead of a branch.
+template <typename real>
+__device__ __forceinline__ void move2(int& i, real& f, real d) {
+  real t = f + d;
+  if (t >= (real)1) {
+    t -= (real)1;
+    ++i;
+  }
+  if (t < (real)0) {
+    t += (real)1;
+    --i;
+  }
+  if (off_unit(t)) advance(i, t, (real)0);  // rounded to 1, -0, NaN, or a longer move
+  f = t;
 }
 
 template <typename real>
@@ -507,11 +531,11 @@ struct Home2 {
         if (c < 2) jz_[a][c] = (real)0;
       }
   }
-  // J of one particle with charge weight q, x-aligned weights (xa0, xa1),
+  // The current (qx, qy, qz) of one particle with x-aligned weights (xa0, xa1),
   // z-aligned (za0, za1) and half-shifted weights xb, zb over the 3 nodes
-  __device__ __forceinline__ void add_j(real q, real vx, real vy, real vz, real xa0, real xa1, real za0, real za1,
+  __device__ __forceinline__ void add_j(real qx, real qy, real qz, real xa0, real xa1, real za0, real za1,
                                         const real (&xb)[3], const real (&zb)[3]) {
-    const real px0 = q * vx * xa0, px1 = q * vx * xa1;
+    const real px0 = qx * xa0, px1 = qx * xa1;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       jx_[0][c] += px0 * zb[c];
@@ -519,7 +543,7 @@ struct Home2 {
     }
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
-      const real py = q * vy * xb[b], pz = q * vz * xb[b];
+      const real py = qy * xb[b], pz = qz * xb[b];
 #pragma unroll
       for (int c = 0; c < 3; ++c) jy_[b][c] += py * zb[c];
       jz_[b][0] += pz * za0;
@@ -554,9 +578,8 @@ struct Home2<float> {
       jy2_[c] = n2_[c] = 0.f;
     }
   }
-  __device__ __forceinline__ void add_j(float q, float vx, float vy, float vz, float xa0, float xa1, float za0,
-                                        float za1, const float (&xb)[3], const float (&zb)[3]) {
-    const float qx = q * vx, qy = q * vy, qz = q * vz;
+  __device__ __forceinline__ void add_j(float qx, float qy, float qz, float xa0, float xa1, float za0, float za1,
+                                        const float (&xb)[3], const float (&zb)[3]) {
     const float2 px = __fmul2_rn(make_float2(qx, qx), make_float2(xa0, xa1));
     const float2 py = __fmul2_rn(make_float2(qy, qy), make_float2(xb[0], xb[1]));
     const float py2 = qy * xb[2];
@@ -621,6 +644,14 @@ __device__ __forceinline__ void home_w3(int i, real f, int h, real (&w)[3]) {
 // once per group; a particle elsewhere adds its terms to the planes directly.
 // 512 resident threads per SM in FP32 (128 registers: the 30 home sums and
 // the particle in flight fit without spills), 256 in FP64.
+//
+// Bound by instructions: 67 % of the issue slots at 4 warps per scheduler, the
+// rest mostly fixed-latency dependences; DRAM at 30 %. So the loop has no
+// branch that splits a warp between home and other particles (a lane without
+// a home particle adds zeros to the home sums), tests the faces and margins
+// with one comparison per axis, and addresses slots and window nodes with
+// 32-bit offsets. The step of 256 FP32 runs of 64^2 .. 256^2 cells: 14.63 ->
+// 14.15 ms, of 8 runs of 64^2 .. 96^2: 0.164 -> 0.161.
 template <typename real, int TX>
 __global__ void __launch_bounds__(TX * 32, (sizeof(real) == 4 ? 512 : 256) / (TX * 32))
     push2d_tiled_kernel(Pools pools, real* F, const Run<real>* __restrict__ runs, Layout2 L,
@@ -674,9 +705,9 @@ __global__ void __launch_bounds__(TX * 32, (sizeof(real) == 4 ? 512 : 256) / (TX
     if (hi < R.nx + 2) {  // warp-uniform
       const PView<real> P = pview<real>(pools, s);
       const int Gi = R.gbase + (hi - 2) * R.nzb + (tile % R.nzb);
-      const long long base = R.poff + L.goff[s][Gi] - L.goff[s][R.gbase] + lane;
-      const long long end = R.poff + RR.cap;  // rows of a layout that overflowed the run were not written
-      const int m = L.gmax[s][Gi];
+      const unsigned base = (unsigned)(R.poff + L.goff[s][Gi] - L.goff[s][R.gbase]) + lane;  // slots are 32-bit
+      // rows of a layout that overflowed the run were not written
+      const int m = (int)min((long long)L.gmax[s][Gi], (R.poff + RR.cap - (long long)(base - lane)) / 32);
       const real T = (real)Ts;
       const real hdt = (real)(0.5 * RR.dt / RR.dx);
       const real qn = (real)(RR.q * RR.nw);
@@ -688,8 +719,8 @@ __global__ void __launch_bounds__(TX * 32, (sizeof(real) == 4 ? 512 : 256) / (TX
       // each lane copies and reads only its own slots, so the per-thread
       // cp.async groups need no warp barrier
       auto fetch = [&](int row) {
-        const long long t = base + 32LL * row;
-        if (kSt > 1 && row < m && t < end) {
+        const unsigned t = base + 32u * row;
+        if (kSt > 1 && row < m) {
           const int st = row % kSt;
           cp_async_ca(&ring_c[warp][st][lane], P.cell + t, 4);
           cp_async_ca(&ring_r[warp][st][0][lane], P.ox + t, sizeof(real));
@@ -719,9 +750,14 @@ __global__ void __launch_bounds__(TX * 32, (sizeof(real) == 4 ? 512 : 256) / (TX
         const Ax2<real> X = ax2(qi, (real)e[1]), Z = ax2(qk, (real)e[2]);
         dep4(pj(3), G, X.b, Z.b, nw, X.b0, X.b1, Z.b0, Z.b1);
       };
+      // interior cells whose stencils lie in the window; cells that are surely
+      // not ballistic (:682-686: z < A2, z > Nz+4-A2, x < A2, x > Nx+4-A2)
+      const int nx0 = max(wx0 + 1, 2), nz0 = max(wz0 + 1, 2);
+      const unsigned nxe = (unsigned)(min(wx0 + WX - 1, R.nx + 2) - nx0), nze = (unsigned)(min(wz0 + WZ - 1, R.nz + 2) - nz0);
+      const unsigned cxe = (unsigned)max(hx - R.a2, 0), cze = (unsigned)max(hz - R.a2, 0);
       for (int row = 0; row < m; ++row) {
         fetch(row + kSt - 1);
-        const long long t = base + 32LL * row;
+        const unsigned t = base + 32u * row;
         int c;
         real fx, fz, vx, vy, vz;
         if (kSt > 1) {
@@ -734,105 +770,110 @@ __global__ void __launch_bounds__(TX * 32, (sizeof(real) == 4 ? 512 : 256) / (TX
           vy = ring_r[warp][st][3][lane];
           vz = ring_r[warp][st][4][lane];
         } else {
-          c = t < end ? P.cell[t] : -1;
-          if (c >= 0) {
-            fx = P.ox[t]; fz = P.oz[t];
-            vx = P.vx[t]; vy = P.vy[t]; vz = P.vz[t];
+          c = P.cell[t];
+          fx = P.ox[t]; fz = P.oz[t];
+          vx = P.vx[t]; vy = P.vy[t]; vz = P.vz[t];
+        }
+        const bool act = c >= 0;
+        pushed += act;
+        int i, k;
+        unpack2(c, i, k);
+        bool push = act;
+        if (!((unsigned)(i - R.a2) < cxe && (unsigned)(k - R.a2) < cze))
+          push = act && !(k < R.a2 || i < R.a2 || k > hz || (k == hz && fz > (real)0) || i > hx ||
+                          (i == hx && fx > (real)0));
+        if (push) {
+          // ex, bz: x aligned, z shifted; ez, bx: x shifted, z aligned; ey: both shifted; by: both aligned
+          EB2<real> e;
+          if ((unsigned)(i - nx0) < nxe && (unsigned)(k - nz0) < nze) {
+            const WinAxis2<real> X = win_axis2(fx, WZ), Z = win_axis2(fz, 1);
+            e = gather_win2<WZ, WN>(fw + ((i - wx0) * WZ + k - wz0), X, Z);
+          } else if (i < 1 || k < 1 || i > R.gx - 2 || k > R.gz - 2) {
+            atomicAdd(err + ERR_DEPOSIT_OOB, 1ull);
+            push = false;
+          } else {
+            const Ax2<real> X = ax2(i, fx), Z = ax2(k, fz);
+            e.ex = bil(F0 + (long long)P_EX * R.nodes, G, X.a, Z.b, X.a0, X.a1, Z.b0, Z.b1);
+            e.ey = bil(F0 + (long long)P_EY * R.nodes, G, X.b, Z.b, X.b0, X.b1, Z.b0, Z.b1);
+            e.ez = bil(F0 + (long long)P_EZ * R.nodes, G, X.b, Z.a, X.b0, X.b1, Z.a0, Z.a1);
+            e.bx = bil(F0 + (long long)P_BX * R.nodes, G, X.b, Z.a, X.b0, X.b1, Z.a0, Z.a1);
+            e.by = bil(F0 + (long long)P_BY * R.nodes, G, X.a, Z.a, X.a0, X.a1, Z.a0, Z.a1);
+            e.bz = bil(F0 + (long long)P_BZ * R.nodes, G, X.a, Z.b, X.a0, X.a1, Z.b0, Z.b1);
+          }
+          if (push) rotate_c4(T, e.ex + ex_add, e.ey + ey_add, e.ez, e.bx, e.by, e.bz, vx, vy, vz);
+        }
+        // From here on every lane runs: one without a particle, or whose
+        // particle is off its home cell, adds zeros (finite weights times a
+        // zero current) to the home sums.
+        if (!act) {
+          fx = fz = (real)0.5;
+          vx = vz = (real)0;
+          i = hi - 1;
+        }
+        const real dx = vx * hdt, dz = vz * hdt;
+        move2(i, fx, dx);
+        move2(k, fz, dz);
+        // J deposit at x^{n+1/2} for dx <= x < (Nx+3) dx, 2 dx <= z < (Nz+2) dx
+        const bool homej = i == hi && k == hk;
+        const bool qj = act && !homej && i >= 1 && i < R.nx + 3 && k >= 2 && k < R.nz + 2;
+        {
+          real xb[3], zb[3];
+          const real ax = homej ? fx : (real)0.5, az = homej ? fz : (real)0.5;  // finite weights
+          home_w3(i, ax, hi, xb);
+          home_w3(k, az, hk, zb);
+          h.add_j(homej ? qn * vx : (real)0, homej ? qn * vy : (real)0, homej ? qn * vz : (real)0, (real)1 - ax, ax,
+                  (real)1 - az, az, xb, zb);
+        }
+        const unsigned mj = kQueue ? __ballot_sync(0xffffffffu, qj) : 0u;
+        if (qj) {
+          if constexpr (kQueue) {
+            float* e = jq_s[warp][njq + __popc(mj & ((1u << lane) - 1u))];
+            e[0] = __int_as_float(pack2(i, k));
+            e[1] = (float)fx; e[2] = (float)fz;
+            e[3] = (float)(qn * vx); e[4] = (float)(qn * vy); e[5] = (float)(qn * vz);
+          } else {
+            const Ax2<real> X = ax2(i, fx), Z = ax2(k, fz);
+            dep4(pj(0), G, X.a, Z.b, qn * vx, X.a0, X.a1, Z.b0, Z.b1);
+            dep4(pj(1), G, X.b, Z.b, qn * vy, X.b0, X.b1, Z.b0, Z.b1);
+            dep4(pj(2), G, X.b, Z.a, qn * vz, X.b0, X.b1, Z.a0, Z.a1);
           }
         }
-        if (t >= end) c = -1;  // rows of a layout that overflowed the run were not written
-        bool qj = false, qnn = false;  // J / n of this particle go to the warp's queues
-        int jc = 0, ncell = 0;
-        real jfx = 0, jfz = 0;
-        if (c >= 0) {
-          ++pushed;
-          int i, k;
-          unpack2(c, i, k);
-          // ballistic margins (:682-686): z < A2, z > Nz+4-A2, x < A2, x > Nx+4-A2 (cells)
-          const bool bal = k < R.a2 || i < R.a2 || k > hz || (k == hz && fz > (real)0) || i > hx ||
-                           (i == hx && fx > (real)0);
-          if (!bal) {
-            if (i < 1 || k < 1 || i > R.gx - 2 || k > R.gz - 2) {
-              atomicAdd(err + ERR_DEPOSIT_OOB, 1ull);
-            } else {
-              const Ax2<real> X = ax2(i, fx), Z = ax2(k, fz);
-              // ex, bz: x aligned, z shifted; ez, bx: x shifted, z aligned; ey: both shifted; by: both aligned
-              real ex, ey, ez, bx, by, bz;
-              if (i - 1 >= wx0 && i + 1 < wx0 + WX && k - 1 >= wz0 && k + 1 < wz0 + WZ) {
-                const EB2<real> e = gather_win2<WZ, WN>(fw, X.a - wx0, X.b - wx0, Z.a - wz0, Z.b - wz0, X, Z);
-                ex = e.ex; ey = e.ey; ez = e.ez; bx = e.bx; by = e.by; bz = e.bz;
-              } else {
-                ex = bil(F0 + (long long)P_EX * R.nodes, G, X.a, Z.b, X.a0, X.a1, Z.b0, Z.b1);
-                ey = bil(F0 + (long long)P_EY * R.nodes, G, X.b, Z.b, X.b0, X.b1, Z.b0, Z.b1);
-                ez = bil(F0 + (long long)P_EZ * R.nodes, G, X.b, Z.a, X.b0, X.b1, Z.a0, Z.a1);
-                bx = bil(F0 + (long long)P_BX * R.nodes, G, X.b, Z.a, X.b0, X.b1, Z.a0, Z.a1);
-                by = bil(F0 + (long long)P_BY * R.nodes, G, X.a, Z.a, X.a0, X.a1, Z.a0, Z.a1);
-                bz = bil(F0 + (long long)P_BZ * R.nodes, G, X.a, Z.b, X.a0, X.a1, Z.b0, Z.b1);
-              }
-              rotate_c4(T, ex + ex_add, ey + ey_add, ez, bx, by, bz, vx, vy, vz);
-            }
+        move2(i, fx, dx);
+        move2(k, fz, dz);
+        // n at x^{n+1}, same range
+        const bool homen = i == hi && k == hk;
+        const bool qnn = act && !homen && i >= 1 && i < R.nx + 3 && k >= 2 && k < R.nz + 2;
+        {
+          real xb[3], zb[3];
+          home_w3(i, homen ? fx : (real)0.5, hi, xb);
+          home_w3(k, homen ? fz : (real)0.5, hk, zb);
+          h.add_n(homen ? nw : (real)0, xb, zb);
+        }
+        const unsigned mn = kQueue ? __ballot_sync(0xffffffffu, qnn) : 0u;
+        if (qnn) {
+          if constexpr (kQueue) {
+            float* e = nq_s[warp][nnq + __popc(mn & ((1u << lane) - 1u))];
+            e[0] = __int_as_float(pack2(i, k));
+            e[1] = (float)fx; e[2] = (float)fz;
+          } else {
+            const Ax2<real> X = ax2(i, fx), Z = ax2(k, fz);
+            dep4(pj(3), G, X.b, Z.b, nw, X.b0, X.b1, Z.b0, Z.b1);
           }
-          advance(i, fx, vx * hdt);
-          advance(k, fz, vz * hdt);
-          // J deposit at x^{n+1/2} for dx <= x < (Nx+3) dx, 2 dx <= z < (Nz+2) dx
-          if (i == hi && k == hk) {
-            real xb[3], zb[3];
-            home_w3(i, fx, hi, xb);
-            home_w3(k, fz, hk, zb);
-            h.add_j(qn, vx, vy, vz, (real)1 - fx, fx, (real)1 - fz, fz, xb, zb);
-          } else if (i >= 1 && i < R.nx + 3 && k >= 2 && k < R.nz + 2) {
-            if constexpr (kQueue) {
-              qj = true;
-              jc = pack2(i, k);
-              jfx = fx;
-              jfz = fz;
-            } else {
-              const Ax2<real> X = ax2(i, fx), Z = ax2(k, fz);
-              dep4(pj(0), G, X.a, Z.b, qn * vx, X.a0, X.a1, Z.b0, Z.b1);
-              dep4(pj(1), G, X.b, Z.b, qn * vy, X.b0, X.b1, Z.b0, Z.b1);
-              dep4(pj(2), G, X.b, Z.a, qn * vz, X.b0, X.b1, Z.a0, Z.a1);
-            }
-          }
-          advance(i, fx, vx * hdt);
-          advance(k, fz, vz * hdt);
-          // n at x^{n+1}, same range
-          if (i == hi && k == hk) {
-            real xb[3], zb[3];
-            home_w3(i, fx, hi, xb);
-            home_w3(k, fz, hk, zb);
-            h.add_n(nw, xb, zb);
-          } else if (i >= 1 && i < R.nx + 3 && k >= 2 && k < R.nz + 2) {
-            if constexpr (kQueue) {
-              qnn = true;
-              ncell = pack2(i, k);
-            } else {
-              const Ax2<real> X = ax2(i, fx), Z = ax2(k, fz);
-              dep4(pj(3), G, X.b, Z.b, nw, X.b0, X.b1, Z.b0, Z.b1);
-            }
-          }
+        }
+        if (act) {
           // x exchange at size 1: forward crossers wrap, backward ones are dropped; then removal
-          if (i == R.nx + 2 && k >= 2 && k < R.nz + 2) i -= R.nx;
-          const bool keep = i >= 2 && i < R.nx + 2 && k >= 2 && k < R.nz + 2;
-          P.cell[t] = keep ? pack2(i, k) : -1;
+          int cnew = pack2(i, k);
+          if (!((unsigned)(i - 2) < (unsigned)R.nx && (unsigned)(k - 2) < (unsigned)R.nz)) {
+            if (i == R.nx + 2 && k >= 2 && k < R.nz + 2) cnew = pack2(2, k);
+            else cnew = -1;
+          }
+          P.cell[t] = cnew;
           P.ox[t] = fx; P.oz[t] = fz;
           P.vx[t] = vx; P.vy[t] = vy; P.vz[t] = vz;
         }
         if constexpr (kQueue) {
-          // warp-uniform: the row's queued lanes take consecutive entries, and
+          // warp-uniform: the row's queued lanes took consecutive entries, and
           // a full warp's worth is deposited by all 32 lanes at once
-          const unsigned below = (1u << lane) - 1u;
-          const unsigned mj = __ballot_sync(0xffffffffu, qj), mn = __ballot_sync(0xffffffffu, qnn);
-          if (qj) {
-            float* e = jq_s[warp][njq + __popc(mj & below)];
-            e[0] = __int_as_float(jc);
-            e[1] = (float)jfx; e[2] = (float)jfz;
-            e[3] = (float)(qn * vx); e[4] = (float)(qn * vy); e[5] = (float)(qn * vz);
-          }
-          if (qnn) {
-            float* e = nq_s[warp][nnq + __popc(mn & below)];
-            e[0] = __int_as_float(ncell);
-            e[1] = (float)fx; e[2] = (float)fz;
-          }
           njq += __popc(mj);
           nnq += __popc(mn);
           if (njq >= 32 || nnq >= 32) {
