@@ -286,7 +286,7 @@ def run_e2e(P, steps: int):
 # from the ncu capture of a 64^3 x 64 ppc launch
 # (profiles/push_tiled_kernel_grid64_64ppc.md); at a fixed number of particles
 # per cell the traffic of a launch grows with its particles.
-PUSH_TRAFFIC_PER_PARTICLE = 73.0
+PUSH_TRAFFIC_PER_PARTICLE = 61.9
 
 
 def roofline(out, npart_species, cells, rsize):
@@ -801,7 +801,7 @@ def main():
             "roofline": {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
                          "frac": ach / peak,
                          "traffic": PUSH_TRAFFIC_PER_PARTICLE * nsp if PPC == 64 else None,
-                         "kernel": "push_tiled_kernel<float,1> (push phase, with its tail push_kernel)",
+                         "kernel": "push_tiled_kernel<float,true,PUSH_FUSED> (push phase)",
                          "peak_kind": peak_kind, "bytes_per_launch": bytes_launch,
                          "ms_per_launch": s_launch * 1e3},
             "step_roofline": {"bytes_per_step": step_bytes, "achieved": step_bytes / (ms_max / args.steps) / 1e6,

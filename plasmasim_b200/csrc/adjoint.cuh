@@ -672,7 +672,7 @@ __global__ void wrap_y_adjoint(PlaneSet<real> s, Geom g) {
   }
 }
 
-// Reverse of wrap_b_kernel on the induced field:
+// Reverse of the ghost copies of B on the induced field:
 // DB[dst] = DB[src] + B0[src] - B0[dst], so besides the copy's transpose the
 // ghost adjoints add lDB[dst] (B0[src] - B0[dst]) / I to dJ/dI (acc[1]).
 template <typename real>

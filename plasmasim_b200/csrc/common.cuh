@@ -5,12 +5,13 @@
 // reference's z, its solar-wind axis) fastest, as grid[k][l][m] of
 // PIC/3d_pic458_domain.c:147. Planes are padded to 256-byte boundaries.
 //
-// Particle layout: structure of arrays per species,
-//   cell : int32, (i << 20) | (j << 10) | k, the containing cell of the padded
-//          grid (i = floor(x/dx)), -1 for an empty slot
-//   ox, oy, oz : in-cell offsets in [0, 1) (x = (i + ox) dx)
-//   vx, vy, vz : velocities in the caller's units
-// 28 bytes per particle in FP32, 52 in FP64.
+// Particle layout: two records of four words per particle, each in its own
+// array per species,
+//   A = (cell, ox, oy, oz): cell an int32, (i << 20) | (j << 10) | k, the
+//       containing cell of the padded grid (i = floor(x/dx)), -1 for an empty
+//       slot; ox, oy, oz in-cell offsets in [0, 1) (x = (i + ox) dx)
+//   B = (vx, vy, vz, unused): velocities in the caller's units
+// 32 bytes per particle in FP32, 64 in FP64.
 #pragma once
 
 #include <cstdint>

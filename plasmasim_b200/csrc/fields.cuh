@@ -1,6 +1,7 @@
 // Field kernels: dipole B0 and damping profile (init_grid), the damped
-// 4th-order B and E updates (renew_b4_2 / renew_e4_2) and the size-1 periodic
-// ghost copies and folds (sr_b / sr_e / sr_current2).
+// 4th-order B and E updates (renew_b4_2 / renew_e4_2), which also write the
+// size-1 periodic ghost copies (sr_b / sr_e), and the fold of J and n
+// (sr_current2).
 //
 // Each update is one thread per interior node, k (z) fastest so that a warp
 // reads and writes 32 consecutive nodes of every plane it touches; the +-1/+-2

@@ -24,11 +24,12 @@
 // Deposit. A lane accumulates the current of the particles that are in its
 // home cell in registers (the 2x3x3 / 3x2x3 / 3x3x2 nodes such a particle can
 // touch) and adds them to a shared-memory window of (TX+4) x (TY+4) x 36 nodes
-// once, after its last particle. The current of particles that have left
-// their home cell since the sort, and every density deposit, go to the window
-// with shared atomics, or, when the stencil leaves the window (periodic wrap,
-// long moves), to global memory with atomics. The window is added to the
-// global planes with one vector reduction per 4 nodes.
+// once, after its last particle. The currents of particles that have left
+// their home cell since the sort are queued per warp and added to the planes
+// 32 at a time; the densities go to the window as fixed-point numbers with
+// shared integer reductions, or, when the stencil leaves the window (periodic
+// wrap, long moves), to global memory. The window is added to the global planes
+// with one vector reduction per 4 nodes.
 //
 // Sort. Between sorts most particles stay in their cell. The sort keeps the
 // order of those "stayers" within their lane column (a warp walks its columns
