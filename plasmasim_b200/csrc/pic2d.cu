@@ -651,7 +651,7 @@ __device__ __forceinline__ void home_w3(int i, real f, int h, real (&w)[3]) {
 // a home particle adds zeros to the home sums), tests the faces and margins
 // with one comparison per axis, and addresses slots and window nodes with
 // 32-bit offsets. The step of 256 FP32 runs of 64^2 .. 256^2 cells: 14.63 ->
-// 14.15 ms, of 8 runs of 64^2 .. 96^2: 0.164 -> 0.161.
+// 14.15 ms (at 8 blocks per SM), of 8 runs of 64^2 .. 96^2: 0.164 -> 0.161.
 template <typename real, int TX>
 __global__ void __launch_bounds__(TX * 32, (sizeof(real) == 4 ? 512 : 256) / (TX * 32))
     push2d_tiled_kernel(Pools pools, real* F, const Run<real>* __restrict__ runs, Layout2 L,
@@ -2237,7 +2237,12 @@ int do_create(pic2d_batch* b) {
   CK2(cudaMalloc(&b->err, sizeof(unsigned long long) * ERR_COUNT));
   CK2(cudaMemset(b->err, 0, sizeof(unsigned long long) * ERR_COUNT));
   CKR2(set_tiles(b, 4));
-  b->push_blocks = persistent(b->n_ptile, 8);
+  // One block per tile: runs differ fourfold in particles per cell, and blocks
+  // that walk the list with a fixed stride end unevenly. The 256-run batch's
+  // step took 14.36 ms with 8 blocks per SM, 14.15 with 16, 13.90 with 64 and
+  // 13.65 with one per tile (109414); 8 small runs have fewer tiles (about
+  // 1000) than 8 blocks per SM, so nothing changes for them.
+  b->push_blocks = std::max(b->n_ptile, 1);
   return PIC_OK;
 }
 
@@ -2343,14 +2348,12 @@ int do_thrust(pic2d_batch* b, double* out) {
 }
 
 // Online tuning: the next steps of the run itself try each push tile shape
-// (1, 2, 4 or 8 group rows of 32 cells, one warp per row) with 8 or 16
-// resident blocks' worth of persistent blocks per SM, timing whole loop
-// bodies, and the fastest is kept; the steps taken are ordinary steps of the
-// run.
+// (1, 2, 4 or 8 group rows of 32 cells, one warp per row) with 16 persistent
+// blocks per SM and with one block per tile, timing whole loop bodies, and the
+// fastest is kept; the steps taken are ordinary steps of the run.
 template <typename real>
 int do_autotune(pic2d_batch* b, int* choice) {
   const int shapes[4] = {1, 2, 4, 8};
-  const int per_sm[2] = {8, 16};
   float best = 1e30f;
   int bt = b->tile_x, bs = b->push_blocks;
   cudaEvent_t e0, e1;
@@ -2361,7 +2364,7 @@ int do_autotune(pic2d_batch* b, int* choice) {
     for (int j = 0; j < 2 && rc == PIC_OK; ++j) {
       rc = set_tiles(b, shapes[i]);
       if (rc != PIC_OK) break;
-      b->push_blocks = persistent(b->n_ptile, per_sm[j]);
+      b->push_blocks = j == 0 ? persistent(b->n_ptile, 16) : std::max(b->n_ptile, 1);
       const bool g = b->use_graph;
       b->use_graph = false;
       cudaEventRecord(e0, b->stream);
