@@ -579,16 +579,18 @@ push_tiled_kernel(const __grid_constant__ Parts<real> P, const __grid_constant__
     }
     // From here to the density every lane runs, with no branch: a lane without
     // a particle, or whose particle is off its home cell, adds zero currents
-    // (weights of offsets in [0, 1], whatever an empty slot holds).
-    if (!quick) fx = fy = fz = (real)0.5;
+    // at offsets of 1/2. Its own may be anything, and 0 times a NaN would stay
+    // in the sums: an empty slot's record holds what its last particle or the
+    // memory's last owner left there.
     const real dx = vx * pc.hdt, dy = vy * pc.hdt, dz = vz * pc.hdt;
     // an offset rounded to 1 or -0 deposits the same current as in the cell it
     // belongs to; the second half step puts it there
     step_cell(c, fx, fy, fz, dx, dy, dz);
     const bool home = quick && c == hcell;
     {
-      const W3<real> bx = home3(fx), by = home3(fy), bz = home3(fz);
-      acc.add(home ? pc.qn * vx : (real)0, home ? pc.qn * vy : (real)0, home ? pc.qn * vz : (real)0, fx, fy, fz, bx, by,
+      const real hx = home ? fx : (real)0.5, hy = home ? fy : (real)0.5, hz = home ? fz : (real)0.5;
+      const W3<real> bx = home3(hx), by = home3(hy), bz = home3(hz);
+      acc.add(home ? pc.qn * vx : (real)0, home ? pc.qn * vy : (real)0, home ? pc.qn * vz : (real)0, hx, hy, hz, bx, by,
               bz);
     }
     // the others' currents go to the warp's queue: the row's queued lanes take
