@@ -92,7 +92,8 @@ struct pic_ctx {
   int* gtop[2] = {nullptr, nullptr};  // rows in use of each group of the current layout
   int* glevel[2] = {nullptr, nullptr};  // its level when it was last sorted or re-laid
   int2* gfree = nullptr;              // a full sort's free slots (NewLayout)
-  int* gcursor = nullptr;             // and its per-group cursor
+  int* gcursor = nullptr;             // its per-group cursor
+  int* newlevel = nullptr;            // and its levels, until it is known to fit
   int lay[2] = {0, 0};                // current layout buffer
   bool layout[2] = {false, false};    // slots [0, tiled_end) follow goff/gmax[lay]
   long long tiled_end[2] = {0, 0};
@@ -875,7 +876,7 @@ int do_sort_species(pic_ctx* c, int s) {
   Slab slabs[5];
   refill_slabs(c, slabs);
   group_size_kernel<<<gblocks, kThreads, 0, c->stream>>>(c->g, tg, stay, moved, source_params(c, s, slabs, 5, 0),
-                                                         c->gmax[s][nw], c->glevel[s], c->gtop[s], c->gfree, c->gcap);
+                                                         c->gmax[s][nw], c->newlevel, c->gfree, c->gcap);
   CKL();
   CKR(scan_exclusive(c, c->gcap, c->goff[s][nw], tg.ngroups, c->scan_tmp, c->scan_tmp_len));
   tiled_total_kernel<<<1, 1, 0, c->stream>>>(c->goff[s][nw], c->gcap, tg.ngroups, c->total_dev);
@@ -883,13 +884,13 @@ int do_sort_species(pic_ctx* c, int s) {
   int total = 0;
   CK(cudaMemcpyAsync(&total, c->total_dev, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
-  if (total > st.cap) return PIC_ERR_CAPACITY;
+  if (total > st.cap) return PIC_ERR_CAPACITY;  // nothing of the present layout has changed
   Parts<real> Q = parts<real>(c, s, 1 - st.cur);
   group_pad_kernel<<<gblocks, kThreads, 0, c->stream>>>(c->g, tg, stay, moved, c->goff[s][nw], c->gmax[s][nw],
-                                                        c->gtop[s], Q.cell);
+                                                        c->newlevel, c->glevel[s], c->gtop[s], Q.cell);
   CKL();
   CK(cudaMemsetAsync(c->gcursor, 0, sizeof(int) * tg.ngroups, c->stream));
-  const NewLayout nl{c->goff[s][nw], c->gtop[s], c->gfree, stay, c->cursor, c->gcursor};
+  const NewLayout nl{c->goff[s][nw], c->newlevel, c->gfree, stay, c->cursor, c->gcursor};
   if (have) {
     tiled_scatter_kernel<real><<<gblocks, kThreads, 0, c->stream>>>(
         P, c->g, tg, c->goff[s][old], c->gmax[s][old], nl, Q);
@@ -1817,14 +1818,15 @@ int pic_create(const pic_config* cfg, pic_ctx** out) {
         if (cudaMalloc(&c->gmax[s][b], sizeof(int) * t.ngroups) != cudaSuccess) return fail(PIC_ERR_CUDA);
       }
     }
-    // gfree, gtop and glevel of both species and gcursor in one block
-    if (cudaMalloc(&c->gfree, (sizeof(int2) * kLanes + sizeof(int) * 5) * t.ngroups) != cudaSuccess)
+    // gfree, gtop and glevel of both species, gcursor and newlevel in one block
+    if (cudaMalloc(&c->gfree, (sizeof(int2) * kLanes + sizeof(int) * 6) * t.ngroups) != cudaSuccess)
       return fail(PIC_ERR_CUDA);
     c->gtop[0] = (int*)(c->gfree + (size_t)kLanes * t.ngroups);
     c->gtop[1] = c->gtop[0] + t.ngroups;
     c->glevel[0] = c->gtop[1] + t.ngroups;
     c->glevel[1] = c->glevel[0] + t.ngroups;
     c->gcursor = c->glevel[1] + t.ngroups;
+    c->newlevel = c->gcursor + t.ngroups;
     if (cudaMalloc(&c->gcap, sizeof(int) * t.ngroups) != cudaSuccess) return fail(PIC_ERR_CUDA);
     if (cudaMalloc(&c->total_dev, sizeof(int)) != cudaSuccess) return fail(PIC_ERR_CUDA);
     if (cudaMalloc(&c->append_dev, sizeof(int)) != cudaSuccess) return fail(PIC_ERR_CUDA);

@@ -210,13 +210,14 @@ __device__ __forceinline__ int warp_sum(int v) {
 __device__ __forceinline__ int group_level(int n) { return n > 0 ? (n + kLanes - 1) / kLanes + kLevelRows : 0; }
 
 // One warp per group, from the (stayers + movers) counts of its 32 cells: the
-// level (into gtop), gmax = the level of the group with every lane's refill
-// reserve counted, plus the slack, and where the group's strangers go: the
-// slots free below the level, numbered lane by lane (NewLayout::free).
+// level, gmax = the level of the group with every lane's refill reserve
+// counted, plus the slack, and where the group's strangers go: the slots free
+// below the level, numbered lane by lane (NewLayout::free). All of it is the
+// new layout's: the sort may still find that it does not fit, and the present
+// layout then goes on.
 __global__ void group_size_kernel(Geom g, TileGeom t, const int* __restrict__ stay,
                                   const int* __restrict__ moved, SourceParams refill, int* gmax,
-                                  int* glevel,
-                                  int* gtop, int2* free, int* gcap) {
+                                  int* newlevel, int2* free, int* gcap) {
   const int G = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (G >= t.ngroups) return;
@@ -230,31 +231,34 @@ __global__ void group_size_kernel(Geom g, TileGeom t, const int* __restrict__ st
   free[G * kLanes + lane] = make_int2(warp_scan(free_below) - free_below, min(c, level));
   if (lane == 0) {
     gmax[G] = rows;
-    gtop[G] = glevel[G] = level;
+    newlevel[G] = level;
     gcap[G] = rows * kLanes;
   }
 }
 
-// Marks the slots of every lane column above its own particles empty (the
-// strangers among them are written afterwards).
+// The first pass that writes the new layout: marks the slots of every lane
+// column above its own particles empty (the strangers among them are written
+// afterwards) and sets the groups' levels and tops.
 template <typename CellArray>
 __global__ void group_pad_kernel(Geom g, TileGeom t, const int* __restrict__ stay,
                                  const int* __restrict__ moved, const int* __restrict__ goff,
-                                 const int* __restrict__ gmax, const int* __restrict__ gtop, CellArray cell) {
+                                 const int* __restrict__ gmax, const int* __restrict__ newlevel, int* glevel,
+                                 int* gtop, CellArray cell) {
   const int G = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (G >= t.ngroups) return;
   LaneCell lc;
   const int home = home_key(g, t, G, lane, lc);
-  const int c = min(home >= 0 ? lane_share(stay[home] + moved[home], lc) : 0, gtop[G]);
+  const int c = min(home >= 0 ? lane_share(stay[home] + moved[home], lc) : 0, newlevel[G]);
   const int m = gmax[G], base = goff[G];
+  if (lane == 0) gtop[G] = glevel[G] = newlevel[G];
   for (int r = c; r < m; ++r) cell[base + r * kLanes + lane] = -1;
 }
 
 // The new layout of a full sort, as the scatter kernels need it.
 struct NewLayout {
   const int* goff;
-  const int* level;   // per group (group_size_kernel's gtop)
+  const int* level;   // per group (group_size_kernel)
   const int2* free;   // per lane of each group: its first stranger's number in the group, its first free row
   const int* stay;    // per cell: stayers
   int* cursor;        // per cell: movers placed so far
