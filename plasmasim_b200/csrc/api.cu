@@ -1786,10 +1786,13 @@ int pic_create(const pic_config* cfg, pic_ctx** out) {
   const bool tiled = k.slot_order == 0;
   long long cap = k.capacity;
   if (cap <= 0) {
-    // the tiled layout gives every lane column room for its fullest cell plus
-    // a refill reserve (refill_reserve): about np + 3 sqrt(np) + 2 slots per
-    // cell, plus an eighth, plus 4; a few more for the unplaced tail. Slot
-    // order keeps the initial load and the refills of about 100 steps.
+    // the tiled layout's rows are a group's mean lane, with the refill's
+    // reserve, and an eighth and three more, and never more than its fullest
+    // cell asks for (tiled.cuh): np + 3 sqrt(np) + 2 slots per cell, plus an
+    // eighth, plus 6, hold both where the groups are whole; the lanes that
+    // sides no tile divides add to a group, and the slots behind the layout,
+    // come out of the 65536. Slot order keeps the initial load and the refills
+    // of about 100 steps.
     const double per_cell = tiled ? 1.125 * (k.np + 3.0 * std::sqrt((double)k.np) + 2.0) + 6.0 : 1.8 * k.np;
     cap = (long long)(per_cell * k.nx * k.ny * k.nz) + 65536;
   }

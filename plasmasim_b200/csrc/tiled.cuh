@@ -47,9 +47,15 @@ namespace pb {
 
 // Rows that a full sort adds to a group above its level, level / kSlackDiv +
 // kSlackRows: room for a group that gains particles until the next full sort
-// (empty rows above gtop cost memory only).
+// (empty rows above gtop cost memory only). No group takes more rows than its
+// fullest cell would with a sixteenth and two rows more, which is the smaller
+// of the two where the cells are evenly filled (19 rows against 21 at 16 per
+// cell): a capacity that holds rows sized that way, and the refills behind
+// them, always holds these.
 constexpr int kSlackDiv = 8;
 constexpr int kSlackRows = 3;
+constexpr int kFullestDiv = 16;
+constexpr int kFullestRows = 2;
 // Rows of the level above the group's mean particles per lane: each spares
 // some of the fuller cells' strangers and adds a partly filled row. One and
 // two rows measured 9.32 and 9.34 ms per step against 9.30 at 128^3 x 64, and
@@ -180,13 +186,11 @@ __global__ void append_count_kernel(Parts<real> P, int first, const int* __restr
 // Rows a lane column keeps for the boundary refill of its cell: the refill's
 // particle count plus an eighth and four, so that the refill fits into the
 // column's empty slots without moving other particles.
-__device__ __forceinline__ int refill_reserve(const SourceParams& sp, const Geom& g, const TileGeom& t,
-                                              int G, int lane) {
+__device__ __forceinline__ int reserve_of(int need) { return need > 0 ? need + need / 8 + 4 : 0; }
+__device__ __forceinline__ int refill_need(const SourceParams& sp, const Geom& g, const TileGeom& t, int G, int lane) {
   int i, j, k;
   LaneCell l;
-  if (!home_cell(g, t, G, lane, i, j, k, l)) return 0;
-  const int need = lane_share(slab_need(sp, i, j, k), l);
-  return need > 0 ? need + need / 8 + 4 : 0;
+  return home_cell(g, t, G, lane, i, j, k, l) ? slab_need(sp, i, j, k) : 0;
 }
 
 // Inclusive sum over the lanes of a warp.
@@ -197,6 +201,11 @@ __device__ __forceinline__ int warp_scan(int v) {
     const int y = __shfl_up_sync(0xffffffffu, v, o);
     if (lane >= o) v += y;
   }
+  return v;
+}
+__device__ __forceinline__ int warp_max(int v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
 __device__ __forceinline__ int warp_sum(int v) {
@@ -223,10 +232,12 @@ __global__ void group_size_kernel(Geom g, TileGeom t, const int* __restrict__ st
   if (G >= t.ngroups) return;
   LaneCell lc;
   const int home = home_key(g, t, G, lane, lc);
-  const int c = home >= 0 ? lane_share(stay[home] + moved[home], lc) : 0;
+  const int cell = home >= 0 ? stay[home] + moved[home] : 0, need = refill_need(refill, g, t, G, lane);
+  const int c = lane_share(cell, lc);
   const int level = group_level(warp_sum(c));
-  const int room = group_level(warp_sum(max(c, refill_reserve(refill, g, t, G, lane))));
-  const int rows = room > 0 ? room + room / kSlackDiv + kSlackRows : 0;
+  const int room = group_level(warp_sum(max(c, reserve_of(lane_share(need, lc)))));
+  const int fullest = warp_max(max(cell, reserve_of(need)));
+  const int rows = room > 0 ? min(room + room / kSlackDiv + kSlackRows, fullest + fullest / kFullestDiv + kFullestRows) : 0;
   const int free_below = max(level - c, 0);
   free[G * kLanes + lane] = make_int2(warp_scan(free_below) - free_below, min(c, level));
   if (lane == 0) {

@@ -1,5 +1,6 @@
 """The capacity of a store: a full sort that does not fit leaves the store as
-it was."""
+it was; evenly filled cells need no more slots than rows sized for each group's
+fullest cell, a sixteenth and two more."""
 import numpy as np
 import pytest
 
@@ -83,3 +84,43 @@ def test_a_sort_that_does_not_fit_changes_nothing(precision):
             if precision == 64:
                 assert rel_norm(canonical(a), canonical(b)) < 1e-6
         assert T.status()[0] == 0
+
+
+def refill(n, ppc):
+    """Particles that a refill puts into each cell: two layers at both ends of
+    z, between them at both ends of y, and low x (over the high y layers too)."""
+    need = np.zeros(n, dtype=int)
+    need[:, :, :2] += ppc
+    need[:, :, -2:] += ppc
+    need[:, :2, 2:-2] += ppc
+    need[:, -2:, 2:-2] += ppc
+    need[:2, 2:, 2:-2] += ppc
+    return need
+
+
+def fullest_slots(n, ppc):
+    """Slots of groups of 32 cells along z whose rows hold the group's fullest
+    cell (its refill with an eighth and four more, where that is larger) and a
+    sixteenth and two more, with ppc particles in every cell."""
+    need = refill(n, ppc)
+    m = np.maximum(ppc, np.where(need > 0, need + need // 8 + 4, 0))
+    m = m.reshape(n[0], n[1], -1, 32).max(axis=-1)
+    return int(32 * (m + m // 16 + 2).sum())
+
+
+@pytest.mark.parametrize("ppc", [4, 16, 64])
+def test_even_cells_fit_where_the_fullest_cell_does(ppc):
+    """A sort of evenly filled cells, and a refill behind the layout, in a
+    capacity of fullest_slots and the refill."""
+    n = (10, 12, 256)  # most groups without a shell's cells, no lane without a cell
+    cap = fullest_slots(n, ppc) + int(refill(n, ppc).sum())
+    with Pic3D(PicConfig.normalized(*n, ppc, precision=32, diag_every_step=0, sort_interval=1000, add_interval=1000,
+                                    capacity=cap)) as P:
+        P.init_grid()
+        P.init_particle_flat()
+        P.sorting()
+        for s in (ION, ELECTRON):  # without the initial load's particle outside the interior
+            assert P.particle_count(s) == ppc * np.prod(n)
+        P.add_flat()
+        P.step(1)
+        assert P.status()[0] == 0
