@@ -37,9 +37,11 @@ __host__ __device__ __forceinline__ void unpack_cell(int c, int& i, int& j, int&
 // of that one's CTAs have called after_prior; its own call then waits until
 // the earlier kernel has ended and its writes can be seen. Every thread of
 // every such kernel calls after_prior before it touches memory, so that a
-// kernel's end still implies that of all before it. (What such a kernel loads
-// in the same breath is not marked __restrict__, so that no load can be taken
-// for one of constant memory and moved ahead of the wait.) It saves the gap
+// kernel's end still implies that of all before it. None of its arguments is
+// marked __restrict__ and none of its loads at an address known from the start
+// goes through __ldg: either lets a load be taken for one of constant memory
+// and moved ahead of the wait. (gather6 does use __ldg, at addresses that come
+// from a particle's record, which is loaded behind the wait.) It saves the gap
 // between two kernels (with a re-layout's clears and counts folded into its
 // passes: 0.144 -> 0.141 ms per step at 32^3 x 8, 0.306 -> 0.288 at 41 x 22 x 70
 // x 30, the re-layout 0.035 -> 0.025 and 0.084 -> 0.074 of it).

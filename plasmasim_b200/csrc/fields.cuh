@@ -254,9 +254,9 @@ __global__ void __launch_bounds__(256) renew_b_kernel(Fields<real> F, Geom g, Ra
   const int m = 2 + t % g.nz, l = 2 + (t / g.nz) % g.ny, k = 2 + t / (g.nz * g.ny);
   const int n = k * g.sx + l * g.gz + m;
   const int sy = g.gz, sx = g.sx;
-  const real* __restrict__ ex = F.f[F_EX];
-  const real* __restrict__ ey = F.f[F_EY];
-  const real* __restrict__ ez = F.f[F_EZ];
+  const real* ex = F.f[F_EX];
+  const real* ey = F.f[F_EY];
+  const real* ez = F.f[F_EZ];
   const real c24 = (real)p.inv24dx;
   // x component at (k+1/2, l, m): sigma[2k+1][2l][2m]
   {
@@ -309,9 +309,9 @@ __global__ void __launch_bounds__(256) renew_e_kernel(Fields<real> F, Geom g, Ra
   const int m = 2 + t % g.nz, l = 2 + (t / g.nz) % g.ny, k = 2 + t / (g.nz * g.ny);
   const int n = k * g.sx + l * g.gz + m;
   const int sy = g.gz, sx = g.sx;
-  const real* __restrict__ bx = F.f[F_DBX];
-  const real* __restrict__ by = F.f[F_DBY];
-  const real* __restrict__ bz = F.f[F_DBZ];
+  const real* bx = F.f[F_DBX];
+  const real* by = F.f[F_DBY];
+  const real* bz = F.f[F_DBZ];
   const real c24 = (real)p.inv24dx;
   const real mu0 = (real)p.mu0;
   {

@@ -118,7 +118,8 @@ __device__ __forceinline__ Gathered<double> gather6_win(const double* __restrict
 }
 
 // The window's planes from F_EX .. F_BZ (16-byte loads where the row pitch
-// allows), zero outside the array.
+// allows; ordinary ones, which stay behind the wait for the launch before),
+// zero outside the array.
 template <typename real, int WX, int WY, int WZ, bool VEC>
 __device__ __forceinline__ void fill_win(real* __restrict__ fw, const Fields<real>& F, const Geom& g, int wx0, int wy0,
                                          int wz0) {
@@ -134,16 +135,16 @@ __device__ __forceinline__ void fill_win(real* __restrict__ fw, const Fields<rea
       const real* src = F.f[p] + (long long)ga * g.sx + gb * g.gz + gc;
       if (VEC && gc + V - 1 < g.gz) {
         if constexpr (V == 4) {
-          const float4 f4 = __ldg(reinterpret_cast<const float4*>(src));
+          const float4 f4 = *reinterpret_cast<const float4*>(src);
           v[0] = f4.x; v[1] = f4.y; v[2] = f4.z; v[3] = f4.w;
         } else {
-          const double2 f2 = __ldg(reinterpret_cast<const double2*>(src));
+          const double2 f2 = *reinterpret_cast<const double2*>(src);
           v[0] = f2.x; v[1] = f2.y;
         }
       } else {
 #pragma unroll
         for (int e = 0; e < V; ++e)
-          if (gc + e < g.gz) v[e] = __ldg(src + e);
+          if (gc + e < g.gz) v[e] = src[e];
       }
     }
     real* dst = fw + p * WN + (a * WY + b) * WZ + V * c;

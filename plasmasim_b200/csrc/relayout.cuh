@@ -86,8 +86,8 @@ __device__ __forceinline__ Rec<real> get_record(const real (&a)[4], const real (
 // 0.185 -> 0.165.
 constexpr int kRowsTogether = 4;
 template <typename real>
-__global__ void __launch_bounds__(256, sizeof(real) == 4 ? 3 : 2) classify_kernel(Parts<real> P, Geom g, TileGeom t, const int* __restrict__ goff,
-                                                       const int* __restrict__ gmax, const int* glevel, int* gtop,
+__global__ void __launch_bounds__(256, sizeof(real) == 4 ? 3 : 2) classify_kernel(Parts<real> P, Geom g, TileGeom t, const int* goff,
+                                                       const int* gmax, const int* glevel, int* gtop,
                                                        int cap, int* holes, int* nholes, int* hfirst, int* append_at,
                                                        int* nonhome, int shell) {
   after_prior();
@@ -283,8 +283,8 @@ __global__ void __launch_bounds__(256) place_count_kernel(Parts<real> P, int fir
 // particle writes its index to its bucket slot.
 template <typename real>
 __global__ void __launch_bounds__(256) place_bucket_kernel(Parts<real> P, int first, const int* append_at,
-                                                           int cap, Geom g, const int* __restrict__ off,
-                                                           const int* __restrict__ rank, int* bucket) {
+                                                           int cap, Geom g, const int* off,
+                                                           const int* rank, int* bucket) {
   after_prior();
   const int span = min(*append_at, cap) - first;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < span; q += gridDim.x * blockDim.x) {
@@ -302,11 +302,11 @@ __global__ void __launch_bounds__(256) place_bucket_kernel(Parts<real> P, int fi
 // what is left then goes to the spare buffer Q. gtop comes in as one past the
 // last row that kept a particle and goes out covering the filled rows as well.
 template <typename real>
-__global__ void place_fill_kernel(Parts<real> P, int first, Geom g, TileGeom t, const int* __restrict__ goff,
-                                  const int* __restrict__ gmax, int* glevel, int* gtop,
-                                  const int* __restrict__ holes, const int* __restrict__ arrivals,
-                                  const int* __restrict__ nholes, const int* __restrict__ hfirst,
-                                  const int* __restrict__ off, const int* __restrict__ bucket, int* nspill,
+__global__ void place_fill_kernel(Parts<real> P, int first, Geom g, TileGeom t, const int* goff,
+                                  const int* gmax, int* glevel, int* gtop,
+                                  const int* holes, const int* arrivals,
+                                  const int* nholes, const int* hfirst,
+                                  const int* off, const int* bucket, int* nspill,
                                   Parts<real> Q) {
   after_prior();
   constexpr int U = 4;  // holes per lane in flight together
