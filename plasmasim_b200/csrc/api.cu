@@ -768,47 +768,64 @@ bool long_tail(const pic_ctx* c, int s) {
   return !c->sp[s].pending && c->sp[s].count - c->tiled_end[s] > 148LL * 2 * kThreads;
 }
 
-// The tiles of species s's layout and, when it is not long, a CTA per SM for
-// its tail, whose length only the device may know. `overlap`: the launch just before on the stream is
-// the same kernel for the other species, which this one may run beside
-// (push_tiled.cuh).
-TileArgs tile_args(const pic_ctx* c, int s, bool overlap) {
-  const long long tail = long_tail(c, s) ? 0 : slot_bound(c, s) - c->tiled_end[s];
-  const int ntail = (int)std::min<long long>((std::max<long long>(tail, 0) + kThreads - 1) / kThreads, 148);
-  return TileArgs{c->tg, c->goff[s][c->lay[s]], c->gtop[s], ntail, (int)c->tiled_end[s], c->sp[s].count_dev, overlap};
-}
+// The species of a launch over the tiles (push_tiled.cuh), added one by one:
+// the tiles of a layout and, when it is not long, a CTA per SM for its tail,
+// whose length only the device may know.
+template <typename real>
+struct TileLaunch {
+  TileJobs<real> jobs{};
+  int n = 0, grid = 0;
+  void add(pic_ctx* c, int s) {
+    const long long tail = long_tail(c, s) ? 0 : slot_bound(c, s) - c->tiled_end[s];
+    const int ntail = (int)std::min<long long>((std::max<long long>(tail, 0) + kThreads - 1) / kThreads, 148);
+    jobs.job[n++] = TileJob<real>{parts<real>(c, s),  push_const<real>(c, s), c->goff[s][c->lay[s]], c->gtop[s],
+                                  ntail, (int)c->tiled_end[s], c->sp[s].count_dev};
+    const int blocks = ntail + c->tg.ntx * c->tg.nty * c->tg.ntz;
+    if (n == 1) jobs.split = blocks;
+    grid += blocks;
+    jobs.t = c->tg;
+  }
+};
 
-// The push of species s, of every part (PUSH_FUSED) or up to the J deposit.
+// The push of a species, or of both (-1), of every part (PUSH_FUSED) or up to
+// the J deposit: the slot-order kernel without a layout and for a long tail,
+// one launch over the tiles for the rest.
 template <typename real, int MODE>
-int do_push_tiled(pic_ctx* c, int s, bool overlap = false) {
-  if (!c->layout[s]) return do_push<real, MODE>(c, s);
-  if (long_tail(c, s)) CKR((do_push<real, MODE>(c, s, c->tiled_end[s])));
-  const TileArgs ta = tile_args(c, s, overlap && !long_tail(c, s));
+int do_push_tiled(pic_ctx* c, int species) {
+  TileLaunch<real> tl;
+  for (int s = 0; s < 2; ++s) {
+    if (species >= 0 && s != species) continue;
+    const long long first = c->layout[s] ? c->tiled_end[s] : 0;
+    if (!c->layout[s] || long_tail(c, s)) CKR((do_push<real, MODE>(c, s, first)));
+    if (c->layout[s]) tl.add(c, s);
+  }
+  if (!tl.n) return PIC_OK;
   const bool vec = c->g.gz * sizeof(real) % 16 == 0;
-  CK(launch_after(c, vec ? push_tiled_kernel<real, true, MODE> : push_tiled_kernel<real, false, MODE>,
-                  ta.ntail + c->tg.ntx * c->tg.nty * c->tg.ntz, kTileX * kTileY * 32, PushSmem<real>::bytes,
-                  parts<real>(c, s), ta, fields<real>(c), c->g, push_const<real>(c, s), c->err));
+  CK(launch_after(c, vec ? push_tiled_kernel<real, true, MODE> : push_tiled_kernel<real, false, MODE>, tl.grid,
+                  kTileX * kTileY * 32, PushSmem<real>::bytes, tl.jobs, fields<real>(c), c->g, c->err));
   CKL();
   return PIC_OK;
 }
 
+// The drift and density deposit of a species or of both, by the same split.
 template <typename real>
-int do_drift_n(pic_ctx* c, int s, bool overlap = false) {
-  if (c->sp[s].count == 0) return PIC_OK;
-  const bool tiles = c->layout[s], apart = !tiles || long_tail(c, s);
-  if (apart) {
-    const long long first = tiles ? c->tiled_end[s] : 0;
-    drift_n_kernel<real><<<particle_blocks(c->sp[s].count - first), kThreads, 0, c->stream>>>(
-        parts<real>(c, s), (int)first, c->sp[s].count_dev, fields<real>(c), c->g, push_const<real>(c, s), c->err);
-    CKL();
+int do_drift_n(pic_ctx* c, int species) {
+  TileLaunch<real> tl;
+  for (int s = 0; s < 2; ++s) {
+    if ((species >= 0 && s != species) || c->sp[s].count == 0) continue;
+    const bool tiles = c->layout[s];
+    if (!tiles || long_tail(c, s)) {
+      const long long first = tiles ? c->tiled_end[s] : 0;
+      drift_n_kernel<real><<<particle_blocks(c->sp[s].count - first), kThreads, 0, c->stream>>>(
+          parts<real>(c, s), (int)first, c->sp[s].count_dev, fields<real>(c), c->g, push_const<real>(c, s), c->err);
+      CKL();
+    }
+    if (tiles) tl.add(c, s);
   }
-  if (tiles) {
-    const TileArgs ta = tile_args(c, s, overlap && !apart);
-    CK(launch_after(c, c->g.gz % 4 == 0 ? drift_tiled_kernel<real, true> : drift_tiled_kernel<real, false>,
-                    ta.ntail + c->tg.ntx * c->tg.nty * c->tg.ntz, kTileX * kTileY * 32, 0, parts<real>(c, s), ta,
-                    fields<real>(c), c->g, push_const<real>(c, s), c->err));
-    CKL();
-  }
+  if (!tl.n) return PIC_OK;
+  CK(launch_after(c, c->g.gz % 4 == 0 ? drift_tiled_kernel<real, true> : drift_tiled_kernel<real, false>, tl.grid,
+                  kTileX * kTileY * 32, 0, tl.jobs, fields<real>(c), c->g, c->err));
+  CKL();
   return PIC_OK;
 }
 
@@ -1369,7 +1386,7 @@ int do_step(pic_ctx* c) {
   // the counts stay on the device: the push and the diagnostics cover the
   // slots up to the capacity and stop at the device count, and the host reads
   // a count back only when an entry point needs it
-  for (int s = 0; s < 2; ++s) CKR((do_push_tiled<real, PUSH_FUSED>(c, s, s == 1 && c->layout[0])));
+  CKR((do_push_tiled<real, PUSH_FUSED>(c, -1)));
   if (c->has_xport) CKR(do_migrate<real>(c));  // sr_particle's exchange between ranks
   CKR(phase_mark(c, PH_PUSH));
   CKR(phase_mark(c, PH_FIELD));
@@ -1962,23 +1979,13 @@ int pic_renew_e4_2(pic_ctx* c) {
 int pic_push_deposit_j(pic_ctx* c, int species) {
   CKR(check_ctx(c));
   if (species < -1 || species > 1) return PIC_ERR_ARG;
-  for (int s = 0; s < 2; ++s) {
-    if (species >= 0 && s != species) continue;
-    const bool overlap = species < 0 && s == 1 && c->layout[0] && c->layout[1];
-    CKR((c->prec == 64 ? do_push_tiled<double, PUSH_J>(c, s, overlap) : do_push_tiled<float, PUSH_J>(c, s, overlap)));
-  }
-  return PIC_OK;
+  return c->prec == 64 ? do_push_tiled<double, PUSH_J>(c, species) : do_push_tiled<float, PUSH_J>(c, species);
 }
 
 int pic_drift_deposit_n(pic_ctx* c, int species) {
   CKR(check_ctx(c));
   if (species < -1 || species > 1) return PIC_ERR_ARG;
-  for (int s = 0; s < 2; ++s) {
-    if (species >= 0 && s != species) continue;
-    const bool overlap = species < 0 && s == 1 && c->layout[0] && c->layout[1] && c->sp[0].count > 0;
-    CKR((c->prec == 64 ? do_drift_n<double>(c, s, overlap) : do_drift_n<float>(c, s, overlap)));
-  }
-  return PIC_OK;
+  return DISPATCH(c, do_drift_n)(c, species);
 }
 
 int pic_reduce_current(pic_ctx* c) {

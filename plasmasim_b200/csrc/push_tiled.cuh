@@ -395,13 +395,32 @@ constexpr int kLeftAll = 1, kLeftEnd = 2;
 template <typename real>
 __device__ __forceinline__ int left_of(const Parts<real>& P, int t) { return (int)P.rb[4 * (long long)t + 3]; }
 
+// One species' part of a launch over the tiles: its store, with ntail CTAs for
+// the slots from `tail` to *count, and a CTA for each tile.
+template <typename real>
+struct TileJob {
+  Parts<real> P;
+  PushConst<real> pc;
+  const int* goff;  // first slot of each group
+  const int* gtop;  // rows of each group up to the last one that holds a particle
+  int ntail, tail;
+  const int* count;
+};
+// The launch: job 0 in the first `split` CTAs, job 1 in the others.
+template <typename real>
+struct TileJobs {
+  TileJob<real> job[2];
+  int split;
+  TileGeom t;
+};
+
 // The slots after the layout (particles without a hole in their group): the
-// slot-order push, in the grid's first blocks.
+// slot-order push, in a job's first blocks.
 template <typename real, int MODE>
-__device__ __noinline__ void push_tail(const Parts<real>& P, const TileArgs& ta, const Fields<real>& F, const Geom& g,
-                                       const PushConst<real>& pc, unsigned long long* err) {
-  push_slots<real, MODE>(P, ta.tail + blockIdx.x * blockDim.x + threadIdx.x, ta.ntail * blockDim.x, *ta.count, F,
-                               g, pc, err);
+__device__ __noinline__ void push_tail(const TileJob<real>& job, int block, const Fields<real>& F, const Geom& g,
+                                       unsigned long long* err) {
+  push_slots<real, MODE>(job.P, job.tail + block * blockDim.x + threadIdx.x, job.ntail * blockDim.x, *job.count, F, g,
+                         job.pc, err);
 }
 
 // What the main loop left of particle t to the general path.
@@ -432,15 +451,18 @@ __device__ __noinline__ void push_rest(const Parts<real>& P, int t, const Fields
 // parts, for one species over the tiled layout;
 // the same arithmetic as push_kernel<real, PUSH_FUSED> apart from the FP32
 // square roots and divisions and, in FP32, the fixed-point sums of the density
-// window. One CTA per tile, one warp per group; the first ntail CTAs take the
-// slots after the layout (a launch of their own, 7 to 12 us per species for
+// window. One CTA per tile, one warp per group; a job's first ntail CTAs take
+// the slots after the layout (a launch of their own, 7 to 12 us per species for
 // next to no particles, before).
 //
-// The second species' launch may start before the first has finished (they
-// share nothing but the error counters): every CTA lets it go once what came
-// before is done, and the second's CTAs end with a wait for the first, so that whatever follows still
-// finds both done (0.068 -> 0.053 ms per step at 32^3 x 8, 0.336 -> 0.327 at
-// 64^3 x 16, the same at 128^3 x 64).
+// Both species go in one launch, the second's CTAs after the first's, so that
+// the first's last wave leaves no SM idle: push per step 0.044 ms at 32^3 x 8,
+// 0.300 at 64^3 x 16, 0.164 at 41 x 22 x 70 x 30, 6.53 at 128^3 x 64, against
+// 0.053, 0.311, 0.183 and 6.55 with a launch each, the second free to start
+// while the first ran. (The constants that the species share are taken from
+// the first's, so that they are operands at fixed addresses: 6.61 at 128^3 x 64
+// with all of them read through the CTA's own species; the kernel's body once
+// per species, 6.73.)
 //
 // J of a particle in its lane's home cell at x^{n+1/2} is summed in registers;
 // the others add theirs to global memory with reductions (a shared J window
@@ -469,14 +491,22 @@ __device__ __noinline__ void push_rest(const Parts<real>& P, int t, const Fields
 #endif
 template <typename real, bool VEC, int MODE>
 __global__ void __launch_bounds__(kTileX * kTileY * 32, sizeof(real) == 4 ? 2 : PB_PUSH64_MIN_BLOCKS)
-push_tiled_kernel(const __grid_constant__ Parts<real> P, const __grid_constant__ TileArgs ta,
-                  const __grid_constant__ Fields<real> F, const __grid_constant__ Geom g,
-                  const __grid_constant__ PushConst<real> pc, unsigned long long* err) {
-  if (!ta.overlap) wait_prior();
-  release_next();
-  if ((int)blockIdx.x < ta.ntail) {
-    push_tail<real, MODE>(P, ta, F, g, pc, err);
-    wait_prior();
+push_tiled_kernel(const __grid_constant__ TileJobs<real> jobs, const __grid_constant__ Fields<real> F,
+                  const __grid_constant__ Geom g, unsigned long long* err) {
+  after_prior();
+  const int second = (int)blockIdx.x >= jobs.split, block = (int)blockIdx.x - (second ? jobs.split : 0);
+  const TileJob<real>& job = jobs.job[second];
+  const Parts<real>& P = job.P;
+  // the species differ in these alone; the others stay immediate operands
+  PushConst<real> pc = jobs.job[0].pc;
+  pc.T = job.pc.T;
+  pc.pjx = job.pc.pjx;
+  pc.pjy = job.pc.pjy;
+  pc.pjz = job.pc.pjz;
+  pc.pn = job.pc.pn;
+  pc.out = job.pc.out;
+  if (block < job.ntail) {
+    push_tail<real, MODE>(job, block, F, g, err);
     return;
   }
   using S = PushSmem<real>;
@@ -485,8 +515,8 @@ push_tiled_kernel(const __grid_constant__ Parts<real> P, const __grid_constant__
   real* wn = reinterpret_cast<real*>(smem_raw);                // [WN]: n
   real* wj = reinterpret_cast<real*>(smem_raw + S::ring_off);  // [3][WN]: jx, jy, jz, after the last row
   real* fw = reinterpret_cast<real*>(smem_raw + S::fwin_off);  // [6][WN]: E, B
-  const int tile = blockIdx.x - ta.ntail;
-  const TileGeom& t = ta.t;
+  const int tile = block - job.ntail;
+  const TileGeom& t = jobs.t;
   const int tz = tile % t.ntz, ty = (tile / t.ntz) % t.nty, tx = tile / (t.ntz * t.nty);
   // window origin: two nodes below the tile's first interior cell (2 + tx*TX)
   const int wx0 = tx * kTileX, wy0 = ty * kTileY, wz0 = tz * kLanes;
@@ -505,7 +535,7 @@ push_tiled_kernel(const __grid_constant__ Parts<real> P, const __grid_constant__
   if (pc.long_moves) near.ex = 0;  // nobody takes the short path
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int G = tile * (kTileX * kTileY) + warp;
-  const int base = ta.goff[G], jmax = ta.gtop[G];
+  const int base = job.goff[G], jmax = job.gtop[G];
   // home cell of this lane
   const int hi = wx0 + 2 + warp / kTileY, hj = wy0 + 2 + warp % kTileY;
   const int nv = tile_cells(g, tz), hk = wz0 + 2 + lane_cell(nv, lane).z;
@@ -513,7 +543,7 @@ push_tiled_kernel(const __grid_constant__ Parts<real> P, const __grid_constant__
   const int wcell0 = (wx0 * WY + wy0) * WZ + wz0;  // window node of a cell: (i WY + j) WZ + k less this
   int slots = 0;
 #pragma unroll
-  for (int w = 0; w < kTileX * kTileY; ++w) slots += ta.gtop[tile * (kTileX * kTileY) + w];
+  for (int w = 0; w < kTileX * kTileY; ++w) slots += job.gtop[tile * (kTileX * kTileY) + w];
   const real nscale = window_scale(pc.nw, slots);
   HomeJ<real> acc;
   acc.zero();
@@ -656,9 +686,9 @@ push_tiled_kernel(const __grid_constant__ Parts<real> P, const __grid_constant__
   // faces of x and y since the last re-layout, mostly), or every row when the
   // list overflowed
   if (nrest > S::kRest) {
-    for (int jj = 0; jj < jmax; ++jj) push_rest<real, MODE>(P, base + jj * kLanes + lane, F, g, pc, err);
+    for (int jj = 0; jj < jmax; ++jj) push_rest<real, MODE>(P, base + jj * kLanes + lane, F, g, job.pc, err);
   } else {
-    for (int q = lane; q < nrest; q += kLanes) push_rest<real, MODE>(P, rest[q], F, g, pc, err);
+    for (int q = lane; q < nrest; q += kLanes) push_rest<real, MODE>(P, rest[q], F, g, job.pc, err);
   }
   // the lane's home-cell sums into the window (nodes h-1 .. h+1 around it)
   cp_async_wait<0>();
@@ -699,7 +729,6 @@ push_tiled_kernel(const __grid_constant__ Parts<real> P, const __grid_constant__
     }
     flush_nodes<VEC>(F.f[planes[q]] + ga * g.sx + gb * g.gz + gc, g.gz - gc, v);
   }
-  wait_prior();
 }
 
 // The drift loop of fdtd (:818-867) over the tiled layout: each particle to
@@ -712,31 +741,32 @@ push_tiled_kernel(const __grid_constant__ Parts<real> P, const __grid_constant__
 // took 3.9 ms, now 2.7, 0.7 of either to read the grid back.
 template <typename real, bool VEC>
 __global__ void __launch_bounds__(kTileX * kTileY * 32)
-drift_tiled_kernel(const __grid_constant__ Parts<real> P, const __grid_constant__ TileArgs ta,
-                   const __grid_constant__ Fields<real> F, const __grid_constant__ Geom g,
-                   const __grid_constant__ PushConst<real> pc, unsigned long long* err) {
+drift_tiled_kernel(const __grid_constant__ TileJobs<real> jobs, const __grid_constant__ Fields<real> F,
+                   const __grid_constant__ Geom g, unsigned long long* err) {
+  after_prior();
   using S = PushSmem<real>;
   constexpr int WY = S::WY, WZ = S::WZ, WN = S::WN, WX = S::WX, U = sizeof(real) == 4 ? 4 : 2;
-  if (!ta.overlap) wait_prior();
-  release_next();
-  if ((int)blockIdx.x < ta.ntail) {
-    drift_slots(P, ta.tail + blockIdx.x * blockDim.x + threadIdx.x, ta.ntail * blockDim.x, *ta.count, F, g, pc, err);
-    wait_prior();
+  const int second = (int)blockIdx.x >= jobs.split, block = (int)blockIdx.x - (second ? jobs.split : 0);
+  const TileJob<real>& job = jobs.job[second];
+  const Parts<real>& P = job.P;
+  const PushConst<real>& pc = job.pc;
+  if (block < job.ntail) {
+    drift_slots(P, job.tail + block * blockDim.x + threadIdx.x, job.ntail * blockDim.x, *job.count, F, g, pc, err);
     return;
   }
   __shared__ real wn[WN];
-  const int tile = blockIdx.x - ta.ntail;
-  const TileGeom& t = ta.t;
+  const int tile = block - job.ntail;
+  const TileGeom& t = jobs.t;
   const int tz = tile % t.ntz, ty = (tile / t.ntz) % t.nty, tx = tile / (t.ntz * t.nty);
   const int wx0 = tx * kTileX, wy0 = ty * kTileY, wz0 = tz * kLanes;
   for (int q = threadIdx.x; q < WN; q += blockDim.x) wn[q] = (real)0;
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int G = tile * (kTileX * kTileY) + warp;
-  const int base = ta.goff[G] + lane, jmax = ta.gtop[G];
+  const int base = job.goff[G] + lane, jmax = job.gtop[G];
   int slots = 0;
 #pragma unroll
-  for (int w = 0; w < kTileX * kTileY; ++w) slots += ta.gtop[tile * (kTileX * kTileY) + w];
+  for (int w = 0; w < kTileX * kTileY; ++w) slots += job.gtop[tile * (kTileX * kTileY) + w];
   const real nscale = window_scale(pc.nw, slots);
   // cells whose stencils lie in the window and the array
   CellRange near;
@@ -779,7 +809,6 @@ drift_tiled_kernel(const __grid_constant__ Parts<real> P, const __grid_constant_
     if (ga >= g.gx || gb >= g.gy || gc >= g.gz) continue;
     flush_nodes<VEC>(F.f[pc.pn] + ga * g.sx + gb * g.gz + gc, g.gz - gc, window_density(wn + (a * WY + b) * WZ + 4 * c4, pc.nw, nscale));
   }
-  wait_prior();
 }
 
 }  // namespace pb

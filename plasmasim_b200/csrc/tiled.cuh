@@ -72,16 +72,6 @@ struct TileGeom {
   int ngroups;        // ntx * nty * ntz * kTileX * kTileY
 };
 
-struct TileArgs {
-  TileGeom t;
-  const int* goff;  // first slot of each group
-  const int* gtop;  // rows of each group up to the last one that holds a particle
-  int ntail;        // CTAs of the grid that take the slots from `tail` to *count instead of a tile
-  int tail;
-  const int* count;
-  int overlap;      // the launch before is the other species' push: no need to wait for its end
-};
-
 // Group and lane of an interior cell (absolute indices), -1 outside the interior.
 __device__ __forceinline__ int group_of(const Geom& g, const TileGeom& t, int i, int j, int k,
                                         int& lane) {

@@ -2,7 +2,9 @@
 api.cu), checked on the sources: a load that the compiler may take for one of
 constant memory could be moved ahead of the kernel's wait for what came before
 it on the stream, so no argument of such a kernel is marked __restrict__ and
-none of its own lines uses __ldg."""
+none of its own lines uses __ldg; and only a kernel that waits itself is
+promised to see what the kernels before it wrote, so the wait is the first
+thing that each of them does."""
 import os
 import re
 
@@ -61,3 +63,9 @@ def test_windows_are_filled_behind_the_wait():
     start = text.index("fill_win(")
     body = text[start:until_closed(text, text.index("{", start), "{}")]
     assert "__ldg" not in body
+
+
+@pytest.mark.parametrize("name", early_kernels())
+def test_waits_first(name):
+    _, body = definition(name)
+    assert re.match(r"\{\s*after_prior\(\);", body)
