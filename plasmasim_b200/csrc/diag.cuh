@@ -204,8 +204,8 @@ __global__ void __launch_bounds__(256, 3) thrust_kernel(const __grid_constant__ 
     };
     fetch(0);
     if constexpr (kWin) {
-      if (a.vec) fill_win<float, S::WX, S::WY, S::WZ, true>(thrust_win, a.F, g, win.x0, win.y0, win.z0);
-      else fill_win<float, S::WX, S::WY, S::WZ, false>(thrust_win, a.F, g, win.x0, win.y0, win.z0);
+      if (a.vec) fill_win<float, S::WX, S::WY, S::WZ, true, 2>(thrust_win, a.F, g, win.x0, win.y0, win.z0);
+      else fill_win<float, S::WX, S::WY, S::WZ, false, 2>(thrust_win, a.F, g, win.x0, win.y0, win.z0);
       win.fw = thrust_win;
       __syncthreads();
     }

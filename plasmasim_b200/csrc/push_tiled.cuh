@@ -118,38 +118,52 @@ __device__ __forceinline__ Gathered<double> gather6_win(const double* __restrict
 }
 
 // The window's planes from F_EX .. F_BZ (16-byte loads where the row pitch
-// allows; ordinary ones, which stay behind the wait for the launch before),
-// zero outside the array.
-template <typename real, int WX, int WY, int WZ, bool VEC>
+// allows; ordinary ones, which stay behind the wait for the launch before, U of
+// them in flight together), zero outside the array. The compiler does not move
+// an ordinary load ahead of the last one's store: with one in flight the push
+// of both species took 0.298 ms per step at 64^3 x 16, 1.115 at 96 x 96 x 128 x
+// 16, FP64 64^3 x 32 1.61, with four 0.292, 1.083 and 1.59. thrust_kernel, which
+// holds its first records meanwhile, has registers for two (0.296 ms at 96 x 96
+// x 128 x 16 against 0.314 with one and 0.321 with four).
+template <typename real, int WX, int WY, int WZ, bool VEC, int U>
 __device__ __forceinline__ void fill_win(real* __restrict__ fw, const Fields<real>& F, const Geom& g, int wx0, int wy0,
                                          int wz0) {
-  constexpr int V = sizeof(real) == 4 ? 4 : 2, NZV = WZ / V, WN = WX * WY * WZ;
-  for (int q = threadIdx.x; q < 6 * WX * WY * NZV; q += blockDim.x) {
-    const int p = q / (WX * WY * NZV), r = q % (WX * WY * NZV);
-    const int a = r / (WY * NZV), b = (r / NZV) % WY, c = r % NZV;
-    const int ga = wx0 + a, gb = wy0 + b, gc = wz0 + V * c;
-    real v[V];
+  constexpr int V = sizeof(real) == 4 ? 4 : 2, NZV = WZ / V, WN = WX * WY * WZ, N = 6 * WX * WY * NZV;
+  for (int q0 = threadIdx.x; q0 < N; q0 += U * blockDim.x) {
+    real v[U][V];
 #pragma unroll
-    for (int e = 0; e < V; ++e) v[e] = (real)0;
-    if (ga < g.gx && gb < g.gy) {
-      const real* src = F.f[p] + (long long)ga * g.sx + gb * g.gz + gc;
-      if (VEC && gc + V - 1 < g.gz) {
-        if constexpr (V == 4) {
-          const float4 f4 = *reinterpret_cast<const float4*>(src);
-          v[0] = f4.x; v[1] = f4.y; v[2] = f4.z; v[3] = f4.w;
+    for (int u = 0; u < U; ++u) {
+      const int q = q0 + u * blockDim.x;
+      const int p = q / (WX * WY * NZV), r = q % (WX * WY * NZV);
+      const int ga = wx0 + r / (WY * NZV), gb = wy0 + (r / NZV) % WY, gc = wz0 + V * (r % NZV);
+#pragma unroll
+      for (int e = 0; e < V; ++e) v[u][e] = (real)0;
+      if (q < N && ga < g.gx && gb < g.gy) {
+        const real* src = F.f[p] + (long long)ga * g.sx + gb * g.gz + gc;
+        if (VEC && gc + V - 1 < g.gz) {
+          if constexpr (V == 4) {
+            const float4 f4 = *reinterpret_cast<const float4*>(src);
+            v[u][0] = f4.x; v[u][1] = f4.y; v[u][2] = f4.z; v[u][3] = f4.w;
+          } else {
+            const double2 f2 = *reinterpret_cast<const double2*>(src);
+            v[u][0] = f2.x; v[u][1] = f2.y;
+          }
         } else {
-          const double2 f2 = *reinterpret_cast<const double2*>(src);
-          v[0] = f2.x; v[1] = f2.y;
-        }
-      } else {
 #pragma unroll
-        for (int e = 0; e < V; ++e)
-          if (gc + e < g.gz) v[e] = src[e];
+          for (int e = 0; e < V; ++e)
+            if (gc + e < g.gz) v[u][e] = src[e];
+        }
       }
     }
-    real* dst = fw + p * WN + (a * WY + b) * WZ + V * c;
-    if constexpr (V == 4) *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
-    else *reinterpret_cast<double2*>(dst) = make_double2(v[0], v[1]);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int q = q0 + u * blockDim.x;
+      if (q >= N) break;
+      const int p = q / (WX * WY * NZV), r = q % (WX * WY * NZV);
+      real* dst = fw + p * WN + r / NZV * WZ + V * (r % NZV);
+      if constexpr (V == 4) *reinterpret_cast<float4*>(dst) = make_float4(v[u][0], v[u][1], v[u][2], v[u][3]);
+      else *reinterpret_cast<double2*>(dst) = make_double2(v[u][0], v[u][1]);
+    }
   }
 }
 
@@ -521,7 +535,7 @@ push_tiled_kernel(const __grid_constant__ TileJobs<real> jobs, const __grid_cons
   // window origin: two nodes below the tile's first interior cell (2 + tx*TX)
   const int wx0 = tx * kTileX, wy0 = ty * kTileY, wz0 = tz * kLanes;
   for (int q = threadIdx.x; q < WN; q += blockDim.x) wn[q] = (real)0;
-  fill_win<real, WX, WY, WZ, VEC>(fw, F, g, wx0, wy0, wz0);
+  fill_win<real, WX, WY, WZ, VEC, 4>(fw, F, g, wx0, wy0, wz0);
   __syncthreads();
   // the interior cells whose stencils lie in the window: a particle in one
   // needs no check of the array's bounds and none of sr_particle's
