@@ -462,10 +462,10 @@ __device__ __noinline__ void push_rest(const Parts<real>& P, int t, const Fields
 
 // The fused particle part of one step (push, J deposit at x^{n+1/2}, drift,
 // n deposit at x^{n+1}, sr_particle), or with MODE = PUSH_J its first two
-// parts, for one species over the tiled layout;
-// the same arithmetic as push_kernel<real, PUSH_FUSED> apart from the FP32
-// square roots and divisions and, in FP32, the fixed-point sums of the density
-// window. One CTA per tile, one warp per group; a job's first ntail CTAs take
+// parts, for one species over the tiled layout; the same arithmetic as
+// push_kernel apart from the order of the sums and, in the FP32 fused push
+// alone, the square roots and divisions and the fixed-point sums of the
+// density window. One CTA per tile, one warp per group; a job's first ntail CTAs take
 // the slots after the layout (a launch of their own, 7 to 12 us per species for
 // next to no particles, before).
 //
@@ -618,7 +618,9 @@ push_tiled_kernel(const __grid_constant__ TileJobs<real> jobs, const __grid_cons
     if (push) {
       const WinAxis<real> X = win_axis(fx, WY * WZ), Y = win_axis(fy, WZ), Z = win_axis(fz, 1);
       const real* n = fw + ((i * WY + j) * WZ + k - wcell0);
-      boris4_fast(pc, gather6_win<WY, WZ, WN>(n, X, Y, Z), vx, vy, vz);
+      const Gathered<real> eb = gather6_win<WY, WZ, WN>(n, X, Y, Z);
+      if (MODE == PUSH_J) boris4(pc, eb, vx, vy, vz);
+      else boris4_fast(pc, eb, vx, vy, vz);
       // one test for the three: |v| < c, so the sum of finite components is finite
       nbad += !isfinite(vx + vy + vz);
     }
