@@ -823,8 +823,7 @@ int do_drift_n(pic_ctx* c, int species) {
     if (tiles) tl.add(c, s);
   }
   if (!tl.n) return PIC_OK;
-  CK(launch_after(c, c->g.gz % 4 == 0 ? drift_tiled_kernel<real, true> : drift_tiled_kernel<real, false>, tl.grid,
-                  kTileX * kTileY * 32, 0, tl.jobs, fields<real>(c), c->g, c->err));
+  CK(launch_after(c, drift_tiled_kernel<real>, tl.grid, kTileX * kTileY * 32, 0, tl.jobs, fields<real>(c), c->g, c->err));
   CKL();
   return PIC_OK;
 }

@@ -747,21 +747,53 @@ push_tiled_kernel(const __grid_constant__ TileJobs<real> jobs, const __grid_cons
   }
 }
 
+// The density of the particles that are in a lane's home cell, summed in
+// registers over the 3x3x3 nodes around it.
+template <typename real>
+struct HomeN {
+  real n[3][3][3];
+  template <typename F>
+  __device__ __forceinline__ void each(F f) {
+#pragma unroll
+    for (int q = 0; q < 27; ++q) f(n[q / 9][q / 3 % 3][q % 3]);
+  }
+  __device__ __forceinline__ void zero() {
+    each([](real& v) { v = (real)0; });
+  }
+  __device__ __forceinline__ void add(real w, const W3<real>& bx, const W3<real>& by, const W3<real>& bz) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int b = 0; b < 3; ++b) {
+        const real xy = (w * bx.w[a]) * by.w[b];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) n[a][b][c] += xy * bz.w[c];
+      }
+  }
+};
+
 // The drift loop of fdtd (:818-867) over the tiled layout: each particle to
-// x^{n+1} and its density, into the tile's window as in push_tiled_kernel; a
-// cell whose stencil leaves the window or the array goes the general way. One
-// CTA per tile, one warp per group, U rows' records in flight; the first ntail
-// CTAs take the slots after the layout. Bound by the records' latency and the
-// shared reductions; with PUSH_J in tiles as well, against a thread per slot and
-// atomics on the planes: four loop bodies of 48^3 x 16 by single functions
-// took 3.9 ms, now 2.7, 0.7 of either to read the grid back.
-template <typename real, bool VEC>
-__global__ void __launch_bounds__(kTileX * kTileY * 32)
+// x^{n+1} and its density, of a particle in its lane's home cell there summed in
+// registers and added to the plane once per lane, of any other through the
+// warp's queue, 32 at a time. The sums are of the particles' own type, as in
+// slot order: in the fused push's fixed-point window a sparse cell beside a
+// crowded one of its tile loses bits. One CTA per tile, one warp per group, the
+// next U rows' records on their way; a job's first ntail CTAs take the slots
+// after the layout.
+//
+// Bound by DRAM when the grid is large (128^3 x 64: 48 bytes a particle in 2.20
+// ms for both species, 89 % of the copy rate), by the records' latency when it
+// is small (58 us at 48^3 x 16). With the fixed-point window 1.95 ms and 47 us,
+// with a thread per slot and atomics on the plane 9.67 ms and 192 us; FP64 64^3 x
+// 32, where the window took FP64 shared atomics: 0.477 -> 0.300 ms. Warps per
+// SM and U: 32 and 2; 24 and 2 or 4 took 2.48 and 2.25 ms, 32 and 1 or 3 2.56
+// and 2.58, 40 and 1 2.77. The sums through a shared window: 2.30.
+template <typename real>
+__global__ void __launch_bounds__(kTileX * kTileY * 32, sizeof(real) == 4 ? 4 : 2)
 drift_tiled_kernel(const __grid_constant__ TileJobs<real> jobs, const __grid_constant__ Fields<real> F,
                    const __grid_constant__ Geom g, unsigned long long* err) {
   after_prior();
-  using S = PushSmem<real>;
-  constexpr int WY = S::WY, WZ = S::WZ, WN = S::WN, WX = S::WX, U = sizeof(real) == 4 ? 4 : 2;
+  constexpr int kWarps = kTileX * kTileY, kQ = 2 * kLanes, U = 2;
   const int second = (int)blockIdx.x >= jobs.split, block = (int)blockIdx.x - (second ? jobs.split : 0);
   const TileJob<real>& job = jobs.job[second];
   const Parts<real>& P = job.P;
@@ -770,61 +802,90 @@ drift_tiled_kernel(const __grid_constant__ TileJobs<real> jobs, const __grid_con
     drift_slots(P, job.tail + block * blockDim.x + threadIdx.x, job.ntail * blockDim.x, *job.count, F, g, pc, err);
     return;
   }
-  __shared__ real wn[WN];
+  // per warp, the densities off the home cells: cell and offsets (5 words, odd, for the banks)
+  __shared__ real queue[kWarps][kQ * 5];
   const int tile = block - job.ntail;
   const TileGeom& t = jobs.t;
   const int tz = tile % t.ntz, ty = (tile / t.ntz) % t.nty, tx = tile / (t.ntz * t.nty);
-  const int wx0 = tx * kTileX, wy0 = ty * kTileY, wz0 = tz * kLanes;
-  for (int q = threadIdx.x; q < WN; q += blockDim.x) wn[q] = (real)0;
-  __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int G = tile * (kTileX * kTileY) + warp;
+  const int G = tile * kWarps + warp;
   const int base = job.goff[G] + lane, jmax = job.gtop[G];
-  int slots = 0;
+  if (jmax == 0) return;
+  const int hi = tx * kTileX + 2 + warp / kTileY, hj = ty * kTileY + 2 + warp % kTileY;
+  const int nv = tile_cells(g, tz), hk = tz * kLanes + 2 + lane_cell(nv, lane).z;
+  real* mine = queue[warp];
+  int nq = 0;
+  const auto deposit_queued = [&](int q) {
+    const real* e = mine + q * 5;
+    int i, j, k;
+    unpack_cell(word_int(e[0]), i, j, k);
+    deposit_n(F, g, pc, axis_weights(i, e[1]), axis_weights(j, e[2]), axis_weights(k, e[3]));
+  };
+  HomeN<real> acc;
+  acc.zero();
+  Rec<real> q[U];
+  const auto fetch = [&](int r0) {
 #pragma unroll
-  for (int w = 0; w < kTileX * kTileY; ++w) slots += job.gtop[tile * (kTileX * kTileY) + w];
-  const real nscale = window_scale(pc.nw, slots);
-  // cells whose stencils lie in the window and the array
-  CellRange near;
-  near.lx = wx0 + 1;
-  near.ly = wy0 + 1;
-  near.lz = wz0 + 1;
-  near.ex = (unsigned)(min(wx0 + WX - 1, g.gx - 1) - near.lx);
-  near.ey = (unsigned)(min(wy0 + WY - 1, g.gy - 1) - near.ly);
-  near.ez = (unsigned)(min(wz0 + WZ - 1, g.gz - 1) - near.lz);
+    for (int u = 0; u < U; ++u)
+      q[u] = r0 + u < jmax ? load_records(P, base + (r0 + u) * kLanes)
+                           : Rec<real>{-1, {(real)0, (real)0, (real)0}, {(real)0, (real)0, (real)0}};
+  };
+  fetch(0);
   for (int r0 = 0; r0 < jmax; r0 += U) {
-    Rec<real> q[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      q[u].cell = -1;
-      if (r0 + u < jmax) q[u] = load_records(P, base + (r0 + u) * kLanes);
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      if (q[u].cell < 0) continue;
+      const bool act = q[u].cell >= 0;
       int i, j, k;
       unpack_cell(q[u].cell, i, j, k);
       real fx = q[u].o[0], fy = q[u].o[1], fz = q[u].o[2];
-      advance(i, fx, q[u].v[0] * pc.hdt);
-      advance(j, fy, q[u].v[1] * pc.hdt);
-      advance(k, fz, q[u].v[2] * pc.hdt);
-      if (near.has(i, j, k)) {
-        const WinAxis<real> X = win_axis(fx, WY * WZ), Y = win_axis(fy, WZ), Z = win_axis(fz, 1);
-        add_density<WY, WZ>(wn + (((i - wx0) * WY + j - wy0) * WZ + k - wz0) + X.s + Y.s + Z.s, nscale, X, Y, Z);
-      } else {
-        drift_density(F, g, pc, i, j, k, fx, fy, fz, err);
+      if (act) {
+        advance(i, fx, q[u].v[0] * pc.hdt);
+        advance(j, fy, q[u].v[1] * pc.hdt);
+        advance(k, fz, q[u].v[2] * pc.hdt);
+        store_position(P, base + (r0 + u) * kLanes, repack(i, j, k, err), fx, fy, fz);
       }
-      store_position(P, base + (r0 + u) * kLanes, repack(i, j, k, err), fx, fy, fz);
+      // a lane without a home particle adds zeros, at offsets of 1/2 whatever its own are
+      const bool home = act && i == hi && j == hj && k == hk;
+      acc.add(home ? pc.nw : (real)0, home3(home ? fx : (real)0.5), home3(home ? fy : (real)0.5),
+              home3(home ? fz : (real)0.5));
+      bool off = act && !home && in_array(g, i, j, k);
+      if (off && !stencil_ok(g, i, j, k)) {
+        count_err(err, ERR_DEPOSIT_OOB);
+        off = false;
+      }
+      const unsigned em = __ballot_sync(0xffffffffu, off);
+      if (off) {
+        real* e = mine + (nq + __popc(em & ((1u << lane) - 1u))) * 5;
+        e[0] = int_word<real>(pack_cell(i, j, k));
+        e[1] = fx; e[2] = fy; e[3] = fz;
+      }
+      nq += __popc(em);
+      if (nq >= kLanes) {
+        __syncwarp();
+        deposit_queued(nq - kLanes + lane);
+        nq -= kLanes;
+        __syncwarp();
+      }
     }
+    fetch(r0 + U);
   }
-  __syncthreads();
-  constexpr int NZ4 = WZ / 4;
-  for (int q4 = threadIdx.x; q4 < WX * WY * NZ4; q4 += blockDim.x) {
-    const int a = q4 / (WY * NZ4), b = (q4 / NZ4) % WY, c4 = q4 % NZ4;
-    const int ga = wx0 + a, gb = wy0 + b, gc = wz0 + 4 * c4;
-    if (ga >= g.gx || gb >= g.gy || gc >= g.gz) continue;
-    flush_nodes<VEC>(F.f[pc.pn] + ga * g.sx + gb * g.gz + gc, g.gz - gc, window_density(wn + (a * WY + b) * WZ + 4 * c4, pc.nw, nscale));
-  }
+  __syncwarp();
+  if (lane < nq) deposit_queued(lane);
+  if (nv < kLanes) merge_lanes(acc, nv, lane);
+  // node h + c - 1 of a lane is its neighbour's: one sum per node and column
+  real* n = F.f[pc.pn] + (hi - 1) * g.sx + (hj - 1) * g.gz + hk;
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      const real below = __shfl_up_sync(0xffffffffu, acc.n[a][b][2], 1);
+      const real above = __shfl_down_sync(0xffffffffu, acc.n[a][b][0], 1);
+      real* p = n + a * g.sx + b * g.gz;
+      if (lane >= nv) continue;
+      atomicAdd(p, acc.n[a][b][1] + (lane > 0 ? below : (real)0) + (lane + 1 < nv ? above : (real)0));
+      if (lane == 0) atomicAdd(p - 1, acc.n[a][b][0]);
+      if (lane + 1 == nv) atomicAdd(p + 1, acc.n[a][b][2]);
+    }
 }
 
 }  // namespace pb

@@ -1,10 +1,11 @@
-"""The FP32 push called by itself over the tiled layout keeps what slot order
-has in precision: correctly rounded square roots and divisions."""
+"""The FP32 push and drift loops called by themselves over the tiled layout
+keep what slot order has in precision: correctly rounded square roots and
+divisions, and FP32 sums however uneven the tile's cells are."""
 import numpy as np
 import pytest
 
 from plasmasim_b200 import ELECTRON, ION, Pic3D, PicConfig
-from util import match_rows
+from util import NE, NI, match_rows
 
 pytestmark = pytest.mark.gpu
 
@@ -41,3 +42,30 @@ def test_velocities_are_as_exact_as_in_slot_order():
             mine, ref = match_rows(P.particles(ION), after)
             rms.append(np.sqrt(((mine[:, 3:6] - ref[:, 3:6]) ** 2).sum() / (ref[:, 3:6] ** 2).sum()))
     assert rms[0] <= 1.005 * rms[1], rms
+
+
+def test_sparse_cells_beside_a_crowd():
+    """Single resting particles in the tile of a cell that holds 20000. Offsets
+    are multiples of 2^-8, so each of a particle's eight weights has at most
+    24 bits and is rounded when it is scaled by the particle's own weight, and
+    once more in each product: 4 x 2^-24 of the node's density."""
+    rng = np.random.default_rng(2)
+    crowd = np.array([2, 2, 2]) + (rng.integers(1, 256, (20000, 3))) / 256
+    cells = np.array([[3, 5, k] for k in range(6, 32, 4)])
+    single = cells + rng.integers(1, 256, cells.shape) / 256
+    xyz = np.concatenate([crowd, single])
+    rows = np.column_stack([xyz, np.zeros_like(xyz), np.full(len(xyz), 0.01 / 4)])
+    with context() as P:
+        for s in (ION, ELECTRON):
+            P.set_particles(s, rows)
+        P.sorting()
+        P.renew_grid()
+        P.drift_deposit_n()
+        g = P.grid()
+    for x in single:
+        base = np.floor(x - 0.5).astype(int)
+        f = x - 0.5 - base
+        for d in np.ndindex(2, 2, 2):
+            w = np.prod(np.where(d, f, 1 - f)) * float(np.float32(0.01 / 4))
+            for q in (NI, NE):
+                assert abs(g[tuple(base + d) + (q,)] - w) <= 4 * 2.0 ** -24 * w
