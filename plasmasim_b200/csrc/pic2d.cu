@@ -1116,7 +1116,7 @@ __global__ void __launch_bounds__(256) dst_gemm_kernel(const Run<real>* __restri
       gemm_tile<real, T>(stage, nz, [&](int r, int k) { return element(a, nx, nz, row0 + r, k); },
                          [&](int k, int c) { return element(Sz, nz, nz, k, col0 + c); }, acc);
     }
-    const double inv = mode == 2 ? 2. / nx : 2. / nz, h2 = (R.dx / 2.) * (R.dx / 2.);
+    const double len = mode == 2 ? nx : nz, inv = 2. / len, h2 = (R.dx / 2.) * (R.dx / 2.);
     const double* ex = sin2 + R.ev;
     const double* ez = ex + nx;
 #pragma unroll
@@ -1130,7 +1130,7 @@ __global__ void __launch_bounds__(256) dst_gemm_kernel(const Run<real>* __restri
           const double e = -(ez[col] + ex[row]) / h2;
           w = e == 0. ? (real)0 : (real)((double)w / e);
         } else if (mode >= 2) {
-          w = (real)(inv * (double)w);
+          w = (real)(sizeof(real) == 4 ? inv * (double)w : 2. * (double)w / len);  // 2 / len is rounded
         }
         cmat[(long long)row * nz + col] = w;
       }

@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(256) dst3_gemm_kernel(DstGemm<real> a) {
         stage, a.K, [&](int m, int k) { return m0 + m < a.M && k < a.K ? L[(m0 + m) * a.lm + k] : (real)0; },
         [&](int k, int n) { return k < a.K && n0 + n < a.N ? R[k * a.rk + n0 + n] : (real)0; }, acc);
     real* C = a.C + b * a.cb;
-    const double scale = a.mul / a.div;
+    const double scale = a.mul / a.div;  // enough for a result rounded to FP32; FP64 divides
 #pragma unroll
     for (int i = 0; i < U; ++i) {
       const int gm = m0 + U * ty + i;
@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(256) dst3_gemm_kernel(DstGemm<real> a) {
       for (int j = 0; j < U; ++j) {
         const int gn = n0 + U * tx + j;
         if (gn >= a.N) continue;
-        double v = scale * (double)acc[i][j];
+        double v = sizeof(real) == 4 ? scale * (double)acc[i][j] : a.mul * (double)acc[i][j] / a.div;
         if (a.solve) {
           const int kx = gm, ky = gn / a.nz, kz = gn % a.nz;
           const double ev = -(a.sin2[a.nx + ky] + a.sin2[a.nx + a.ny + kz] + a.sin2[kx]) / a.h2;
