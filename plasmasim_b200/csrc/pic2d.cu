@@ -362,8 +362,8 @@ template <typename real>
 __global__ void __launch_bounds__(256) zero_sources_kernel(real* F, const Run<real>* __restrict__ runs) {
   const Run<real>& R = runs[blockIdx.x];
   real* base = F + R.foff + (long long)P_JIX * R.nodes;
-  const int n = (P_COUNT - P_JIX) * R.nodes;
-  for (int q = blockIdx.y * blockDim.x + threadIdx.x; q < n; q += gridDim.y * blockDim.x) base[q] = (real)0;
+  const long long n = (long long)(P_COUNT - P_JIX) * R.nodes;  // beyond 2^31 from 15447 nodes a side on
+  for (long long q = blockIdx.y * blockDim.x + threadIdx.x; q < n; q += gridDim.y * blockDim.x) base[q] = (real)0;
 }
 
 // ------------------------------------------------------------ particles
