@@ -134,6 +134,10 @@ REF2D_CONFIGS = {
 }
 
 
+class ReferenceMissing(FileNotFoundError):
+    """A compiled reference is neither there nor to be built: no source."""
+
+
 def ref2d_lib_path(name: str) -> str:
     return os.path.join(REF_OUT, f"libref2d_{name}.so")
 
@@ -145,7 +149,7 @@ def build_ref2d(name: str, force: bool = False) -> str:
     if os.path.isfile(out) and not force:
         return out
     if not os.path.isfile(REF2D_SRC):
-        raise FileNotFoundError(f"2D reference source not found at {REF2D_SRC}")
+        raise ReferenceMissing(f"2D reference source not found at {REF2D_SRC}")
     os.makedirs(REF_OUT, exist_ok=True)
     defs = [f"-D{k}={_fmt(v)}" for k, v in REF2D_CONFIGS[name].items()]
     sed = subprocess.run(["sed", "-f", os.path.join(HERE, "ref2d_patch.sed"), REF2D_SRC],
