@@ -744,13 +744,9 @@ __global__ void fold_y_adjoint(PlaneSet<real> s, Geom g) {
   }
 }
 
-// Stable compaction with its slot map (the adjoint run's refill): map[t] is
-// the new slot of live slot t, -1 for an empty one. pos = exclusive scan of
-// the live flags.
 // Sort keys of the refill's compaction: the linear node index of a live
 // slot's cell ((i gy + j) gz + k, below the node count), `dead` for an empty
-// slot; the values are the slot indices. The keys span few bits, so the radix
-// sort makes few passes.
+// slot; the values are the slot indices.
 template <typename real>
 __global__ void cell_key_kernel(Parts<real> P, int n, Geom g, int dead, int* key, int* slot) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;

@@ -40,8 +40,8 @@ struct Store {
   long long cap = 0;
   long long count = 0;  // slots in use (live and empty); the host's copy of *count_dev unless `pending`
   int* count_dev = nullptr;
-  // *count_dev has moved on without the host (a placement, a re-listing push,
-  // a refill appended on the device): kernels cover the slots up to the
+  // *count_dev has moved on without the host (a placement, a refill appended
+  // on the device): kernels cover the slots up to the
   // capacity and stop at *count_dev, and sync_count reads it back when the
   // host needs it
   bool pending = false;
@@ -927,14 +927,13 @@ int do_sort_species(pic_ctx* c, int s) {
   return PIC_OK;
 }
 
-// In-place re-layout (relayout.cuh): movers and appended particles into the
-// holes of their columns, which a classify pass lists (relayout_launch). It
-// issues the placement, set the new count on the device and read the
-// spill count back into pinned memory without waiting; check_spill acts on
-// that read-back when it has landed (a full sort when many particles found no
+// The placement of an in-place re-layout (relayout.cuh): the movers and
+// appended particles, from tiled_end to *append_dev, into the holes of their
+// groups, which a classify pass has listed in st.holes and st.nholes
+// (relayout_launch). It sets the new count on the device and starts a read-back
+// of the spill count into pinned memory without waiting for it: check_spill
+// acts on that when it has landed (a full sort when many particles found no
 // hole), sync_count reads the count itself when the host needs it.
-// The placement of the particles in [tiled_end, *count_dev) into the holes
-// that st.holes / st.nholes list (place_launch).
 template <typename real>
 int place_launch(pic_ctx* c, int s) {
   Store& st = c->sp[s];
@@ -1850,7 +1849,7 @@ int pic_create(const pic_config* cfg, pic_ctx** out) {
     if (cudaMalloc(&c->total_dev, sizeof(int)) != cudaSuccess) return fail(PIC_ERR_CUDA);
     if (cudaMalloc(&c->append_dev, sizeof(int)) != cudaSuccess) return fail(PIC_ERR_CUDA);
     if (tiled) {  // re-layout scratch
-      for (int s = 0; s < 2; ++s) {  // each species' hole lists live from its push to its next placement
+      for (int s = 0; s < 2; ++s) {  // each species' hole lists live from its classify pass to its placement
         if (cudaMalloc(&c->sp[s].holes, sizeof(int) * (size_t)cap) != cudaSuccess) return fail(PIC_ERR_CUDA);
         if (cudaMalloc(&c->sp[s].nholes, sizeof(int) * 2 * kLanes * t.ngroups) != cudaSuccess) return fail(PIC_ERR_CUDA);
         if (cudaMalloc(&c->sp[s].nspill, 2 * sizeof(int)) != cudaSuccess) return fail(PIC_ERR_CUDA);

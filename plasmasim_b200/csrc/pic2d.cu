@@ -1134,7 +1134,6 @@ __global__ void __launch_bounds__(256) dst_gemm_kernel(const Run<real>* __restri
         }
         cmat[(long long)row * nz + col] = w;
       }
-    __syncthreads();  // the next tile's stage may be written
   }
 }
 

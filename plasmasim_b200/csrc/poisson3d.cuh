@@ -110,7 +110,6 @@ __global__ void __launch_bounds__(256) dst3_gemm_kernel(DstGemm<real> a) {
         C[gm * a.cm + gn] = (real)v;
       }
     }
-    __syncthreads();  // the next tile's stage may be written
   }
 }
 

@@ -49,7 +49,8 @@ __device__ __forceinline__ void load_run(const double* p, double (&v)[U]) {
 // U ty .. U ty + U - 1 and columns U tx .. of the tile (tx = thread % 16, ty =
 // thread / 16). left(row, k) and right(k, col) give the elements of the tile's
 // rows, columns and all k, zero outside the matrices. Every thread of the
-// block calls it; `first` tells that no earlier product's stage is still read.
+// block calls it; each stage begins with a barrier, which also keeps it from the
+// last one's readers of an earlier product.
 template <typename real, int T, typename Left, typename Right>
 __device__ __forceinline__ void gemm_tile(GemmStage<real, T>& st, int K, Left left, Right right,
                                           real (&acc)[T / 16][T / 16]) {

@@ -26,9 +26,9 @@
 // touch) and adds them to a shared-memory window of (TX+4) x (TY+4) x 36 nodes
 // once, after its last particle. The currents of particles that have left
 // their home cell since the sort are queued per warp and added to the planes
-// 32 at a time; the densities go to the window as fixed-point numbers with
-// shared integer reductions, or, when the stencil leaves the window (periodic
-// wrap, long moves), to global memory. The window is added to the global planes
+// 32 at a time; the densities of the fused push go to the window, in FP32 as
+// fixed-point numbers with shared integer reductions, or, when the stencil
+// leaves the window (periodic wrap, long moves), to global memory. The window is added to the global planes
 // with one vector reduction per 4 nodes.
 //
 // Sort. Between sorts most particles stay in their cell. The sort keeps the
