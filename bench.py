@@ -286,17 +286,18 @@ def run_e2e(P, steps: int):
 # from the ncu capture of a 64^3 x 64 ppc launch
 # (profiles/push_tiled_kernel_grid64_64ppc.md); at a fixed number of particles
 # per cell the traffic of a launch grows with its particles.
-PUSH_TRAFFIC_PER_PARTICLE = 61.9
+PUSH_TRAFFIC_PER_PARTICLE = 64.0
 
 
-def roofline(out, npart_species, cells, rsize):
-    """Push kernel: algorithmic bytes per launch = particles x (read + write of
-    the SoA state: 4 + 6 rsize bytes each way) + cells x rsize x (6 gathered
-    field components + 4 deposited quantities)."""
+def roofline(out, cells, rsize):
+    """Push kernel, one launch per step for both species: algorithmic bytes per
+    launch = particles x (read + write of the state: 4 + 6 rsize bytes each
+    way) + cells x rsize x (6 gathered field components + 4 deposited
+    quantities of each species)."""
     pushes = out["pushed"]
-    launches = out["phase_pairs"]["push"] * 2
+    launches = out["phase_pairs"]["push"]
     per_particle = 2 * (4 + 6 * rsize)
-    bytes_total = pushes * per_particle + launches * cells * rsize * 10
+    bytes_total = pushes * per_particle + launches * cells * rsize * 14
     secs = out["phase_ms"]["push"] / 1e3
     return bytes_total / secs / 1e9, bytes_total / max(launches, 1), secs / max(launches, 1)
 
@@ -712,8 +713,7 @@ def main():
     ms_max, pushed_all = combine_over_ranks(ms, pushed, dist)
     value = pushed_all / (ms_max / 1e3)
     cells = (NX + 4) * (NY + 4) * (NZ + 4)
-    nsp = pushed / max(args.steps, 1) / 2
-    ach, bytes_launch, s_launch = roofline(out, nsp, cells, 4)
+    ach, bytes_launch, s_launch = roofline(out, cells, 4)
     peak, peak_kind = measured_peaks()
     step_bytes = pushed / max(args.steps, 1) * 56 + NX * NY * NZ * 200
 
@@ -800,7 +800,7 @@ def main():
                        "parallelism": f"replicas{world}"},
             "roofline": {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
                          "frac": ach / peak,
-                         "traffic": PUSH_TRAFFIC_PER_PARTICLE * nsp if PPC == 64 else None,
+                         "traffic": PUSH_TRAFFIC_PER_PARTICLE * pushed / max(args.steps, 1) if PPC == 64 else None,
                          "kernel": "push_tiled_kernel<float,true,PUSH_FUSED> (push phase)",
                          "peak_kind": peak_kind, "bytes_per_launch": bytes_launch,
                          "ms_per_launch": s_launch * 1e3},

@@ -485,8 +485,8 @@ __device__ __noinline__ void push_rest(const Parts<real>& P, int t, const Fields
 // window with shared reductions (every active lane at once): integer ones on
 // fixed-point sums in FP32, FP64 atomics in FP64.
 //
-// Bound by instruction issue (16 warps per SM, 55 % of the slots issue; DRAM at
-// 17 %), so the loop is written for few instructions: cells stay packed while
+// Bound by instruction issue (16 warps per SM, 65 % of the slots issue; DRAM at
+// 29 %), so the loop is written for few instructions: cells stay packed while
 // they move (step_cell), one range test says that a particle needs no bounds
 // checks, window addresses come from one multiply-add chain and the lanes
 // without a particle run along with zero currents instead of branching. What
